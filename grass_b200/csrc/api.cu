@@ -273,40 +273,37 @@ int open_impl(ByteSource &src, const uint8_t *ob, uint64_t osize, int mode, int 
     Nvtx nv("device layout");
     const uint64_t E = stats[0];
     uint64_t *d_rp = nullptr, *d_P = nullptr;
-    uint32_t *d_cl = nullptr, *d_meta = nullptr, *d_fp = nullptr;
+    uint32_t *d_cl = nullptr, *d_meta = nullptr;
     GRASS_CUDA(cudaMalloc(&d_rp, (n + 1) * sizeof(uint64_t)));
     tmp.dev.push_back(d_rp);
     GRASS_CUDA(cudaMalloc(&d_cl, std::max<uint64_t>(E, 1) * 4));
     tmp.dev.push_back(d_cl);
     GRASS_CUDA(cudaMalloc(&d_meta, n * 4));
     tmp.dev.push_back(d_meta);
-    GRASS_CUDA(cudaMalloc(&d_fp, n * 4));
-    tmp.dev.push_back(d_fp);
     GRASS_CUDA(cudaMalloc(&d_P, n * sizeof(uint64_t)));
     tmp.dev.push_back(d_P);
-    launch_degrees64(g->view(), d_rp, st);
-    launch_scan_u64_inplace(d_rp, n, d_scan, st);
+    launch_scan_degrees(g->d_recs, n, d_rp, d_scan, st);
     launch_disk_decode(mode, g->d_words, g->d_recs, (uint32_t)n, d_rp, d_cl, st);
-    launch_slot_choose(mode, d_rp, d_cl, (uint32_t)n, d_meta, d_fp, st);
+    launch_slot_choose(d_rp, d_cl, (uint32_t)n, d_meta, st);
     std::vector<uint32_t> meta(n);
     std::vector<uint64_t> rp(n + 1), P(n, 0);
     GRASS_CUDA(cudaMemcpyAsync(meta.data(), d_meta, n * 4, cudaMemcpyDeviceToHost, st));
     GRASS_CUDA(cudaMemcpyAsync(rp.data(), d_rp, (n + 1) * 8, cudaMemcpyDeviceToHost, st));
     GRASS_CUDA(cudaStreamSynchronize(st));
     GRASS_CUDA(cudaGetLastError());
+    cudaFree(g->d_words);  // the on-disk stream is in the temporary CSR now
+    g->d_words = nullptr;
     // First fit in vertex order: a vertex whose slots fit in one sector goes
     // at the current bit if it does not cross the sector end; a larger one
-    // starts on the next sector.  Slots: GT ceil(d / T), LE ceil((d - 1) / T)
-    // (an LE vertex of degree 1 keeps its neighbor in the record).
-    const bool gt = mode == GRASS_MODE_GT;
+    // starts on the next sector.  (A vertex of degree 1 keeps its neighbor in
+    // the record.)
     uint64_t pos = 0;
     for (uint64_t v = 0; v < n; v++) {
       const uint64_t d = rp[v + 1] - rp[v];
-      if (d < (gt ? 1u : 2u)) continue;
+      if (d < 2) continue;
       const uint32_t m = meta[v];
       const uint64_t T = m & 0xFFu, b = (m >> 8) & 0xFFu, K = (m >> 16) & 0xFFu, a = m >> 24;
-      const uint64_t cb = gt ? a + (T - 1) * b : 2 * a + (T - 1) * (b + 1);
-      const uint64_t C = gt ? (d - 1) / T + 1 : (d - 2) / T + 1;
+      const uint64_t cb = a + (T - 1) * b, C = (d - 1) / T + 1;
       if (C <= K) {
         if ((pos & 255) + C * cb > 256) pos = (pos + 255) & ~255ull;
       } else {
@@ -322,14 +319,12 @@ int open_impl(ByteSource &src, const uint8_t *ob, uint64_t osize, int mode, int 
     words_alloc = (nw + kGuardWords + 7) / 8 * 8;
     uint32_t *d_slots = nullptr;
     GRASS_CUDA(cudaMalloc(&d_slots, words_alloc * 4));
-    tmp.dev.push_back(d_slots);
+    g->d_words = d_slots;
     GRASS_CUDA(cudaMemsetAsync(d_slots, 0, words_alloc * 4, st));
     GRASS_CUDA(cudaMemcpyAsync(d_P, P.data(), n * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    launch_slot_write(mode, d_rp, d_cl, (uint32_t)n, d_meta, d_fp, d_P, d_slots, g->d_recs, st);
+    launch_slot_write(d_rp, d_cl, (uint32_t)n, d_meta, d_P, d_slots, g->d_recs, st);
     GRASS_CUDA(cudaStreamSynchronize(st));
     GRASS_CUDA(cudaGetLastError());
-    tmp.dev.back() = g->d_words;  // the on-disk stream is freed with tmp
-    g->d_words = d_slots;
     g->n_words = nw;
   }
 
@@ -541,8 +536,7 @@ int grass_decode_all(const grass_graph *g, uint64_t *d_rowptr, uint32_t *d_cols,
   uint64_t *scan_tmp = nullptr;
   GRASS_CUDA(scratch_alloc(reinterpret_cast<void **>(&scan_tmp),
                            (scan_tmp_words(n) + 1) * sizeof(uint64_t), st));
-  launch_degrees64(g->view(), d_rowptr, st);
-  launch_scan_u64_inplace(d_rowptr, n, scan_tmp, st);
+  launch_scan_degrees(g->d_recs, n, d_rowptr, scan_tmp, st);
   int rc = launch_decode_planned(g, d_rowptr, d_cols, g->d_err, st);
   scratch_free(scan_tmp, st);
   return rc ? rc : check_launch();

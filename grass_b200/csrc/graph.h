@@ -159,22 +159,23 @@ void launch_scan_u32(const uint32_t *counts, uint64_t n, uint64_t *out, uint64_t
 void launch_validate(const DevGraph &g, uint32_t *deg, unsigned long long *stats,
                      cudaStream_t s);
 void launch_build_records(const DevGraph &g, uint4 *recs, cudaStream_t s);
-// Device layout (sector slots, device_common.cuh) of mode GT or LE: pass 0
-// decodes the on-disk stream into a CSR (rowptr = scanned degrees); pass 1
-// picks each vertex's chunk length, field widths and slots per sector (meta)
-// and first_pos (fpos); the host places the vertices (P, bit offsets); pass 2
-// writes the slots into dst (zeroed) and rewrites the records in place.
+// Device layout (sector slots, device_common.cuh): pass 0 decodes the on-disk
+// stream of mode GT or LE into a CSR (rowptr = scanned degrees); pass 1 picks
+// each vertex's chunk length, field widths and slots per sector (meta); the
+// host places the vertices (P, bit offsets); pass 2 writes the slots into dst
+// (zeroed) and rewrites the records in place.
 void launch_disk_decode(int mode, const uint32_t *words, const uint4 *recs, uint32_t n,
                         const uint64_t *rowptr, uint32_t *cols, cudaStream_t s);
-void launch_slot_choose(int mode, const uint64_t *rowptr, const uint32_t *cols, uint32_t n,
-                        uint32_t *meta, uint32_t *fpos, cudaStream_t s);
-void launch_slot_write(int mode, const uint64_t *rowptr, const uint32_t *cols, uint32_t n,
-                       const uint32_t *meta, const uint32_t *fpos, const uint64_t *P,
-                       uint32_t *dst, uint4 *recs, cudaStream_t s);
+void launch_slot_choose(const uint64_t *rowptr, const uint32_t *cols, uint32_t n, uint32_t *meta,
+                        cudaStream_t s);
+void launch_slot_write(const uint64_t *rowptr, const uint32_t *cols, uint32_t n,
+                       const uint32_t *meta, const uint64_t *P, uint32_t *dst, uint4 *recs,
+                       cudaStream_t s);
 void launch_degrees(const DevGraph &g, uint32_t *deg, cudaStream_t s);
-void launch_degrees64(const DevGraph &g, uint64_t *deg, cudaStream_t s);
-// In-place exclusive scan of vals[0..n) into vals[0..n]; tmp as above.
-void launch_scan_u64_inplace(uint64_t *vals, uint64_t n, uint64_t *tmp, cudaStream_t s);
+// Row pointers: the exclusive scan of the records' degrees into rowptr[0..n];
+// tmp as above.
+void launch_scan_degrees(const uint4 *recs, uint64_t n, uint64_t *rowptr, uint64_t *tmp,
+                         cudaStream_t s);
 
 // ---- decode (kernels_decode.cu) ----
 // E = rowptr[n] (the number of edges, known from load-time validation).

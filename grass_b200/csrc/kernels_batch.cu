@@ -16,23 +16,18 @@
 
 #include "batch.h"
 
-// Resident blocks per SM the compiler must allow for, per graph mode (the
-// register budget).  The batched-jobs workload waits on memory, so more
-// resident warps pay until spills cost more: measured on the 256-job mix,
-// LE is best at 3 (80 registers; 2x over 1), GT and CSR at 4 (64 registers).
-#ifndef GRASS_BATCH_MIN_BLOCKS_LE
-#define GRASS_BATCH_MIN_BLOCKS_LE 3
-#endif
-#ifndef GRASS_BATCH_MIN_BLOCKS_OTHER
-#define GRASS_BATCH_MIN_BLOCKS_OTHER 4
+// Resident blocks per SM the compiler must allow for (the register budget):
+// the batched-jobs workload waits on memory, so more resident warps pay until
+// spills cost more.
+#ifndef GRASS_BATCH_MIN_BLOCKS
+#define GRASS_BATCH_MIN_BLOCKS 4
 #endif
 
 namespace grass {
 namespace {
 
 template <int MODE, int DEPTH>
-__global__ void __launch_bounds__(256, MODE == 1 ? GRASS_BATCH_MIN_BLOCKS_LE
-                                               : GRASS_BATCH_MIN_BLOCKS_OTHER) batch_kernel(DevGraph g, const BatchJob *__restrict__ jobs,
+__global__ void __launch_bounds__(256, GRASS_BATCH_MIN_BLOCKS) batch_kernel(DevGraph g, const BatchJob *__restrict__ jobs,
                                                     const BatchTask *__restrict__ tasks,
                                                     uint32_t ncta, uint32_t ntasks,
                                                     unsigned int *queue,
@@ -40,7 +35,6 @@ __global__ void __launch_bounds__(256, MODE == 1 ? GRASS_BATCH_MIN_BLOCKS_LE
                                                     unsigned int *err) {
   __shared__ SmemHdr sh[8];
   __shared__ CtaSmem<8> csm;
-  __shared__ __align__(16) uint32_t dbuf[8][32 * kDrawBufWords];  // k-hop draw staging
   SmemHdr &my = sh[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   uint64_t all = 0;
@@ -85,8 +79,7 @@ __global__ void __launch_bounds__(256, MODE == 1 ? GRASS_BATCH_MIN_BLOCKS_LE
     } else if (jb.type == GRASS_JOB_KHOP) {
       const uint32_t parts = max(1u, tk.pad >> 8), part = tk.pad & 0xFFu;
       for (uint64_t s = tk.begin; s < tk.end; s++)
-        khop_seed_warp<MODE>(g, jb.in, jb.khop, s, my, dbuf[threadIdx.x >> 5], cnt, bad, part,
-                             parts);
+        khop_seed_warp<MODE>(g, jb.in, jb.khop, s, my, cnt, bad, part, parts);
     } else {
       for (uint64_t s = tk.begin; s < tk.end; s++) {
         if (jb.gen_roots) {
@@ -114,11 +107,13 @@ using BatchKernel = void (*)(DevGraph, const BatchJob *, const BatchTask *, uint
                              unsigned int *, unsigned long long *, unsigned int *);
 
 BatchKernel pick_kernel(int mode, uint32_t depth) {
-  if (mode == GRASS_MODE_GT)
-    return depth == 4 ? batch_kernel<0, 4> : depth == 2 ? batch_kernel<0, 2> : batch_kernel<0, 1>;
   if (mode == GRASS_MODE_CSR_INTERNAL)
-    return depth == 4 ? batch_kernel<2, 4> : depth == 2 ? batch_kernel<2, 2> : batch_kernel<2, 1>;
-  return depth == 4 ? batch_kernel<1, 4> : depth == 2 ? batch_kernel<1, 2> : batch_kernel<1, 1>;
+    return depth == 4   ? batch_kernel<kCsr, 4>
+           : depth == 2 ? batch_kernel<kCsr, 2>
+                        : batch_kernel<kCsr, 1>;
+  return depth == 4   ? batch_kernel<kSlots, 4>
+         : depth == 2 ? batch_kernel<kSlots, 2>
+                      : batch_kernel<kSlots, 1>;
 }
 
 grass_batch_config resolve(const grass_batch_config &c, int mode) {

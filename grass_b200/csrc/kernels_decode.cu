@@ -14,13 +14,9 @@
 //  2. for each round of 32 consecutive neighbors, loads the row ends and
 //     records of a window of 32 vertices (coalesced), maps every lane to its
 //     vertex by a shuffle binary search and takes the header by shuffle;
-//  3. decodes: LE -- each neighbor is two rocks and one signed sea
-//     (independent); GT -- each lane reads its own field (block head or gap)
-//     and a segmented warp scan turns gaps into ids, with the running value
-//     carried from round to round (and, at a task start inside a block,
-//     decoded once by lane 0);
+//  3. decodes each neighbor as one independent draw (its slot's head and one
+//     offset);
 //  4. writes its 32 ids with one coalesced store.
-#include <type_traits>
 #include <vector>
 
 #include "graph.h"
@@ -32,19 +28,9 @@ namespace {
 constexpr unsigned FULL = 0xFFFFFFFFu;
 constexpr uint32_t kTaskNeighbors = 2048;  // multiple of 32
 
-__device__ __forceinline__ VHdr shfl_hdr(const VHdr &h, int src) {
-  VHdr o;
-  o.P = __shfl_sync(FULL, h.P, src);
-  o.v = __shfl_sync(FULL, h.v, src);
-  o.d = __shfl_sync(FULL, h.d, src);
-  o.bn = __shfl_sync(FULL, h.bn, src);
-  o.bl = __shfl_sync(FULL, h.bl, src);
-  o.om = __shfl_sync(FULL, h.om, src);
-  o.fp = __shfl_sync(FULL, h.fp, src);
-  o.cx = __shfl_sync(FULL, h.cx, src);
-  o.a = __shfl_sync(FULL, h.a, src);
-  o.b = __shfl_sync(FULL, h.b, src);
-  return o;
+__device__ __forceinline__ uint4 shfl_rec(const uint4 &r, int src) {
+  return make_uint4(__shfl_sync(FULL, r.x, src), __shfl_sync(FULL, r.y, src),
+                    __shfl_sync(FULL, r.z, src), __shfl_sync(FULL, r.w, src));
 }
 
 // Largest v in [0, n) with rowptr[v] <= x, for x < rowptr[n].
@@ -75,7 +61,6 @@ __device__ __forceinline__ uint32_t row_of_serial(const uint64_t *rowptr, uint32
   return lo;
 }
 
-template <int MODE>
 __global__ void __launch_bounds__(256) decode_all_kernel(DevGraph g, const uint64_t *rowptr,
                                                            uint32_t *cols, uint64_t E,
                                                            unsigned int *err) {
@@ -113,7 +98,7 @@ __global__ void __launch_bounds__(256) decode_all_kernel(DevGraph g, const uint6
         // Fast path: the round lies inside vertex vr (most rounds of a
         // skewed graph): no window, no owner search.
         if (!ch_ok) {
-          ch = header<MODE>(g, vr);
+          ch = header<kSlots>(g, vr);
           ch_ok = true;
         }
         hk = ch;
@@ -123,12 +108,7 @@ __global__ void __launch_bounds__(256) decode_all_kernel(DevGraph g, const uint6
         const uint32_t wv = vr + lane;
         const uint64_t base = rowptr[vr];
         const uint64_t e = wv < g.n ? rowptr[wv + 1] : ~0ull;
-        VHdr hw;
-        if (wv < g.n) {
-          hw = header<MODE>(g, wv);
-        } else {
-          hw.d = 0; hw.P = 0; hw.v = 0; hw.bn = hw.bl = hw.om = hw.fp = 0; hw.a = hw.b = hw.cx = 0;
-        }
+        const uint4 rw = wv < g.n ? load_record(g.recs + wv) : make_uint4(0u, 0u, 0u, 0u);
         // owner lane k: number of window rows that end at or before gl
         // (binary lifting over 31 probes gives the exact count when it is
         // below 32)
@@ -143,16 +123,16 @@ __global__ void __launch_bounds__(256) decode_all_kernel(DevGraph g, const uint6
         far = act && e31 <= gl;
         const int src = far ? 0 : k;
         const uint64_t prev_e = __shfl_sync(FULL, e, src > 0 ? src - 1 : 0);
-        hk = shfl_hdr(hw, src);
+        hk = record_header<kSlots>(shfl_rec(rw, src));
         startv = src == 0 ? base : prev_e;
         if (far) {
           const uint32_t v = row_of_serial(rowptr, vr + 32, g.n, gl);
-          hk = header<MODE>(g, v);
+          hk = header<kSlots>(g, v);
           startv = rowptr[v];
         }
       }
       // each neighbor is one independent draw of one sector slot
-      const uint32_t val = act ? neighbor<MODE>(g, hk, (uint32_t)(gl - startv)) : 0u;
+      const uint32_t val = act ? neighbor<kSlots>(g, hk, (uint32_t)(gl - startv)) : 0u;
       if (act) {
         if (val >= g.n) bad = true;
         cols[gl] = val;
@@ -186,71 +166,33 @@ constexpr uint32_t kBigDegree = 32;
 #endif
 constexpr uint32_t kRange = GRASS_DECODE_RANGE;  // neighbors per range item
 
-// Sequential decoders of one vertex (one lane each), from neighbor 0.
-struct LeSeq {
+// Sequential decoder of one vertex (one lane), from neighbor 0.
+struct SlotSeq {
   const uint32_t *w;
   VHdr h;
-  uint32_t c, id, L;  // chunk, index in it, its length
-  uint32_t off;       // bit offset of the chunk's slot in sector A
+  uint32_t c, id;  // slot, index in it
+  DrawAt at;
   Sec A;
 
-  __device__ __forceinline__ void load_chunk() {
-    const uint64_t pos = slot_pos(h, c);
-    A = load_sector(w, pos >> 8);
-    off = (uint32_t)pos & 255u;
-    L = min(h.bl, h.d - 1 - c * h.bl);
+  __device__ __forceinline__ void load_slot() {
+    at = slot_at(h, c);
+    A = load_sector(w, at.sec);
   }
   __device__ __forceinline__ void init(const uint32_t *words, const VHdr &hd) {
     w = words;
     h = hd;
     c = id = 0;
-    if (h.d > 1) load_chunk();
+    if (h.cb) load_slot();
   }
   __device__ __forceinline__ uint32_t next() {
-    if (h.d == 1) return h.fp;
-    const uint32_t val = le_slot_value(A, off, h, c, id, L);
-    if (++id == L && c + 1 < h.bn) {  // the next chunk's left rock is this one's right rock
+    if (h.cb == 0) return h.base;
+    if (id == h.T) {
       c++;
       id = 0;
-      load_chunk();
+      load_slot();
     }
-    return val;
-  }
-};
-
-struct GtSeq {
-  const uint32_t *w;
-  VHdr h;
-  uint32_t c, id, L;  // slot, index in it, its length
-  uint32_t off, x;    // bit offset of the slot in sector A; the previous value
-  Sec A;
-
-  __device__ __forceinline__ void load_chunk() {
-    const uint64_t pos = slot_pos(h, c);
-    A = load_sector(w, pos >> 8);
-    off = (uint32_t)pos & 255u;
-    L = min(h.bl, h.d - c * h.bl);
-  }
-  __device__ __forceinline__ void init(const uint32_t *words, const VHdr &hd) {
-    w = words;
-    h = hd;
-    c = id = 0;
-    if (h.d) load_chunk();
-  }
-  __device__ __forceinline__ uint32_t next() {
-    if (id == 0) {
-      const uint32_t hv = (uint32_t)sec1_field(A, off, h.a) + 1u;
-      x = c >= h.fp ? h.v + hv : h.v - hv;
-    } else {
-      x += (h.b ? (uint32_t)sec1_field(A, off + (uint32_t)h.a + (id - 1) * (uint32_t)h.b, h.b)
-                : 0u) + 1u;
-    }
-    if (++id == L && c + 1 < h.bn) {
-      c++;
-      id = 0;
-      load_chunk();
-    }
-    return x;
+    at.id = id++;
+    return draw_value(A, at, h);
   }
 };
 
@@ -351,7 +293,7 @@ __global__ void plan_fill_kernel(const uint4 *__restrict__ recs, uint32_t n, uin
 constexpr int kDecodeWarps = 8;          // warps per range block
 constexpr uint32_t kGroupBytes = 1056;   // 32 slots lie in at most 32 sectors; + one
                                          // sector that field reads may touch
-constexpr uint32_t kOutWords = 32 * 33;  // a group's neighbors (32 chunks of <= 32, + 1)
+constexpr uint32_t kOutWords = 32 * 32;  // a group's neighbors (32 slots of <= 32)
 // Polls of the copy's mbarrier before the warp gives up (far beyond the
 // microseconds one copy takes).
 #ifndef GRASS_STAGE_POLLS
@@ -412,7 +354,7 @@ __device__ __forceinline__ bool stage_wait(uint64_t *bar, uint32_t parity) {
 struct RangeMeta {
   uint4 rec[32];
   uint64_t base[32];
-  uint32_t v[32], i0[32], i1[32];
+  uint32_t i0[32], i1[32];
 };
 
 // Shared memory of one range warp, in a block of its own that starts on a
@@ -430,7 +372,7 @@ struct WarpSmem {
 static_assert(kGroupBytes % 16 == 0 && (kOutWords * 4) % 16 == 0 && sizeof(RangeMeta) % 16 == 0,
               "staging alignment");
 
-// Range sweep on the device layout (GT or LE): one lane per chunk slot.  A
+// Range sweep: one lane per chunk slot.  A
 // warp takes 32 range items at a time: lane k loads item k's record and row
 // start, and a scan over the lanes numbers the items' groups of 32 slots
 // 0 .. total-1 in item order.  The warp then walks that sequence: each lane
@@ -440,7 +382,7 @@ static_assert(kGroupBytes % 16 == 0 && (kOutWords * 4) % 16 == 0 && sizeof(Range
 // each group's sectors in shared memory DEPTH - 1 groups ahead (across item
 // boundaries, see above).  Measured on R-MAT s22 ef32, the unstaged sweep is
 // the fastest: 7 % (LE) and 23 % (GT) faster than staging at depth 1.
-template <int MODE, int DEPTH>
+template <int DEPTH>
 __global__ void __launch_bounds__(256) decode_range_kernel(DevGraph g, const uint64_t *rowptr,
                                                            uint32_t *cols,
                                                            const uint4 *__restrict__ items,
@@ -470,17 +412,14 @@ __global__ void __launch_bounds__(256) decode_range_kernel(DevGraph g, const uin
     uint32_t c0 = 0, c1 = 0, ng = 0;
     if (t < nitems) {
       const uint4 it = items[t];
-      const uint4 r = graph_record<MODE>(g, it.x);
-      const VHdr h = record_header<MODE>(r, it.x);
+      const uint4 r = load_record(g.recs + it.x);
+      const VHdr h = record_header<kSlots>(r);
       m.rec[lane] = r;
-      m.v[lane] = it.x;
       m.base[lane] = rowptr[it.x];
       m.i0[lane] = it.y;
       m.i1[lane] = it.z;
-      // slot of neighbor i: i / T (LE: the last neighbor is slot C-1's right rock)
-      const uint32_t last = h.d - 1;
-      c0 = MODE == 0 || it.y < last ? div_small(it.y, h.bl) : h.bn - 1;
-      c1 = MODE == 0 || it.z - 1 < last ? div_small(it.z - 1, h.bl) : h.bn - 1;
+      c0 = div_small(it.y, h.T);
+      c1 = div_small(it.z - 1, h.T);
       ng = (c1 - c0) / 32 + 1;
     }
     uint32_t incl = ng;
@@ -501,10 +440,10 @@ __global__ void __launch_bounds__(256) decode_range_kernel(DevGraph g, const uin
       const int k = item_of(s);
       const uint32_t j = s - __shfl_sync(FULL, excl, k);
       const uint32_t kc0 = __shfl_sync(FULL, c0, k), kc1 = __shfl_sync(FULL, c1, k);
-      const VHdr hk = record_header<MODE>(m.rec[k], m.v[k]);
+      const VHdr hk = record_header<kSlots>(m.rec[k]);
       const uint32_t ca = kc0 + 32 * j, cz = min(kc1, ca + 31);
-      qa = slot_pos(hk, ca) >> 8;
-      qb = slot_pos(hk, cz) >> 8;
+      qa = slot_at(hk, ca).sec;
+      qb = slot_at(hk, cz).sec;
     };
     auto issue = [&](uint32_t s) {
       if (DEPTH == 0 || !stage_ok) return;
@@ -527,7 +466,7 @@ __global__ void __launch_bounds__(256) decode_range_kernel(DevGraph g, const uin
       const int k = item_of(s);
       if (k != kcur) {  // the next item: its header and range from the metadata
         kcur = k;
-        h = record_header<MODE>(m.rec[k], m.v[k]);
+        h = record_header<kSlots>(m.rec[k]);
         base = m.base[k];
         i0 = m.i0[k];
         i1 = m.i1[k];
@@ -535,7 +474,7 @@ __global__ void __launch_bounds__(256) decode_range_kernel(DevGraph g, const uin
         kc1 = __shfl_sync(FULL, c1, k);
         kex = __shfl_sync(FULL, excl, k);
       }
-      const uint32_t T = h.bl, last = h.d - 1, j = s - kex;
+      const uint32_t T = h.T, j = s - kex;
       bool staged = false;
       const uint32_t b = s % D;
       if (DEPTH > 0 && stage_ok) {
@@ -550,25 +489,20 @@ __global__ void __launch_bounds__(256) decode_range_kernel(DevGraph g, const uin
       }
       const uint32_t cg = kc0 + 32 * j, c = cg + lane;
       if (c <= kc1) {
-        const uint64_t pos = slot_pos(h, c);
+        const DrawAt at = slot_at(h, c);
         // the slot's sector as words: from the staged group, or (after a
         // timeout) from global memory
         const uint32_t *w;
         if (staged) {
-          const uint64_t qa = slot_pos(h, cg) >> 8;
-          w = reinterpret_cast<const uint32_t *>(stage + b * kGroupBytes + ((pos >> 8) - qa) * 32u);
+          const uint32_t qa = slot_at(h, cg).sec;
+          w = reinterpret_cast<const uint32_t *>(stage + b * kGroupBytes + (at.sec - qa) * 32u);
         } else {
-          w = g.words + (pos >> 8) * 8;
+          w = g.words + (uint64_t)at.sec * 8;
         }
-        if constexpr (MODE == 0) {
-          gt_slot_decode_w(w, (uint32_t)pos & 255u, h, c, min(T, h.d - c * T), out + (c - cg) * T);
-        } else {  // the last chunk also holds neighbor d-1, its right rock
-          le_slot_decode_w(w, (uint32_t)pos & 255u, h, c, min(T, last - c * T), c + 1 == h.bn,
-                           out + (c - cg) * T);
-        }
+        slot_decode_w(w, at.off, h, min(T, h.d - c * T), out + (c - cg) * T);
       }
       __syncwarp();
-      const uint32_t nb0 = cg * T, nhi = cg + 32 >= h.bn ? h.d : (cg + 32) * T;
+      const uint32_t nb0 = cg * T, nhi = min(h.d, (cg + 32) * T);
       const uint32_t lo = max(i0, nb0), hi = min(i1, nhi);
       for (uint32_t q = lo + lane; q < hi; q += 32) {
         const uint32_t val = out[q - nb0];
@@ -587,37 +521,98 @@ __global__ void __launch_bounds__(256) decode_range_kernel(DevGraph g, const uin
 
 // ---- the flat sweep (the default) ----
 // A warp takes one item of the flat plan: a run of consecutive vertices
-// [v0, v1) (i1 == 0), or one vertex's neighbor range [i0, i1) (hubs, degree
-// >= kRange).  The item's output is one contiguous stretch of the CSR, and
-// its chunk slots, taken in vertex order, fill it in order.  So the warp
-// walks the item 32 vertices at a time (lane k loads vertex k's record and
-// counts its slots), numbers their slots by a warp scan, and decodes them 32
-// at a time, one slot per lane, whatever vertex each belongs to: a group of
-// 32 slots is a contiguous stretch of at most 32 * 33 neighbors, decoded into
-// shared memory and written with coalesced stores.  A lane reads its slot's
-// fields as 32-bit words from global memory through L1 (one funnel shift per
-// field); measured faster than loading the sector into registers and reading
-// the fields in order from there (LE 1.00 against 1.04 ms, GT 1.16 against
-// 1.43 ms on R-MAT s22 ef32).  LE vertices of degree 1 count as one slot (the
-// neighbor is in the record).
+// [v0, v1) (w == 0), or one vertex's neighbor range [z, w) (hubs, degree >=
+// kFlatHub).  It walks a run 32 vertices at a time (lane k loads vertex k's
+// record) and decodes one neighbor per lane, straight to the CSR:
+//  * vertices of degree >= 32 one after another (flat_big): everything but
+//    the lane's place in the slots is warp-uniform, and that place advances by
+//    a constant from one round of 32 neighbors to the next;
+//  * the other vertices together: their neighbors are numbered by a warp scan,
+//    and in a round of 32 each lane finds its vertex from the bit mask of the
+//    vertices that start in the round (one OR-reduction and a population
+//    count).
+// A neighbor is n_0 + head + offset, two fields of one slot, so lanes need
+// nothing from one another.  R-MAT s21 ef16, 63 M neighbors: 0.259 ms a sweep;
+// one lane per slot took 0.466 ms on this layout (slots of 3 neighbors leave
+// most of the work to per-slot set-up) and 0.340 ms on LE's own code.
 constexpr uint32_t kFlatHub = kRange;  // degree from which a vertex is split into ranges
+constexpr uint32_t kFlatBig = 32;      // degree from which a vertex is decoded by itself
 
-// Resident 256-thread blocks per SM: 4 (64 registers, no spill; 4 x 33 KB of
-// shared memory).  Unbounded, the LE kernel took 80 registers (3 blocks) and
-// ran 1.08 ms against 0.94 ms at 4 (GT: 74 registers, 1.43 against 1.17 ms)
-// on R-MAT s22 ef32.
+// Resident 256-thread blocks per SM.
 #ifndef GRASS_DECODE_FLAT_MIN_BLOCKS
 #define GRASS_DECODE_FLAT_MIN_BLOCKS 4
 #endif
 
+// A warp's share of shared memory.
+struct FlatSmem {
+  uint32_t stage[32 * 8 + 4];  // 32 sectors, and the word that a field's read may touch
+  uint4 rec[32];               // the round's small vertices with neighbors, in order:
+  uint64_t ob[32];             // record, first entry in the CSR,
+  uint32_t ex[32];             // number of the first neighbor in the group
+};
+
+// The field of `width` (0..32) bits at bit `off` from word w.
+__device__ __forceinline__ uint32_t word_field(const uint32_t *w, uint32_t off, uint32_t width) {
+  const uint32_t *q = w + (off >> 5);
+  return shr_clamp(__funnelshift_l(q[1], q[0], off), 32u - width);
+}
+
+// Neighbors [i0, i1) of a vertex of header h (warp-uniform, cb > 0) to
+// out[i0 .. i1).  The vertex's sectors are consecutive, so the warp copies 32
+// at a time into shared memory with two 16-byte loads a lane, the next 32
+// already on their way in registers, and reads the fields from there.
+__device__ __forceinline__ void flat_big(const uint32_t *words, const VHdr &h, uint32_t i0,
+                                         uint32_t i1, uint32_t n, uint32_t *out, uint32_t *stage,
+                                         bool &bad) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t T = h.T, K = h.K, N = T * K;  // N neighbors a sector
+  const uint32_t q0 = div_small(div_small(i0, T), K);
+  const uint32_t nq = div_small(div_small(i1 - 1, T), K) - q0 + 1;
+  // the lane's place in a chunk of sectors, and its advance per round
+  const uint32_t dT = div_small(32u, T), rT = 32u - dT * T, dK = div_small(dT, K), rK = dT - dK * K;
+  const uint32_t c0 = div_small(lane, T), id0 = lane - c0 * T;
+  const uint32_t k0 = div_small(c0, K), s0 = c0 - k0 * K;
+  const uint4 *src = reinterpret_cast<const uint4 *>(words + (uint64_t)(h.sec + q0) * 8) + lane;
+  uint4 *dst = reinterpret_cast<uint4 *>(stage) + lane;
+  const uint32_t half = lane >> 1;  // the lane's sector of 16
+  uint4 x = make_uint4(0, 0, 0, 0), y = x;
+  if (half < nq) x = __ldg(src);
+  if (half + 16 < nq) y = __ldg(src + 32);
+  for (uint32_t q = 0; q < nq; q += 32) {  // warp-uniform
+    dst[0] = x;
+    dst[32] = y;
+    __syncwarp();
+    src += 64;
+    if (q + 32 + half < nq) x = __ldg(src);
+    if (q + 48 + half < nq) y = __ldg(src + 32);
+    const uint32_t j0 = (q0 + q) * N, j1 = min(i1, j0 + 32u * N);
+    uint32_t k = k0, s = s0, id = id0;
+    for (uint32_t i = j0 + lane; i < j1; i += 32) {
+      const uint32_t *w = stage + k * 8;
+      const uint32_t at = h.off + s * h.cb;
+      uint32_t v = h.base + word_field(w, at, h.a);
+      if (T > 1) v += word_field(w, id ? at + h.a + (id - 1) * h.b : at, id ? h.b : 0u);
+      bad |= v >= n;
+      if (i >= i0) out[i] = v;
+      id += rT;
+      s += rK;
+      k += dK;
+      if (id >= T) id -= T, s++;
+      if (s >= K) s -= K, k++;
+    }
+    __syncwarp();
+  }
+}
+
 template <int MODE>
-__global__ void __launch_bounds__(256, GRASS_DECODE_FLAT_MIN_BLOCKS) decode_flat_kernel(DevGraph g, const uint64_t *rowptr,
-                                                          uint32_t *cols,
+__global__ void __launch_bounds__(256, GRASS_DECODE_FLAT_MIN_BLOCKS) decode_flat_kernel(DevGraph g, const uint64_t *__restrict__ rowptr,
+                                                          uint32_t *__restrict__ cols,
                                                           const uint4 *__restrict__ items,
                                                           uint64_t nitems, unsigned int *err) {
-  __shared__ __align__(16) uint32_t out_all[8][kOutWords];
-  uint32_t *out = out_all[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31;
+  __shared__ __align__(16) FlatSmem smem[8];
+  FlatSmem &sm = smem[threadIdx.x >> 5];
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t upto = 0xFFFFFFFFu >> (31 - lane);  // this lane and those below
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   bool bad = false;
@@ -626,85 +621,59 @@ __global__ void __launch_bounds__(256, GRASS_DECODE_FLAT_MIN_BLOCKS) decode_flat
     const bool run = it.w == 0;
     const uint32_t v0 = it.x, v1 = run ? it.y : it.x + 1;
     for (uint32_t vb = v0; vb < v1; vb += 32) {
-      // lane k: vertex vb + k, its slots [c0, c0 + ns) and first output position
       const uint32_t v = vb + lane;
-      const bool vok = v < v1;
       uint4 r = make_uint4(0, 0, 0, 0);
-      uint32_t c0 = 0, ns = 0;
-      uint64_t ob = 0;  // output position of the vertex's slot c0's first neighbor
-      if (vok) {
+      uint64_t ob = 0;
+      if (v < v1) {
         r = graph_record<MODE>(g, v);
-        const VHdr h = record_header<MODE>(r, v);
-        const uint32_t i0 = run ? 0u : it.z, i1 = run ? h.d : it.w;
-        if (MODE == 1 && h.d == 1) {
-          ns = 1;
-        } else if (h.d) {
-          const uint32_t last = h.d - 1;
-          c0 = MODE == 0 || i0 < last ? div_small(i0, h.bl) : h.bn - 1;
-          const uint32_t c1 = MODE == 0 || i1 - 1 < last ? div_small(i1 - 1, h.bl) : h.bn - 1;
-          ns = c1 - c0 + 1;
-        }
-        ob = rowptr[v] + (uint64_t)c0 * h.bl;
+        ob = rowptr[v];
       }
-      uint32_t sincl = ns;
+      const bool big = r.z >= kFlatBig;
+      // the small vertices of the group
+      const uint32_t d = big ? 0u : r.z;
+      uint32_t incl = d;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(FULL, sincl, o);
-        if (lane >= o) sincl += y;
+        const uint32_t y = __shfl_up_sync(FULL, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
       }
-      const uint32_t sexcl = sincl - ns, stot = __shfl_sync(FULL, sincl, 31);
-      // the item's stored stretch: [lo, hi) of the CSR
-      const uint64_t v_lo = run ? __shfl_sync(FULL, ob, 0) : rowptr[v0] + it.z;
-      const uint64_t v_hi = run ? rowptr[min(v1, vb + 32)] : rowptr[v0] + it.w;
-      for (uint32_t sg = 0; sg < stot; sg += 32) {  // warp-uniform
-        const uint32_t sl = sg + lane;
-        // the lane's vertex: the last k with sexcl_k <= sl
-        int k = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1) {
-          const uint32_t e = __shfl_sync(FULL, sexcl, k + step);
-          if (k + step < 32 && e <= sl) k += step;
-        }
-        const uint32_t kx = __shfl_sync(FULL, r.x, k), ky = __shfl_sync(FULL, r.y, k);
-        const uint32_t kz = __shfl_sync(FULL, r.z, k), kw = __shfl_sync(FULL, r.w, k);
-        const uint32_t kc0 = __shfl_sync(FULL, c0, k), kse = __shfl_sync(FULL, sexcl, k);
-        const uint64_t kob = __shfl_sync(FULL, ob, k);
-        const bool act = sl < stot;
-        const VHdr h = record_header<MODE>(make_uint4(kx, ky, kz, kw), vb + (uint32_t)k);
-        const uint32_t c = kc0 + (sl - kse);
-        const uint64_t pos0 = kob + (uint64_t)(sl - kse) * h.bl;  // slot's first output position
-        const uint64_t g_lo = __shfl_sync(FULL, pos0, 0);
-        // the slot's neighbors: GT min(T, d - cT); LE min(T, d-1-cT) (+ the right
-        // rock in the last slot); LE degree 1: the record's neighbor
-        uint32_t len = 0;
-        if (act) {
-          if (MODE == 1 && h.d == 1) {
-            len = 1;
-            out[pos0 - g_lo] = h.fp;
-          } else {
-            const uint64_t p = slot_pos(h, c);
-            const uint32_t *w = g.words + (p >> 8) * 8;
-            if constexpr (MODE == 0) {
-              len = min(h.bl, h.d - c * h.bl);
-              gt_slot_decode_w(w, (uint32_t)p & 255u, h, c, len, out + (pos0 - g_lo));
-            } else {
-              const uint32_t L = min(h.bl, h.d - 1 - c * h.bl);
-              const bool right = c + 1 == h.bn;
-              le_slot_decode_w(w, (uint32_t)p & 255u, h, c, L, right, out + (pos0 - g_lo));
-              len = L + (right ? 1u : 0u);
-            }
+      const uint32_t ex = incl - d, total = __shfl_sync(FULL, incl, 31);
+      const unsigned has = __ballot_sync(FULL, d > 0);
+      if (d) {
+        const uint32_t at = __popc(has & upto) - 1;
+        sm.rec[at] = r;
+        sm.ob[at] = ob;
+        sm.ex[at] = ex;
+      }
+      __syncwarp();
+      uint32_t before = 0;  // vertices that start before the round
+      for (uint32_t j = 0; j < total; j += 32) {
+        const unsigned starts =
+            __reduce_or_sync(FULL, d && ex >= j && ex < j + 32 ? 1u << (ex - j) : 0u);
+        const uint32_t own = before + __popc(starts & upto) - 1;
+        before += __popc(starts);
+        if (j + lane < total) {
+          const VHdr h = record_header<MODE>(sm.rec[own]);
+          const uint32_t i = j + lane - sm.ex[own];
+          uint32_t x = h.base;
+          if (h.cb) {
+            const DrawAt at = draw_at(h, i);
+            const uint32_t *w = g.words + (uint64_t)at.sec * 8;
+            if (h.a) x += word_field(w, at.off, h.a);
+            if (at.id) x += word_field(w, at.off + h.a + (at.id - 1) * h.b, h.b);
           }
+          bad |= x >= g.n;
+          cols[sm.ob[own] + i] = x;
         }
-        const uint64_t g_hi = __reduce_max_sync(FULL, act ? (uint32_t)(pos0 - g_lo) + len : 0u) + g_lo;
-        __syncwarp();
-        const uint64_t lo = max(g_lo, v_lo), hi = min(g_hi, v_hi);
-        for (uint64_t q = lo + lane; q < hi; q += 32) {
-          const uint32_t val = out[q - g_lo];
-          bad |= val >= g.n;
-          cols[q] = val;
-        }
-        __syncwarp();  // the group's buffer is free for the next group
       }
+      // the large ones
+      for (unsigned m = __ballot_sync(FULL, big); m; m &= m - 1) {
+        const int k = __ffs(m) - 1;
+        const VHdr h = record_header<MODE>(shfl_rec(r, k));
+        uint32_t *out = cols + __shfl_sync(FULL, ob, k);
+        flat_big(g.words, h, run ? 0u : it.z, run ? h.d : it.w, g.n, out, sm.stage, bad);
+      }
+      __syncwarp();  // the group's shared memory is free
     }
   }
   if (bad && err) atomicOr(err, 1u);
@@ -779,7 +748,6 @@ __global__ void flat_plan_link_kernel(uint4 *items, uint64_t nitems, uint32_t n)
   if (items[k].w == 0) items[k].y = k + 1 < nitems ? items[k + 1].x : n;
 }
 
-template <int MODE>
 __global__ void __launch_bounds__(256) decode_small_kernel(DevGraph g, const uint64_t *rowptr,
                                                              uint32_t *cols,
                                                              const uint32_t *__restrict__ verts,
@@ -790,10 +758,10 @@ __global__ void __launch_bounds__(256) decode_small_kernel(DevGraph g, const uin
     const uint64_t q = q0 + threadIdx.x;
     uint32_t d = 0;
     uint32_t *out = nullptr;
-    std::conditional_t<MODE == 0, GtSeq, LeSeq> st;
+    SlotSeq st;
     if (q < nv) {
       const uint32_t v = verts[q];
-      const VHdr h = header<MODE>(g, v);
+      const VHdr h = header<kSlots>(g, v);
       d = h.d;
       out = cols + rowptr[v];
       st.init(g.words, h);
@@ -812,28 +780,27 @@ __global__ void __launch_bounds__(256) decode_small_kernel(DevGraph g, const uin
 static void launch_plan_kernels(const grass_graph *g, const uint64_t *rowptr, uint32_t *cols,
                                 unsigned int *err, cudaStream_t s);
 
-template <int MODE, int DEPTH>
+template <int DEPTH>
 static void launch_range(const DevGraph &v, const uint64_t *rowptr, uint32_t *cols,
                          const grass_graph *g, unsigned grid, unsigned int *err, cudaStream_t s) {
   const uint32_t smem = kDecodeWarps * WarpSmem<DEPTH>::bytes();
   static std::once_flag once;  // opt in to more than 48 KB of dynamic shared memory
   std::call_once(once, [&] {
-    cudaFuncSetAttribute(decode_range_kernel<MODE, DEPTH>,
+    cudaFuncSetAttribute(decode_range_kernel<DEPTH>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
-  decode_range_kernel<MODE, DEPTH><<<grid, 32 * kDecodeWarps, smem, s>>>(
+  decode_range_kernel<DEPTH><<<grid, 32 * kDecodeWarps, smem, s>>>(
       v, rowptr, cols, g->d_plan_big, g->plan_nbig, err);
 }
 
-template <int MODE>
 static void launch_range_depth(const DevGraph &v, const uint64_t *rowptr, uint32_t *cols,
                                const grass_graph *g, unsigned grid, unsigned int *err,
                                cudaStream_t s) {
   switch (g->tuning.decode_stage_depth) {
-    case 1: launch_range<MODE, 1>(v, rowptr, cols, g, grid, err, s); break;
-    case 2: launch_range<MODE, 2>(v, rowptr, cols, g, grid, err, s); break;
-    case 4: launch_range<MODE, 4>(v, rowptr, cols, g, grid, err, s); break;
-    default: launch_range<MODE, 0>(v, rowptr, cols, g, grid, err, s);  // unstaged
+    case 1: launch_range<1>(v, rowptr, cols, g, grid, err, s); break;
+    case 2: launch_range<2>(v, rowptr, cols, g, grid, err, s); break;
+    case 4: launch_range<4>(v, rowptr, cols, g, grid, err, s); break;
+    default: launch_range<0>(v, rowptr, cols, g, grid, err, s);  // unstaged
   }
 }
 
@@ -893,10 +860,7 @@ static void launch_flat(const grass_graph *g, const uint64_t *rowptr, uint32_t *
   const DevGraph v = g->view();
   const unsigned grid = (unsigned)std::max<uint64_t>(
       1, std::min<uint64_t>((g->plan_nflat + 7) / 8, (uint64_t)sm_count(g->device) * 8));
-  if (g->mode == GRASS_MODE_GT)
-    decode_flat_kernel<0><<<grid, 256, 0, s>>>(v, rowptr, cols, g->d_plan_flat, g->plan_nflat, err);
-  else
-    decode_flat_kernel<1><<<grid, 256, 0, s>>>(v, rowptr, cols, g->d_plan_flat, g->plan_nflat, err);
+  decode_flat_kernel<kSlots><<<grid, 256, 0, s>>>(v, rowptr, cols, g->d_plan_flat, g->plan_nflat, err);
   count_launch();
 }
 
@@ -997,18 +961,13 @@ static void launch_plan_kernels(const grass_graph *g, const uint64_t *rowptr, ui
   if (g->plan_nbig) {
     const unsigned grid = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>((g->plan_nbig + 7) / 8, (uint64_t)sm_count(dev) * per_sm));
-    if (g->mode == GRASS_MODE_GT) launch_range_depth<0>(v, rowptr, cols, g, grid, err, s);
-    else launch_range_depth<1>(v, rowptr, cols, g, grid, err, s);
+    launch_range_depth(v, rowptr, cols, g, grid, err, s);
     count_launch();
   }
   if (g->plan_nsmall) {
     const unsigned grid = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>((g->plan_nsmall + 255) / 256, (uint64_t)sm_count(dev) * per_sm));
-    if (g->mode == GRASS_MODE_GT)
-      decode_small_kernel<0><<<grid, 256, 0, s>>>(v, rowptr, cols, g->d_plan_small,
-                                                  g->plan_nsmall, err);
-    else
-      decode_small_kernel<1><<<grid, 256, 0, s>>>(v, rowptr, cols, g->d_plan_small,
+    decode_small_kernel<<<grid, 256, 0, s>>>(v, rowptr, cols, g->d_plan_small,
                                                   g->plan_nsmall, err);
     count_launch();
   }
@@ -1023,10 +982,7 @@ void launch_decode_all(const DevGraph &g, const uint64_t *rowptr, uint32_t *cols
   const uint64_t blocks_needed = (tasks + 7) / 8;
   const unsigned grid = (unsigned)std::max<uint64_t>(
       1, std::min<uint64_t>(blocks_needed, (uint64_t)sm_count(dev) * 8));
-  if (g.mode == GRASS_MODE_GT)
-    decode_all_kernel<0><<<grid, 256, 0, s>>>(g, rowptr, cols, E, err);
-  else
-    decode_all_kernel<1><<<grid, 256, 0, s>>>(g, rowptr, cols, E, err);
+  decode_all_kernel<<<grid, 256, 0, s>>>(g, rowptr, cols, E, err);
   count_launch();
 }
 

@@ -47,16 +47,14 @@ struct FieldLoader {  // n ubl-bit big-endian fields, ubl in [1, 64]
   }
 };
 
+struct DegreeLoader {  // degrees from the vertex records
+  const uint4 *recs;
+  __device__ __forceinline__ uint64_t operator()(uint64_t u) const { return __ldg(&recs[u].z); }
+};
+
 struct CountLoader {
   const uint32_t *counts;
   __device__ __forceinline__ uint64_t operator()(uint64_t u) const { return counts[u]; }
-};
-
-// Reads u64 values that tile_scan may overwrite in place: every CTA reads its
-// whole tile before its block scan and writes only after it.
-struct U64Loader {
-  const uint64_t *vals;
-  __device__ __forceinline__ uint64_t operator()(uint64_t u) const { return vals[u]; }
 };
 
 template <class Loader>
@@ -151,7 +149,7 @@ __global__ void validate_kernel(DevGraph g, uint32_t *deg, unsigned long long *s
     uint64_t end = 0;
     if (MODE == 0) {
       uint32_t hb = c.gamma(), bb = c.gamma(), fp = c.gamma();
-      VHdr h = gt_header(g, (uint32_t)v);
+      DiskHdr h = gt_header(g, (uint32_t)v);
       ok = hb >= (d ? 1u : 0u) && hb <= 32 && bb <= 32 && fp <= h.bn + 1 && d < 0x7FFFFFFFu;
       end = ok ? payload_end<0>(g, h) : 0;
     } else {
@@ -163,7 +161,7 @@ __global__ void validate_kernel(DevGraph g, uint32_t *deg, unsigned long long *s
         end = c.pos(g.words);
       } else {
         uint32_t rb = c.gamma(), sb = c.gamma(), fp = c.gamma();
-        VHdr h = le_header(g, (uint32_t)v);
+        DiskHdr h = le_header(g, (uint32_t)v);
         ok = rb >= 1 && rb <= 32 && sb <= 32 && fp <= h.bn + 2 && d < 0x7FFFFFFFu;
         end = ok ? payload_end<1>(g, h) : 0;
       }
@@ -188,11 +186,10 @@ __global__ void validate_kernel(DevGraph g, uint32_t *deg, unsigned long long *s
   }
 }
 
-template <int MODE, class T>
-__global__ void degrees_kernel(DevGraph g, T *deg) {
+__global__ void degrees_kernel(DevGraph g, uint32_t *deg) {
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < g.n;
        v += (uint64_t)gridDim.x * blockDim.x)
-    deg[v] = (T)record_degree(g, (uint32_t)v);
+    deg[v] = record_degree(g, (uint32_t)v);
 }
 
 // One record per vertex from its stream header (run once, after validation).
@@ -223,11 +220,11 @@ __device__ __forceinline__ void or_bits(uint32_t *w, uint64_t off, uint64_t val,
   if (lo) atomicOr(w + (off >> 5) + 1, lo);
 }
 
-// ---- LE device layout (sector slots, device_common.cuh) ----
+// ---- device layout (sector slots, device_common.cuh) ----
 
 // Neighbor i of an LE vertex in the on-disk layout: rocks at P + c a, seas at
 // P + (chunk_num + 1) a + k (sea_bit + 1) (LE/src/bcg.cuh:195-261).
-__device__ __forceinline__ uint32_t le_disk_neighbor(const uint32_t *words, const VHdr &h,
+__device__ __forceinline__ uint32_t le_disk_neighbor(const uint32_t *words, const DiskHdr &h,
                                                      uint32_t i) {
   if (h.d == 1) return h.fp;
   uint32_t tl = h.bl + 1;
@@ -261,118 +258,11 @@ __global__ void __launch_bounds__(256) le_disk_decode_kernel(const uint32_t *__r
   const int lane = threadIdx.x & 31;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t v = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; v < n; v += nwarps) {
-    const VHdr h = le_disk_record_header(recs[v], (uint32_t)v);
+    const DiskHdr h = le_disk_record_header(recs[v], (uint32_t)v);
     uint32_t *out = cols + rowptr[v];
     for (uint32_t i = lane; i < h.d; i += 32) out[i] = le_disk_neighbor(words, h, i);
   }
 }
-
-__device__ __forceinline__ uint32_t bit_len64(uint64_t x) { return x ? 64u - __clzll(x) : 1u; }
-
-// Chunk lengths tried per vertex; slots must fit a sector (cb <= 256).
-__constant__ uint8_t kChunkLens[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 20, 24, 28, 32};
-constexpr int kNumChunkLens = sizeof(kChunkLens);
-constexpr uint32_t kMaxSlots = 63;  // K is stored in 6 bits
-
-// Pass 1: per vertex of degree >= 2, the chunk length T with the fewest
-// bits (a vertex of one sector: C cb; larger: whole sectors), its sea_bit
-// (largest residual magnitude's bit count, as get_bit_num), K, rock width a
-// (bits of max(|n_0 - v|, |n_{d-1} - v|), LE/chunk_compress/compressor.hpp:69)
-// and first_pos (rocks below v).  meta[v] = T | sea_bit << 8 | K << 16 | a << 24.
-__global__ void __launch_bounds__(256) le_choose_kernel(const uint64_t *__restrict__ rowptr,
-                                                        const uint32_t *__restrict__ cols,
-                                                        uint32_t n, uint32_t *__restrict__ meta,
-                                                        uint32_t *__restrict__ fpos) {
-  const int lane = threadIdx.x & 31;
-  const unsigned FULLM = 0xFFFFFFFFu;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t v = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; v < n; v += nwarps) {
-    const uint64_t base = rowptr[v];
-    const uint32_t d = (uint32_t)(rowptr[v + 1] - base);
-    if (d < 2) {
-      if (lane == 0) meta[v] = 0, fpos[v] = 0;
-      continue;
-    }
-    const uint32_t *nb = cols + base;
-    const int64_t vv = (int64_t)v;
-    const uint32_t a = bit_len64((uint64_t)max(llabs((int64_t)nb[0] - vv),
-                                               llabs((int64_t)nb[d - 1] - vv)));
-    const uint32_t last = d - 1;
-    uint64_t best = ~0ull;
-    uint32_t bT = 1, bsb = 0, bK = 1;
-    for (int t = 0; t < kNumChunkLens; t++) {
-      const uint32_t T = kChunkLens[t];
-      if (T > 1 && T >= d) break;  // one chunk already holds every neighbor
-      uint32_t sb = 0;
-      for (uint32_t i = lane; i < last; i += 32) {
-        const uint32_t c = i / T, id = i - c * T;
-        if (!id) continue;
-        const uint32_t L = min(T, last - c * T);
-        const uint32_t r1 = nb[c * T], r2 = nb[c * T + L];
-        const int64_t res = (int64_t)nb[i] - ((int64_t)r1 + (int64_t)id * ((r2 - r1) / L));
-        sb = max(sb, bit_len64((uint64_t)llabs(res)));
-      }
-      sb = __reduce_max_sync(FULLM, sb);
-      const uint32_t cb = 2 * a + (T - 1) * (sb + 1);
-      if (cb > 256) continue;
-      const uint32_t K = min(256u / cb, kMaxSlots);
-      const uint32_t C = (last - 1) / T + 1;
-      const uint64_t cost = C <= K ? (uint64_t)C * cb : (uint64_t)((C + K - 1) / K) * 256u;
-      if (cost < best) best = cost, bT = T, bsb = sb, bK = K;
-    }
-    // first_pos: the rocks (n[cT] for c < C, and n[d-1]) below v
-    const uint32_t C = (last - 1) / bT + 1;
-    uint32_t below = 0;
-    for (uint32_t c = lane; c <= C; c += 32) below += (c < C ? nb[c * bT] : nb[last]) < v;
-    below = __reduce_add_sync(FULLM, below);
-    if (lane == 0) {
-      meta[v] = bT | bsb << 8 | bK << 16 | a << 24;
-      fpos[v] = below;
-    }
-  }
-}
-
-// Pass 2: every vertex's slots at its offset P[v] in dst (zeroed), and its
-// record rewritten in place in the device format.
-__global__ void __launch_bounds__(256) le_write_kernel(const uint64_t *__restrict__ rowptr,
-                                                       const uint32_t *__restrict__ cols,
-                                                       uint32_t n,
-                                                       const uint32_t *__restrict__ meta,
-                                                       const uint32_t *__restrict__ fpos,
-                                                       const uint64_t *__restrict__ P,
-                                                       uint32_t *dst, uint4 *recs) {
-  const int lane = threadIdx.x & 31;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t v = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; v < n; v += nwarps) {
-    const uint64_t base = rowptr[v];
-    const uint32_t d = (uint32_t)(rowptr[v + 1] - base);
-    if (d < 2) {
-      if (lane == 0) recs[v] = d ? pack_slot_record(0, 0, 0, 0, 0, 1, cols[base]) : make_uint4(0, 0, 0, 0);
-      continue;
-    }
-    const uint32_t *nb = cols + base;
-    const uint32_t m = meta[v];
-    const uint32_t T = m & 0xFFu, sb = (m >> 8) & 0xFFu, K = (m >> 16) & 0xFFu, a = m >> 24;
-    const uint32_t sw = sb + 1, cb = 2 * a + (T - 1) * sw, last = d - 1, C = (last - 1) / T + 1;
-    for (uint32_t c = lane; c < C; c += 32) {
-      const uint32_t q = c / K;
-      const uint64_t at = P[v] + (uint64_t)q * 256u + (uint64_t)(c - q * K) * cb;
-      const uint32_t L = min(T, last - c * T);
-      const uint32_t r1 = nb[c * T], r2 = nb[c * T + L];
-      or_bits(dst, at, (uint64_t)llabs((int64_t)r1 - (int64_t)v), a);
-      const uint32_t step = (r2 - r1) / L;
-      for (uint32_t id = 1; id < L; id++) {
-        const int64_t res = (int64_t)nb[c * T + id] - ((int64_t)r1 + (int64_t)id * step);
-        const uint64_t f = ((uint64_t)llabs(res) << 1) | (res < 0 ? 1u : 0u);
-        if (f) or_bits(dst, at + a + (uint64_t)(id - 1) * sw, f, sw);
-      }
-      or_bits(dst, at + a + (uint64_t)(T - 1) * sw, (uint64_t)llabs((int64_t)r2 - (int64_t)v), a);
-    }
-    if (lane == 0) recs[v] = pack_slot_record(P[v], a, sb, T, K, d, fpos[v]);
-  }
-}
-
-// ---- GT device layout (sector slots, device_common.cuh) ----
 
 // Pass 0: every GT neighbor list, decoded from the on-disk stream into a
 // temporary CSR: one warp per vertex, one lane per block, each block's head
@@ -385,7 +275,7 @@ __global__ void __launch_bounds__(256) gt_disk_decode_kernel(const uint32_t *__r
   const int lane = threadIdx.x & 31;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t v = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; v < n; v += nwarps) {
-    const VHdr h = gt_disk_record_header(recs[v], (uint32_t)v);
+    const DiskHdr h = gt_disk_record_header(recs[v], (uint32_t)v);
     uint32_t *out = cols + rowptr[v];
     for (uint32_t blk = lane; blk < h.bn; blk += 32) {
       const uint32_t L = blk < h.om ? h.bl + 1 : h.bl;
@@ -403,95 +293,98 @@ __global__ void __launch_bounds__(256) gt_disk_decode_kernel(const uint32_t *__r
   }
 }
 
-// Pass 1: per vertex of degree >= 1, the chunk length T with the fewest bits
-// (as for LE), the head width a (bits of the largest |n_cT - v| - 1), the gap
-// width b (bits of the largest n_i - n_{i-1} - 1 inside a chunk; 0 without
-// gaps), K, and first_pos (chunks whose head lies below v).
-// meta[v] = T | b << 8 | K << 16 | a << 24.
-__global__ void __launch_bounds__(256) gt_choose_kernel(const uint64_t *__restrict__ rowptr,
-                                                        const uint32_t *__restrict__ cols,
-                                                        uint32_t n, uint32_t *__restrict__ meta,
-                                                        uint32_t *__restrict__ fpos) {
+__device__ __forceinline__ uint32_t bit_len(uint32_t x) { return 32u - __clz(x); }
+
+// Chunk lengths tried per vertex; slots must fit a sector (cb <= 256).
+constexpr int kNumChunkLens = 16;
+constexpr uint32_t kMaxSlots = 63;  // K is stored in 6 bits
+
+// Pass 1: per vertex of degree >= 2, the chunk length T with the fewest bits
+// (a vertex of one sector: C cb; larger: whole sectors), the head width a
+// (bits of the largest n_cT - n_0; 0 with one chunk), the offset width b (bits
+// of the largest n_i - n_cT) and K.  meta[v] = T | b << 8 | K << 16 | a << 24.
+// One warp per vertex; one pass over its neighbors serves all chunk lengths
+// (they are compile-time constants, so i % T is a multiplication).
+__global__ void __launch_bounds__(256) slot_choose_kernel(const uint64_t *__restrict__ rowptr,
+                                                          const uint32_t *__restrict__ cols,
+                                                          uint32_t n, uint32_t *__restrict__ meta) {
+  constexpr uint32_t lens[kNumChunkLens] = {1, 2,  3,  4,  5,  6,  7,  8,
+                                            10, 12, 14, 16, 20, 24, 28, 32};
   const int lane = threadIdx.x & 31;
   const unsigned FULLM = 0xFFFFFFFFu;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t v = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; v < n; v += nwarps) {
     const uint64_t base = rowptr[v];
     const uint32_t d = (uint32_t)(rowptr[v + 1] - base);
-    if (d == 0) {
-      if (lane == 0) meta[v] = 0, fpos[v] = 0;
+    if (d < 2) {
+      if (lane == 0) meta[v] = 0;
       continue;
     }
     const uint32_t *nb = cols + base;
-    const int64_t vv = (int64_t)v;
+    const uint32_t n0 = nb[0];
+    uint32_t hd[kNumChunkLens], of[kNumChunkLens];  // largest head, largest offset
+#pragma unroll
+    for (int t = 0; t < kNumChunkLens; t++) hd[t] = of[t] = 0;
+    for (uint32_t i = lane; i < d; i += 32) {
+      const uint32_t x = nb[i];
+#pragma unroll
+      for (int t = 0; t < kNumChunkLens; t++) {
+        const uint32_t first = nb[i - i % lens[t]];
+        hd[t] = max(hd[t], first - n0);
+        of[t] = max(of[t], x - first);
+      }
+    }
     uint64_t best = ~0ull;
     uint32_t bT = 1, bb = 0, bK = 1, ba = 1;
+#pragma unroll
     for (int t = 0; t < kNumChunkLens; t++) {
-      const uint32_t T = kChunkLens[t];
-      if (T > 1 && T > d) break;  // one chunk already holds every neighbor
-      uint32_t a = 1, b = 0;
-      for (uint32_t i = lane; i < d; i += 32) {
-        if (i % T == 0) {
-          a = max(a, bit_len64((uint64_t)(llabs((int64_t)nb[i] - vv) - 1)));
-        } else {
-          b = max(b, bit_len64((uint64_t)(nb[i] - nb[i - 1] - 1)));
-        }
+      const uint32_t a = __reduce_max_sync(FULLM, bit_len(hd[t]));
+      const uint32_t b = max(__reduce_max_sync(FULLM, bit_len(of[t])), lens[t] > 1 ? 1u : 0u);
+      const uint32_t T = min(lens[t], d);  // (T >= d: one chunk, whatever lens[t])
+      const uint32_t cb = max(a + (T - 1) * b, 1u);  // a slot has at least one bit
+      if (cb <= 256) {
+        const uint32_t K = min(256u / cb, kMaxSlots);
+        const uint32_t C = (d - 1) / T + 1;
+        const uint64_t cost = C <= K ? (uint64_t)C * cb : (uint64_t)((C + K - 1) / K) * 256u;
+        if (cost < best) best = cost, bT = T, bb = b, bK = K, ba = cb - (T - 1) * b;
       }
-      a = __reduce_max_sync(FULLM, a);
-      b = __reduce_max_sync(FULLM, b);
-      const uint32_t cb = a + (T - 1) * b;
-      if (cb > 256) continue;
-      const uint32_t K = min(256u / cb, kMaxSlots);
-      const uint32_t C = (d - 1) / T + 1;
-      const uint64_t cost = C <= K ? (uint64_t)C * cb : (uint64_t)((C + K - 1) / K) * 256u;
-      if (cost < best) best = cost, bT = T, bb = b, bK = K, ba = a;
     }
-    const uint32_t C = (d - 1) / bT + 1;
-    uint32_t below = 0;
-    for (uint32_t c = lane; c < C; c += 32) below += nb[c * bT] < v;
-    below = __reduce_add_sync(FULLM, below);
-    if (lane == 0) {
-      meta[v] = bT | bb << 8 | bK << 16 | ba << 24;
-      fpos[v] = below;
-    }
+    if (lane == 0) meta[v] = bT | bb << 8 | bK << 16 | ba << 24;
   }
 }
 
 // Pass 2: every vertex's slots at its offset P[v] in dst (zeroed), and its
 // record rewritten in place in the device format.
-__global__ void __launch_bounds__(256) gt_write_kernel(const uint64_t *__restrict__ rowptr,
-                                                       const uint32_t *__restrict__ cols,
-                                                       uint32_t n,
-                                                       const uint32_t *__restrict__ meta,
-                                                       const uint32_t *__restrict__ fpos,
-                                                       const uint64_t *__restrict__ P,
-                                                       uint32_t *dst, uint4 *recs) {
+__global__ void __launch_bounds__(256) slot_write_kernel(const uint64_t *__restrict__ rowptr,
+                                                         const uint32_t *__restrict__ cols,
+                                                         uint32_t n,
+                                                         const uint32_t *__restrict__ meta,
+                                                         const uint64_t *__restrict__ P,
+                                                         uint32_t *dst, uint4 *recs) {
   const int lane = threadIdx.x & 31;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t v = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; v < n; v += nwarps) {
     const uint64_t base = rowptr[v];
     const uint32_t d = (uint32_t)(rowptr[v + 1] - base);
-    if (d == 0) {
-      if (lane == 0) recs[v] = make_uint4(0, 0, 0, 0);
+    const uint32_t *nb = cols + base;
+    if (d < 2) {
+      if (lane == 0)
+        recs[v] = d ? pack_slot_record(0, 0, 0, 1, 1, 1, nb[0]) : make_uint4(0, 0, 0, 0);
       continue;
     }
-    const uint32_t *nb = cols + base;
-    const uint32_t m = meta[v];
+    const uint32_t m = meta[v], n0 = nb[0];
     const uint32_t T = m & 0xFFu, b = (m >> 8) & 0xFFu, K = (m >> 16) & 0xFFu, a = m >> 24;
     const uint32_t cb = a + (T - 1) * b, C = (d - 1) / T + 1;
     for (uint32_t c = lane; c < C; c += 32) {
       const uint32_t q = c / K;
       uint64_t at = P[v] + (uint64_t)q * 256u + (uint64_t)(c - q * K) * cb;
-      const uint32_t i0 = c * T, L = min(T, d - i0);
-      const uint64_t head = (uint64_t)(llabs((int64_t)nb[i0] - (int64_t)v) - 1);
-      if (head) or_bits(dst, at, head, a);
+      const uint32_t i0 = c * T, L = min(T, d - i0), x = nb[i0];
+      if (x != n0) or_bits(dst, at, x - n0, a);
       at += a;
-      for (uint32_t t = 1; t < L; t++, at += b) {
-        const uint32_t gap = nb[i0 + t] - nb[i0 + t - 1] - 1;
-        if (gap) or_bits(dst, at, gap, b);
-      }
+      for (uint32_t t = 1; t < L; t++, at += b)
+        if (nb[i0 + t] != x) or_bits(dst, at, nb[i0 + t] - x, b);
     }
-    if (lane == 0) recs[v] = pack_slot_record(P[v], a, b, T, K, d, fpos[v]);
+    if (lane == 0) recs[v] = pack_slot_record(P[v], a, b, T, K, d, n0);
   }
 }
 
@@ -523,6 +416,11 @@ void launch_scan_u32(const uint32_t *counts, uint64_t n, uint64_t *out, uint64_t
   scan_impl(CountLoader{counts}, n, out, tmp, s);
 }
 
+void launch_scan_degrees(const uint4 *recs, uint64_t n, uint64_t *rowptr, uint64_t *tmp,
+                         cudaStream_t s) {
+  scan_impl(DegreeLoader{recs}, n, rowptr, tmp, s);
+}
+
 void launch_validate(const DevGraph &g, uint32_t *deg, unsigned long long *stats,
                      cudaStream_t s) {
   int dev = 0;
@@ -552,26 +450,20 @@ void launch_disk_decode(int mode, const uint32_t *words, const uint4 *recs, uint
   count_launch();
 }
 
-void launch_slot_choose(int mode, const uint64_t *rowptr, const uint32_t *cols, uint32_t n,
-                        uint32_t *meta, uint32_t *fpos, cudaStream_t s) {
+void launch_slot_choose(const uint64_t *rowptr, const uint32_t *cols, uint32_t n, uint32_t *meta,
+                        cudaStream_t s) {
   int dev = 0;
   cudaGetDevice(&dev);
-  const unsigned grid = (unsigned)sm_count(dev) * 8;
-  if (mode == GRASS_MODE_GT) gt_choose_kernel<<<grid, 256, 0, s>>>(rowptr, cols, n, meta, fpos);
-  else le_choose_kernel<<<grid, 256, 0, s>>>(rowptr, cols, n, meta, fpos);
+  slot_choose_kernel<<<(unsigned)sm_count(dev) * 8, 256, 0, s>>>(rowptr, cols, n, meta);
   count_launch();
 }
 
-void launch_slot_write(int mode, const uint64_t *rowptr, const uint32_t *cols, uint32_t n,
-                       const uint32_t *meta, const uint32_t *fpos, const uint64_t *P,
-                       uint32_t *dst, uint4 *recs, cudaStream_t s) {
+void launch_slot_write(const uint64_t *rowptr, const uint32_t *cols, uint32_t n,
+                       const uint32_t *meta, const uint64_t *P, uint32_t *dst, uint4 *recs,
+                       cudaStream_t s) {
   int dev = 0;
   cudaGetDevice(&dev);
-  const unsigned grid = (unsigned)sm_count(dev) * 8;
-  if (mode == GRASS_MODE_GT)
-    gt_write_kernel<<<grid, 256, 0, s>>>(rowptr, cols, n, meta, fpos, P, dst, recs);
-  else
-    le_write_kernel<<<grid, 256, 0, s>>>(rowptr, cols, n, meta, fpos, P, dst, recs);
+  slot_write_kernel<<<(unsigned)sm_count(dev) * 8, 256, 0, s>>>(rowptr, cols, n, meta, P, dst, recs);
   count_launch();
 }
 
@@ -579,22 +471,8 @@ void launch_degrees(const DevGraph &g, uint32_t *deg, cudaStream_t s) {
   int dev = 0;
   cudaGetDevice(&dev);
   unsigned grid = grid_for(g.n, 256, dev);
-  if (g.mode == GRASS_MODE_GT) degrees_kernel<0, uint32_t><<<grid, 256, 0, s>>>(g, deg);
-  else degrees_kernel<1, uint32_t><<<grid, 256, 0, s>>>(g, deg);
+  degrees_kernel<<<grid, 256, 0, s>>>(g, deg);
   count_launch();
-}
-
-void launch_degrees64(const DevGraph &g, uint64_t *deg, cudaStream_t s) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  unsigned grid = grid_for(g.n, 256, dev);
-  if (g.mode == GRASS_MODE_GT) degrees_kernel<0, uint64_t><<<grid, 256, 0, s>>>(g, deg);
-  else degrees_kernel<1, uint64_t><<<grid, 256, 0, s>>>(g, deg);
-  count_launch();
-}
-
-void launch_scan_u64_inplace(uint64_t *vals, uint64_t n, uint64_t *tmp, cudaStream_t s) {
-  scan_impl(U64Loader{vals}, n, vals, tmp, s);
 }
 
 }  // namespace grass

@@ -15,15 +15,9 @@
 #include <mutex>
 
 // Resident 512-thread blocks per SM each walk kernel is compiled for (its
-// register budget), as measured on the 1M x 80 walk: the LE walk keeps all
-// the registers it wants (79 at one walker per thread; launched as 256-thread
-// blocks, three per SM, which ran 17% faster than 512-thread blocks), the GT
-// walk is 23% faster at 64 registers or fewer, the CSR walk 2% faster.
-#ifndef GRASS_RW_LE_MIN_BLOCKS
-#define GRASS_RW_LE_MIN_BLOCKS 1
-#endif
-#ifndef GRASS_RW_GT_MIN_BLOCKS
-#define GRASS_RW_GT_MIN_BLOCKS 2
+// register budget).
+#ifndef GRASS_RW_MIN_BLOCKS
+#define GRASS_RW_MIN_BLOCKS 2
 #endif
 #ifndef GRASS_RW_CSR_MIN_BLOCKS
 #define GRASS_RW_CSR_MIN_BLOCKS 2
@@ -42,7 +36,7 @@ __device__ __forceinline__ void store_path(uint32_t *paths, int layout, uint64_t
 // w0: walker id of starts[0] -- draws use walker id w0 + w, so a batch split
 // into chunks produces the same walks as one launch.
 template <int MODE, int DEPTH>
-__global__ void __launch_bounds__(512, MODE == 0 ? GRASS_RW_GT_MIN_BLOCKS : GRASS_RW_LE_MIN_BLOCKS) rw_kernel(DevGraph g, const uint32_t *__restrict__ starts,
+__global__ void __launch_bounds__(512, GRASS_RW_MIN_BLOCKS) rw_kernel(DevGraph g, const uint32_t *__restrict__ starts,
                                                  uint64_t W, uint32_t L, uint64_t seed,
                                                  uint64_t w0, int layout,
                                                  uint32_t *__restrict__ paths,
@@ -66,28 +60,16 @@ __global__ void __launch_bounds__(512, MODE == 0 ? GRASS_RW_GT_MIN_BLOCKS : GRAS
       }
     }
     for (uint32_t s = 0; s < L; s++) {
+      walk_step<MODE, DEPTH>(g, v, [&](int k) {
+        if ((s & 3) == 0) {
+          const uint64_t id = w0 + base + k * nthreads;
+          r[k] = philox4x32_10(seed, s >> 2, (uint32_t)id, (uint32_t)(id >> 32), TAG_RW);
+        }
+        return pick(r[k], s & 3);
+      }, cnt, bad);
 #pragma unroll
       for (int k = 0; k < DEPTH; k++) {
         const uint64_t w = base + k * nthreads;
-        if ((s & 3) == 0) {
-          const uint64_t id = w0 + w;
-          r[k] = philox4x32_10(seed, s >> 2, (uint32_t)id, (uint32_t)(id >> 32), TAG_RW);
-        }
-        if (v[k] != INVALID_VERTEX) {
-          const VHdr h = header<MODE>(g, v[k]);
-          if (h.d == 0) {
-            v[k] = INVALID_VERTEX;
-          } else {
-            const uint32_t nv = neighbor<MODE>(g, h, mulhi_u32(pick(r[k], s & 3), h.d));
-            if (nv >= g.n) {
-              bad = true;
-              v[k] = INVALID_VERTEX;
-            } else {
-              v[k] = nv;
-              cnt++;
-            }
-          }
-        }
         if (w < W) store_path(paths, layout, W, L, w, s + 1, v[k]);
       }
     }
@@ -109,18 +91,15 @@ struct N2vArgs {
   uint64_t t_ret, t_in, t_out;  // acceptance thresholds in [0, 2^32]
 };
 
-// The first neighbor of slot c (GT: its head; LE: its left rock): one field
-// of at most 32 bits, read as one or two 32-bit words (the second only when
-// the field crosses into it).
-template <int MODE>
-__device__ __forceinline__ uint32_t slot_first(const DevGraph &g, const VHdr &h, uint32_t c) {
-  const uint64_t pos = slot_pos(h, c);
-  const uint32_t *q = g.words + (pos >> 5);
-  const uint32_t s = (uint32_t)pos & 31u, w = (uint32_t)h.a;
-  const uint32_t hi = ldw(q), lo = s + w > 32u ? ldw(q + 1) : 0u;
-  const uint32_t m = w ? __funnelshift_l(lo, hi, s) >> (32u - w) : 0u;
-  if constexpr (MODE == 0) return c >= h.fp ? h.v + m + 1u : h.v - m - 1u;
-  else return c < h.fp ? h.v - m : h.v + m;
+// The head of slot c (its first neighbor less n_0): one field of at most 32
+// bits, read as one or two 32-bit words (the second only when the field
+// crosses into it).
+__device__ __forceinline__ uint32_t slot_head(const DevGraph &g, const VHdr &h, uint32_t c) {
+  const DrawAt at = slot_at(h, c);
+  const uint32_t *q = g.words + (uint64_t)at.sec * 8 + (at.off >> 5);
+  const uint32_t s = at.off & 31u;
+  const uint32_t hi = ldw(q), lo = s + h.a > 32u ? ldw(q + 1) : 0u;
+  return shr_clamp(__funnelshift_l(lo, hi, s), 32u - h.a);
 }
 
 // The last index in [lo, hi] whose key is <= x, given key(lo) <= x, for
@@ -138,38 +117,30 @@ __device__ __forceinline__ uint32_t last_le(uint32_t lo, uint32_t hi, uint32_t x
 }
 
 // Whether x is a neighbor of the vertex of header h.  Compressed: a search
-// over the slots' first neighbors for the one slot that can hold x, then a
-// search of that slot inside its sector, in registers (GT: a scan of the
-// gaps; LE: a binary search of the closed-form values).  CSR: a search of
-// the row.
+// over the slots' heads for the one slot that can hold x, then a search of
+// that slot's offsets inside its sector, in registers.  CSR: a search of the
+// row.
 template <int MODE>
 __device__ __forceinline__ bool has_neighbor(const DevGraph &g, const VHdr &h, uint32_t x) {
   if (h.d == 0) return false;
-  if constexpr (MODE == 2) {
+  if constexpr (MODE == kCsr) {
     if (neighbor<MODE>(g, h, 0) > x) return false;
     const uint32_t i = last_le(0u, h.d - 1, x, [&](uint32_t k) { return neighbor<MODE>(g, h, k); });
     return neighbor<MODE>(g, h, i) == x;
   } else {
-    if (MODE == 1 && h.d == 1) return h.fp == x;
-    if (slot_first<MODE>(g, h, 0) > x) return false;
-    const uint32_t c = last_le(0u, h.bn - 1, x, [&](uint32_t k) { return slot_first<MODE>(g, h, k); });
-    // slot c holds indices c bl .. c bl + last
-    const uint32_t last = c + 1 == h.bn ? h.d - 1 - c * h.bl : h.bl - 1;
-    const uint64_t pos = slot_pos(h, c);
-    const Sec A = load_sector(g.words, pos >> 8);
-    const uint32_t off = (uint32_t)pos & 255u;
-    if constexpr (MODE == 0) {
-      const uint32_t hv = (uint32_t)sec1_field(A, off, h.a) + 1u;
-      uint32_t y = c >= h.fp ? h.v + hv : h.v - hv;
-      uint32_t p = off + (uint32_t)h.a;
-      for (uint32_t t = 0; y < x && t < last; t++, p += (uint32_t)h.b)
-        y += (h.b ? (uint32_t)sec1_field(A, p, h.b) : 0u) + 1u;
-      return y == x;
-    } else {
-      const uint32_t L = min(h.bl, h.d - 1 - c * h.bl);
-      const uint32_t id = last_le(0u, last, x, [&](uint32_t k) { return le_slot_value(A, off, h, c, k, L); });
-      return le_slot_value(A, off, h, c, id, L) == x;
-    }
+    if (x <= h.base || h.cb == 0) return x == h.base;
+    const uint32_t y = x - h.base;
+    const uint32_t c = last_le(0u, div_small(h.d - 1, h.T), y,
+                               [&](uint32_t k) { return slot_head(g, h, k); });
+    const DrawAt at = slot_at(h, c);
+    const Sec A = load_sector(g.words, at.sec);
+    const uint32_t z = y - sec_field(A, at.off, h.a);  // the offset looked for
+    if (z == 0) return true;
+    const uint32_t last = min(h.T, h.d - c * h.T) - 1;
+    auto offset = [&](uint32_t id) {  // of index id in the slot
+      return sec_field(A, at.off + h.a + (id - 1) * h.b, id ? h.b : 0u);
+    };
+    return offset(last_le(0u, last, z, offset)) == z;
   }
 }
 
@@ -188,7 +159,7 @@ __device__ __forceinline__ bool has_neighbor(const DevGraph &g, const VHdr &h, u
 #endif
 
 template <int MODE>
-__global__ void __launch_bounds__(256, MODE == 2 ? GRASS_N2V_CSR_MIN_BLOCKS : GRASS_N2V_MIN_BLOCKS) n2v_kernel(DevGraph g, const uint32_t *__restrict__ starts,
+__global__ void __launch_bounds__(256, MODE == kCsr ? GRASS_N2V_CSR_MIN_BLOCKS : GRASS_N2V_MIN_BLOCKS) n2v_kernel(DevGraph g, const uint32_t *__restrict__ starts,
                                                   uint64_t W, N2vArgs a,
                                                   uint32_t *__restrict__ paths,
                                                   unsigned long long *edges, unsigned int *err) {
@@ -245,27 +216,8 @@ __global__ void __launch_bounds__(256, MODE == 2 ? GRASS_N2V_CSR_MIN_BLOCKS : GR
   if (bad && err) atomicOr(err, 1u);
 }
 
-// Stream bits a draw of neighbor i reads (the payload fields; the header is
-// in the vertex record), and the 32-byte sectors those reads span.
-template <int MODE>
-__device__ __forceinline__ void draw_footprint(const DevGraph &g, const VHdr &h, uint32_t i,
-                                               uint64_t &bits, uint64_t &sectors) {
-  (void)g;
-  sectors = 1;  // a chunk slot never crosses a sector
-  if (MODE == 0) {  // the slot's head and the gaps up to neighbor i
-    bits = (uint64_t)h.a + (uint64_t)(i % h.bl) * h.b;
-  } else if (h.d > 1) {  // the left rock; for an inner neighbor the right rock and a sea
-    uint32_t c, id, L;
-    le_locate(h, i, c, id, L);
-    bits = id == 0 ? (uint64_t)h.a : id == L ? 2ull * h.a : 2ull * h.a + h.b + 1;
-  } else {  // LE degree 1: the neighbor is in the record
-    bits = 0;
-    sectors = 0;
-  }
-}
-
 // Replays a walk (same stream as rw_kernel) and sums, per draw, the
-// algorithmic bytes 16 (vertex record) + ceil(payload bits read / 8) + 4
+// algorithmic bytes 16 (vertex record) + ceil(slot bits read / 8) + 4
 // (path entry) and the 32-byte sectors the reads span (+1 for the record).
 // out[0] = bytes, out[1] = sectors, out[2] = draws.  Start entries add 4
 // bytes each.
@@ -295,7 +247,6 @@ __global__ void __launch_bounds__(256) random_read_kernel(const uint32_t *__rest
   if ((threadIdx.x & 31) == 0) atomicAdd(sink, (unsigned long long)acc);
 }
 
-template <int MODE>
 __global__ void __launch_bounds__(256) rw_account_kernel(DevGraph g,
                                                          const uint32_t *__restrict__ starts,
                                                          uint64_t W, uint32_t L, uint64_t seed,
@@ -311,18 +262,18 @@ __global__ void __launch_bounds__(256) rw_account_kernel(DevGraph g,
       if ((s & 3) == 0) r = philox4x32_10(seed, s >> 2, (uint32_t)w, (uint32_t)(w >> 32), TAG_RW);
       bytes += 4;
       if (v == INVALID_VERTEX) continue;
-      const VHdr h = header<MODE>(g, v);
+      const VHdr h = header<kSlots>(g, v);
       if (h.d == 0) {
         v = INVALID_VERTEX;
         continue;
       }
       const uint32_t i = mulhi_u32(pick(r, s & 3), h.d);
-      uint64_t b, sc;
-      draw_footprint<MODE>(g, h, i, b, sc);
-      bytes += 16 + (b + 7) / 8;
-      sect += 1 + sc;
+      // the slot's head and, past its first neighbor, one offset; nothing for degree 1
+      const uint32_t bits = h.a + (i % h.T ? h.b : 0u);
+      bytes += 16 + (bits + 7) / 8;
+      sect += 1 + (h.cb ? 1 : 0);
       draws++;
-      const uint32_t nv = neighbor<MODE>(g, h, i);
+      const uint32_t nv = neighbor<kSlots>(g, h, i);
       v = nv < g.n ? nv : INVALID_VERTEX;
     }
   }
@@ -392,9 +343,6 @@ __global__ void __launch_bounds__(512, GRASS_RW_CSR_MIN_BLOCKS) rw_csr_kernel(De
 #ifndef GRASS_KHOP_MIN_BLOCKS
 #define GRASS_KHOP_MIN_BLOCKS 4
 #endif
-// Words of a warp's draw-staging buffers (dynamic shared memory).
-constexpr uint32_t kKhopBufWords = GRASS_KHOP_INFLIGHT * 32 * kDrawBufWords;
-
 // k-hop.  One warp per seed (khop_seed_warp).
 
 template <int MODE>
@@ -402,15 +350,13 @@ __global__ void __launch_bounds__(256, GRASS_KHOP_MIN_BLOCKS) khop_kernel(DevGra
                                                    uint64_t S, KhopArgs A,
                                                    unsigned long long *edges, unsigned int *err) {
   __shared__ SmemHdr sh[8];
-  extern __shared__ __align__(16) uint32_t khop_dbuf[];  // 8 warps x kKhopBufWords
   SmemHdr &my = sh[threadIdx.x >> 5];
-  uint32_t *dbuf = khop_dbuf + (threadIdx.x >> 5) * kKhopBufWords;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   uint64_t cnt = 0;
   bool bad = false;
   for (uint64_t s = warp; s < S; s += nwarps)
-    khop_seed_warp<MODE, GRASS_KHOP_INFLIGHT>(g, seeds, A, s, my, dbuf, cnt, bad);
+    khop_seed_warp<MODE, GRASS_KHOP_INFLIGHT>(g, seeds, A, s, my, cnt, bad);
   warp_add_u64(edges, cnt);
   if (bad && err) atomicOr(err, 1u);
 }
@@ -432,7 +378,7 @@ __global__ void __launch_bounds__(256, GRASS_KHOP_MIN_BLOCKS) khop_csr_kernel(De
   uint64_t cnt = 0;
   bool bad = false;
   for (uint64_t s = warp; s < S; s += nwarps)
-    khop_seed_warp<2, GRASS_KHOP_INFLIGHT>(g, seeds, A, s, my, nullptr, cnt, bad);
+    khop_seed_warp<kCsr, GRASS_KHOP_INFLIGHT>(g, seeds, A, s, my, cnt, bad);
   warp_add_u64(edges, cnt);
 }
 
@@ -615,9 +561,8 @@ int apply_tuning(int device, const grass_tuning &t, const void *base, size_t byt
 }
 
 // Defaults measured on B200 (R-MAT s22 ef32, 1M walkers x 80, step-major
-// paths): the LE walk is 2% faster with one walker per thread than with two
-// or four (3.60 / 3.67 / 3.68 ms), the CSR walk 0.5% faster with four; GT,
-// whose warps synchronise every step, is 11% faster with one than with two.
+// paths): the compressed walk is fastest with one walker per thread, the CSR
+// walk 0.5% faster with four.
 grass_tuning resolve_tuning(const grass_tuning &t, int kind) {
   grass_tuning r = t;
   if (!r.rw_depth) r.rw_depth = kind == 2 ? 4 : 1;
@@ -640,27 +585,26 @@ static unsigned resident_grid(K kern, int threads, uint32_t want_per_sm, uint64_
   return (unsigned)std::max<uint64_t>(1, std::min(need, cap));
 }
 
-template <int MODE, int DEPTH>
+template <int DEPTH>
 static void rw_launch_depth(const DevGraph &g, const grass_rw_params &p, const uint32_t *starts,
                             uint64_t W, uint32_t *paths, unsigned long long *edges,
                             unsigned int *err, cudaStream_t s, const grass_tuning &t,
                             const L2Window &win, uint64_t w0) {
-  auto kern = rw_kernel<MODE, DEPTH>;
+  auto kern = rw_kernel<kSlots, DEPTH>;
   const unsigned grid =
       resident_grid(kern, (int)t.rw_threads, t.rw_blocks_per_sm, W, (uint64_t)t.rw_threads * DEPTH);
   launch_with_window(kern, grid, t.rw_threads, s, win, g, starts, W, p.length, p.seed, w0,
                      (int)p.layout, paths, edges, err);
 }
 
-template <int MODE>
 static void rw_dispatch(const DevGraph &g, const grass_rw_params &p, const uint32_t *starts,
                         uint64_t W, uint32_t *paths, unsigned long long *edges,
                         unsigned int *err, cudaStream_t s, const grass_tuning &t,
                         const L2Window &win, uint64_t w0) {
   switch (t.rw_depth) {
-    case 1: rw_launch_depth<MODE, 1>(g, p, starts, W, paths, edges, err, s, t, win, w0); break;
-    case 4: rw_launch_depth<MODE, 4>(g, p, starts, W, paths, edges, err, s, t, win, w0); break;
-    default: rw_launch_depth<MODE, 2>(g, p, starts, W, paths, edges, err, s, t, win, w0);
+    case 1: rw_launch_depth<1>(g, p, starts, W, paths, edges, err, s, t, win, w0); break;
+    case 4: rw_launch_depth<4>(g, p, starts, W, paths, edges, err, s, t, win, w0); break;
+    default: rw_launch_depth<2>(g, p, starts, W, paths, edges, err, s, t, win, w0);
   }
 }
 
@@ -669,8 +613,7 @@ void launch_rw(const DevGraph &g, const grass_rw_params &p, const uint32_t *star
                const grass_tuning &tin, const L2Window &win, uint64_t w0) {
   if (!W) return;
   const grass_tuning t = resolve_tuning(tin, g.mode);
-  if (g.mode == GRASS_MODE_GT) rw_dispatch<0>(g, p, starts, W, paths, edges, err, s, t, win, w0);
-  else rw_dispatch<1>(g, p, starts, W, paths, edges, err, s, t, win, w0);
+  rw_dispatch(g, p, starts, W, paths, edges, err, s, t, win, w0);
   count_launch();
 }
 
@@ -688,10 +631,7 @@ void launch_rw_account(const DevGraph &g, const grass_rw_params &p, const uint32
                        uint64_t W, unsigned long long *out, cudaStream_t s) {
   if (!W) return;
   const unsigned grid = grid_warps(W, 256, cur_dev(), 8);
-  if (g.mode == GRASS_MODE_GT)
-    rw_account_kernel<0><<<grid, 256, 0, s>>>(g, starts, W, p.length, p.seed, out);
-  else
-    rw_account_kernel<1><<<grid, 256, 0, s>>>(g, starts, W, p.length, p.seed, out);
+  rw_account_kernel<<<grid, 256, 0, s>>>(g, starts, W, p.length, p.seed, out);
   count_launch();
 }
 
@@ -745,16 +685,7 @@ void launch_khop(const DevGraph &g, const grass_khop_params &p, const uint32_t *
   if (!S) return;
   const KhopArgs A = khop_args(p, hop_out);
   const unsigned grid = grid_warps(S, 8, cur_dev(), 8);
-  const uint32_t smem = 8 * kKhopBufWords * 4;
-  static std::once_flag once;  // opt in to more than 48 KB of shared memory
-  std::call_once(once, [&] {
-    cudaFuncSetAttribute(khop_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(khop_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  });
-  if (g.mode == GRASS_MODE_GT)
-    khop_kernel<0><<<grid, 256, smem, s>>>(g, seeds, S, A, edges, err);
-  else
-    khop_kernel<1><<<grid, 256, smem, s>>>(g, seeds, S, A, edges, err);
+  khop_kernel<kSlots><<<grid, 256, 0, s>>>(g, seeds, S, A, edges, err);
   count_launch();
 }
 
@@ -772,9 +703,10 @@ void launch_node2vec(const DevGraph &g, const grass_node2vec_params &p, const ui
   a.t_in = t[1];
   a.t_out = t[2];
   const unsigned grid = grid_warps(W, 256, cur_dev(), 8);
-  if (g.mode == GRASS_MODE_GT) n2v_kernel<0><<<grid, 256, 0, s>>>(g, starts, W, a, paths, edges, err);
-  else if (g.mode == GRASS_MODE_LE) n2v_kernel<1><<<grid, 256, 0, s>>>(g, starts, W, a, paths, edges, err);
-  else n2v_kernel<2><<<grid, 256, 0, s>>>(g, starts, W, a, paths, edges, err);
+  if (g.mode == GRASS_MODE_CSR_INTERNAL)
+    n2v_kernel<kCsr><<<grid, 256, 0, s>>>(g, starts, W, a, paths, edges, err);
+  else
+    n2v_kernel<kSlots><<<grid, 256, 0, s>>>(g, starts, W, a, paths, edges, err);
   count_launch();
 }
 
@@ -799,7 +731,7 @@ int launch_mrw(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots, ui
        (p.steps >= 1024 || S < (uint64_t)sm_count(cur_dev()) * 8))) {
     const int threads = (int)std::min<uint64_t>(
         512, std::max<uint64_t>(128, ((uint64_t)p.walkers / 2 + 31) / 32 * 32));
-    auto kern = g.mode == GRASS_MODE_GT ? mrw_cta_kernel<0> : mrw_cta_kernel<1>;
+    auto kern = mrw_cta_kernel<kSlots>;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0);
     const uint64_t grid =
@@ -822,7 +754,7 @@ int launch_mrw(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots, ui
     cudaError_t e =
         scratch_alloc(reinterpret_cast<void **>(&rec), S * (uint64_t)p.walkers * sizeof(uint4), s);
     if (e != cudaSuccess) return cuda_fail(e, "multi-RW scratch");
-    auto kern = g.mode == GRASS_MODE_GT ? mrw_global_kernel<0> : mrw_global_kernel<1>;
+    auto kern = mrw_global_kernel<kSlots>;
     kern<<<grid_warps(S, 8, cur_dev(), 8), 256, 0, s>>>(g, roots, rec, S, p.walkers, p.steps,
                                                         (int)p.select, p.seed, src, dst, edges,
                                                         err);
@@ -833,7 +765,7 @@ int launch_mrw(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots, ui
   const size_t budget = 200 * 1024;
   const int warps = (int)std::min<size_t>(8, budget / per_warp);
   const size_t smem = per_warp * warps;
-  auto kern = g.mode == GRASS_MODE_GT ? mrw_kernel<0> : mrw_kernel<1>;
+  auto kern = mrw_kernel<kSlots>;
   if (smem > 48 * 1024)
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const unsigned grid = grid_warps(S, warps, cur_dev(), 8);

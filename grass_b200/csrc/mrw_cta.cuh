@@ -265,7 +265,7 @@ __device__ void mrw_uniform_cta(const DevGraph &g, uint32_t *roots, uint32_t *sr
           continue;
         }
         const uint32_t ry = philox4x32_10(seed, t, s_lo, s_hi, TAG_MRW).y;
-        const VHdr h = record_header<MODE>(rc[q], v[q]);
+        const VHdr h = record_header<MODE>(rc[q]);
         const uint32_t nv = neighbor<MODE>(g, h, mulhi_u32(ry, h.d));
         if (nv >= g.n) {
           bad = true;
@@ -364,7 +364,7 @@ __device__ void mrw_ct_cta(const DevGraph &g, uint32_t *roots, uint32_t *src, ui
             if (!(s[q].t <= H)) continue;
             any = true;
             const uint32_t w = w0 + q * nt;
-            const VHdr h = record_header<MODE>(r[q], s[q].v);
+            const VHdr h = record_header<MODE>(r[q]);
             const uint32_t nv = neighbor<MODE>(g, h, mulhi_u32(s[q].z, h.d));
             if (nv >= g.n) {  // corrupt payload: the walker stops
               bad = true;

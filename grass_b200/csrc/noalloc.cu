@@ -63,8 +63,7 @@ extern "C" int grass_decode_all_noalloc(const grass_graph *g, uint64_t *d_rowptr
   // Nothing in the scratch has to start at zero: the scan writes every tile
   // sum it later reads.  All calls share the array, so calls that overlap on
   // the GPU (other streams, other threads) race on it.
-  launch_degrees64(g->view(), d_rowptr, st);
-  launch_scan_u64_inplace(d_rowptr, n, scratch, st);
+  launch_scan_degrees(g->d_recs, n, d_rowptr, scratch, st);
   // The planned sweep once an earlier grass_decode_all has built the graph's
   // plan (launching it allocates nothing); until then the unplanned sweep,
   // which needs no plan and is about 3x slower.

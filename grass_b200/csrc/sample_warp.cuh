@@ -16,8 +16,50 @@ __device__ __forceinline__ void path_store(uint32_t *paths, int layout, uint64_t
   else store_out_u32(paths + (uint64_t)s * W + w, v);
 }
 
+// One step of DEPTH independent walkers: every record load is issued before
+// the random words are made, and every sector load before any is decoded, so
+// a lane's loads overlap and the Philox rounds run while the records arrive.
+// v[k] is the walker's vertex (INVALID_VERTEX: stopped), word(k) its random
+// word of the step.
+template <int MODE, int DEPTH, class Word>
+__device__ __forceinline__ void walk_step(const DevGraph &g, uint32_t (&v)[DEPTH], Word word,
+                                          uint64_t &cnt, bool &bad) {
+  uint4 rec[DEPTH];
+#pragma unroll
+  for (int k = 0; k < DEPTH; k++)
+    rec[k] = v[k] != INVALID_VERTEX ? graph_record<MODE>(g, v[k]) : make_uint4(0u, 0u, 0u, 0u);
+  VHdr h[DEPTH];
+  DrawAt at[DEPTH];
+  Sec A[DEPTH];
+  uint32_t nv[DEPTH];
+#pragma unroll
+  for (int k = 0; k < DEPTH; k++) {
+    const uint32_t rnd = word(k);
+    h[k] = record_header<MODE>(rec[k]);
+    nv[k] = h[k].base;  // (degree 1)
+    const uint32_t i = mulhi_u32(rnd, h[k].d);
+    if constexpr (MODE == kCsr) {
+      if (h[k].d) nv[k] = load_cold_u32(g.cols + h[k].P + i);
+    } else if (h[k].cb) {
+      at[k] = draw_at(h[k], i);
+      A[k] = load_sector(g.words, at[k].sec);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < DEPTH; k++) {
+    if constexpr (MODE != kCsr)
+      if (h[k].cb) nv[k] = draw_value(A[k], at[k], h[k]);
+    const bool ok = nv[k] < g.n;
+    if (h[k].d) {
+      bad |= !ok;
+      cnt += ok;
+    }
+    v[k] = h[k].d && ok ? nv[k] : INVALID_VERTEX;
+  }
+}
+
 // Random walk of walkers [b, e) of a job of W walkers (starts[0..W)), DEPTH
-// walkers per lane per pass.  Same draws as rw_kernel / rw_gt_kernel:
+// walkers per lane per pass.  Same draws as rw_kernel:
 // walker w uses Philox(seed; step>>2, w0+w, .., TAG_RW).
 template <int MODE, int DEPTH>
 __device__ __forceinline__ void rw_warp(const DevGraph &g, const uint32_t *starts, uint64_t W,
@@ -40,33 +82,16 @@ __device__ __forceinline__ void rw_warp(const DevGraph &g, const uint32_t *start
       }
     }
     for (uint32_t s = 0; s < L; s++) {
+      walk_step<MODE, DEPTH>(g, v, [&](int k) {
+        if ((s & 3) == 0) {
+          const uint64_t id = w0 + wb + (uint64_t)k * 32 + lane;
+          r[k] = philox4x32_10(seed, s >> 2, (uint32_t)id, (uint32_t)(id >> 32), TAG_RW);
+        }
+        return pick(r[k], s & 3);
+      }, cnt, bad);
 #pragma unroll
       for (int k = 0; k < DEPTH; k++) {
         const uint64_t w = wb + (uint64_t)k * 32 + lane;
-        if ((s & 3) == 0) {
-          const uint64_t id = w0 + w;
-          r[k] = philox4x32_10(seed, s >> 2, (uint32_t)id, (uint32_t)(id >> 32), TAG_RW);
-        }
-        bool active = v[k] != INVALID_VERTEX;
-        uint32_t nv = INVALID_VERTEX;
-        if (active) {
-          const VHdr h = header<MODE>(g, v[k]);
-          if (h.d == 0) {
-            active = false;
-            v[k] = INVALID_VERTEX;
-          } else {
-            nv = neighbor<MODE>(g, h, mulhi_u32(pick(r[k], s & 3), h.d));
-          }
-        }
-        if (active) {
-          if (nv >= g.n) {
-            bad = true;
-            v[k] = INVALID_VERTEX;
-          } else {
-            v[k] = nv;
-            cnt++;
-          }
-        }
         if (w < e) path_store(paths, layout, W, L, w, s + 1, v[k]);
       }
     }
@@ -87,69 +112,16 @@ struct KhopArgs {
   uint64_t seed;
 };
 
+// A warp's frontier group: transit i's record (degree 0: none) and first
+// output slot (parent index * fanout).
 struct SmemHdr {
-  uint64_t P[32];
-  uint32_t v[32], d[32], bn[32], bl[32], om[32], fp[32];
-  int a[32], b[32], cx[32];
-  uint64_t ob[32];  // k-hop: first output slot of transit i (parent index * fanout)
-  __device__ __forceinline__ void put(int i, const VHdr &h) {
-    P[i] = h.P; v[i] = h.v; d[i] = h.d; bn[i] = h.bn; bl[i] = h.bl; om[i] = h.om; fp[i] = h.fp;
-    a[i] = h.a; b[i] = h.b; cx[i] = h.cx;
-  }
-  __device__ __forceinline__ VHdr get(int i) const {
-    VHdr h;
-    h.P = P[i]; h.v = v[i]; h.d = d[i]; h.bn = bn[i]; h.bl = bl[i]; h.om = om[i]; h.fp = fp[i];
-    h.a = a[i]; h.b = b[i]; h.cx = cx[i];
-    return h;
-  }
+  uint4 rec[32];
+  uint64_t ob[32];
 };
 
 // Word k (0..3) of a Philox block held as four values.
 __device__ __forceinline__ uint32_t pick4(uint32_t x, uint32_t y, uint32_t z, uint32_t w, int k) {
   return k == 0 ? x : k == 1 ? y : k == 2 ? z : w;
-}
-
-// Per-lane staging of a k-hop draw's slot sector: 32 bytes copied by two
-// 16-byte cp.async (no registers held while the copy is in flight), in a
-// buffer of kDrawBufWords words (the sector, and the words that field reads
-// past its end may touch; a multiple of 16 bytes).
-constexpr uint32_t kDrawBufWords = 12;
-__device__ __forceinline__ void draw_copy(uint32_t *dst, const uint32_t *words, uint64_t sector) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  const uint32_t *src = words + sector * 8;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16), "l"(src + 4) : "memory");
-}
-__device__ __forceinline__ void draw_copy_wait() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-// A GT neighbor from its slot's words (slot at bit off): the head, then id gaps.
-__device__ __forceinline__ uint32_t gt_draw_w(const uint32_t *w, uint32_t off, uint32_t v,
-                                              uint32_t fp, int a, int b, uint32_t c,
-                                              uint32_t id) {
-  const uint32_t hv = word_field(w, off, a) + 1u;
-  uint32_t x = (c >= fp ? v + hv : v - hv) + id;
-  uint32_t at = off + (uint32_t)a;
-  for (uint32_t t = 0; t < id; t++, at += (uint32_t)b) x += word_field(w, at, b);
-  return x;
-}
-
-// An LE neighbor from its slot's words: the left rock (id 0), the right rock
-// (id == L), or the interpolated base plus the signed sea.
-__device__ __forceinline__ uint32_t le_draw_w(const uint32_t *w, uint32_t off, uint32_t v,
-                                              uint32_t fp, int a, int sb, uint32_t T, uint32_t c,
-                                              uint32_t id, uint32_t L) {
-  const uint32_t sw = (uint32_t)sb + 1u;
-  const uint32_t r1m = word_field(w, off, a);
-  const uint32_t r1 = c < fp ? v - r1m : v + r1m;
-  if (id == 0) return r1;
-  const uint32_t s0 = off + (uint32_t)a;
-  const uint32_t r2m = word_field(w, s0 + (T - 1) * sw, a);
-  const uint32_t r2 = c + 1 < fp ? v - r2m : v + r2m;
-  if (id == L) return r2;
-  // (r2 - r1) >= 0 for sorted rows: unsigned division is the compressor's
-  return word_sea(w, s0 + (id - 1) * sw, (int)sw, div_small(r2 - r1, L) * id + r1);
 }
 
 // With parts > 1, `parts` warps share the seed: warp `part` takes the subtrees
@@ -167,12 +139,11 @@ __device__ __forceinline__ uint32_t le_draw_w(const uint32_t *w, uint32_t off, u
 // lanes compute the group's Philox blocks once per 128 draws, lane l block l of
 // the window, and hand the words out by shuffles; otherwise each draw
 // computes its own block.  INFLIGHT: draws a lane has in flight at once (every
-// load is issued before any is decoded).  MODE 2 is the CSR (one column load
-// per draw).
+// load is issued before any is decoded).  On a CSR a draw is one column load.
 template <int MODE, int INFLIGHT = 1>
 __device__ __forceinline__ void khop_seed_warp(const DevGraph &g, const uint32_t *seeds,
                                                const KhopArgs &A, uint64_t s, SmemHdr &my,
-                                               uint32_t *dbuf, uint64_t &cnt, bool &bad,
+                                               uint64_t &cnt, bool &bad,
                                                uint32_t part = 0, uint32_t parts = 1) {
   static_assert(INFLIGHT == 1 || INFLIGHT == 2 || INFLIGHT == 4, "INFLIGHT in {1, 2, 4}");
   const int lane = threadIdx.x & 31;
@@ -202,18 +173,7 @@ __device__ __forceinline__ void khop_seed_warp(const DevGraph &g, const uint32_t
         ob = par * f;
         t = hop ? prev[par] : seeds[s];
       }
-      VHdr h;
-      if (t < g.n) {
-        h = header<MODE>(g, t);
-      } else {
-        h.d = 0;
-        h.P = 0;
-        h.v = t;
-        h.bn = h.bl = h.om = h.fp = 0;
-        h.cx = 0;
-        h.a = h.b = 0;
-      }
-      my.put(lane, h);
+      my.rec[lane] = t < g.n ? graph_record<MODE>(g, t) : make_uint4(0u, 0u, 0u, 0u);
       my.ob[lane] = ob;
       __syncwarp();
       const uint32_t nP = (uint32_t)min((uint64_t)G, P - pc);
@@ -236,107 +196,50 @@ __device__ __forceinline__ void khop_seed_warp(const DevGraph &g, const uint32_t
             rnd[u] = pick4(x, y, z, w, lane & 3);
           }
         }
-        if constexpr (MODE != 2) {
-          // phase 1: each draw's slot, its sector copied into this lane's buffer u
-          uint32_t di[INFLIGHT], dc[INFLIGHT], doff[INFLIGHT];
+        // phase 1: each draw's load; phase 2: its value, stored
+        Sec S[INFLIGHT];
+        DrawAt at[INFLIGHT];
+        uint32_t col[INFLIGHT];
 #pragma unroll
-          for (int u = 0; u < INFLIGHT; u++) {
-            const uint64_t j = j0 + (uint64_t)u * 32 + lane;
-            di[u] = dc[u] = doff[u] = 0;
-            if (j < total) {
-              const uint32_t pl = div_by((uint32_t)j, f, Mf);
-              const uint32_t d = my.d[pl];
-              if (d > (MODE == 1 ? 1u : 0u)) {  // (LE degree 1: the record holds it)
-                if (!contig) {
-                  const uint64_t slot = my.ob[pl] + ((uint32_t)j - pl * f);
-                  rnd[u] = pick(philox4x32_10(A.seed, (uint32_t)(slot >> 2), (uint32_t)s,
-                                              (uint32_t)(s >> 32), TAG_KHOP | hop),
-                                (int)(slot & 3));
-                }
-                const uint32_t i = mulhi_u32(rnd[u], d), T = my.bl[pl], K = my.om[pl];
-                // slot c of neighbor i (LE: neighbor d-1 is slot C-1's right rock)
-                const uint32_t c = div_small(MODE == 1 ? min(i, d - 2) : i, T);
-                const uint32_t q = div_small(c, K);
-                const uint64_t pos = my.P[pl] + (uint64_t)q * 256u + (uint64_t)(c - q * K) * (uint32_t)my.cx[pl];
-                draw_copy(dbuf + ((uint32_t)u * 32 + lane) * kDrawBufWords, g.words, pos >> 8);
-                di[u] = i;
-                dc[u] = c;
-                doff[u] = (uint32_t)pos & 255u;
-              }
-            }
+        for (int u = 0; u < INFLIGHT; u++) {
+          const uint64_t j = j0 + (uint64_t)u * 32 + lane;
+          if (j >= total) continue;
+          const uint32_t pl = div_by((uint32_t)j, f, Mf);
+          const VHdr h = record_header<MODE>(my.rec[pl]);
+          col[u] = h.base;  // (degree 1)
+          if (MODE == kCsr ? h.d == 0 : h.cb == 0) continue;
+          if (!contig) {
+            const uint64_t slot = my.ob[pl] + ((uint32_t)j - pl * f);
+            rnd[u] = pick(philox4x32_10(A.seed, (uint32_t)(slot >> 2), (uint32_t)s,
+                                        (uint32_t)(s >> 32), TAG_KHOP | hop),
+                          (int)(slot & 3));
           }
-          draw_copy_wait();
-          // phase 2: decode from the buffers, store
+          const uint32_t i = mulhi_u32(rnd[u], h.d);
+          if constexpr (MODE == kCsr) {
+            col[u] = load_cold_u32(g.cols + h.P + i);
+          } else {
+            at[u] = draw_at(h, i);
+            S[u] = load_sector(g.words, at[u].sec);
+          }
+        }
 #pragma unroll
-          for (int u = 0; u < INFLIGHT; u++) {
-            const uint64_t j = j0 + (uint64_t)u * 32 + lane;
-            if (j >= total) continue;
-            const uint32_t pl = div_by((uint32_t)j, f, Mf);
-            const uint32_t d = my.d[pl];
-            const uint64_t slot = contig ? sbase + j : my.ob[pl] + ((uint32_t)j - pl * f);
-            uint32_t nv = INVALID_VERTEX;
-            if (d > (MODE == 1 ? 1u : 0u)) {
-              const uint32_t *w = dbuf + ((uint32_t)u * 32 + lane) * kDrawBufWords;
-              const uint32_t T = my.bl[pl], id = di[u] - dc[u] * T;
-              if constexpr (MODE == 0) {
-                nv = gt_draw_w(w, doff[u], my.v[pl], my.fp[pl], my.a[pl], my.b[pl], dc[u], id);
-              } else {
-                const uint32_t L = min(T, d - 1 - dc[u] * T);
-                nv = le_draw_w(w, doff[u], my.v[pl], my.fp[pl], my.a[pl], my.b[pl], T, dc[u], id,
-                               L);
-              }
-            } else if (d == 1) {
-              nv = my.fp[pl];  // LE degree 1
-            }
-            if (d) {
-              if (nv >= g.n) {
-                bad = true;
-                nv = INVALID_VERTEX;
-              } else if (count) {
-                cnt++;
-              }
-            }
-            if (last_hop) store_out_u32(out + slot, nv);
-            else out[slot] = nv;  // read back by the next hop
+        for (int u = 0; u < INFLIGHT; u++) {
+          const uint64_t j = j0 + (uint64_t)u * 32 + lane;
+          if (j >= total) continue;
+          const uint32_t pl = div_by((uint32_t)j, f, Mf);
+          const VHdr h = record_header<MODE>(my.rec[pl]);
+          const uint64_t slot = contig ? sbase + j : my.ob[pl] + ((uint32_t)j - pl * f);
+          uint32_t nv = col[u];
+          if constexpr (MODE != kCsr)
+            if (h.cb) nv = draw_value(S[u], at[u], h);
+          const bool ok = nv < g.n;
+          if (h.d) {
+            bad |= !ok;
+            if (ok && count) cnt++;
           }
-        } else {  // CSR: one column load per draw
-          uint32_t col[INFLIGHT];
-#pragma unroll
-          for (int u = 0; u < INFLIGHT; u++) {
-            const uint64_t j = j0 + (uint64_t)u * 32 + lane;
-            col[u] = INVALID_VERTEX;
-            if (j < total) {
-              const uint32_t pl = div_by((uint32_t)j, f, Mf);
-              const uint32_t d = my.d[pl];
-              if (d) {
-                if (!contig) {
-                  const uint64_t slot = my.ob[pl] + ((uint32_t)j - pl * f);
-                  rnd[u] = pick(philox4x32_10(A.seed, (uint32_t)(slot >> 2), (uint32_t)s,
-                                              (uint32_t)(s >> 32), TAG_KHOP | hop),
-                                (int)(slot & 3));
-                }
-                col[u] = load_cold_u32(g.cols + my.P[pl] + mulhi_u32(rnd[u], d));
-              }
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < INFLIGHT; u++) {
-            const uint64_t j = j0 + (uint64_t)u * 32 + lane;
-            if (j >= total) continue;
-            const uint32_t pl = div_by((uint32_t)j, f, Mf);
-            const uint64_t slot = contig ? sbase + j : my.ob[pl] + ((uint32_t)j - pl * f);
-            uint32_t nv = col[u];
-            if (my.d[pl]) {
-              if (nv >= g.n) {
-                bad = true;
-                nv = INVALID_VERTEX;
-              } else if (count) {
-                cnt++;
-              }
-            }
-            if (last_hop) store_out_u32(out + slot, nv);
-            else out[slot] = nv;  // read back by the next hop
-          }
+          nv = h.d && ok ? nv : INVALID_VERTEX;
+          if (last_hop) store_out_u32(out + slot, nv);
+          else out[slot] = nv;  // read back by the next hop
         }
       }
       __syncwarp();
@@ -449,7 +352,7 @@ __device__ __forceinline__ void mrw_warp(const DevGraph &g, uint32_t *vtx, uint4
         if (od == 0) {
           dst[io] = INVALID_VERTEX;
         } else {
-          const VHdr h = record_header<MODE>(r, v);
+          const VHdr h = record_header<MODE>(r);
           const uint32_t nv = neighbor<MODE>(g, h, mulhi_u32(ry, h.d));
           if (nv >= g.n) {
             bad = true;

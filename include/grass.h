@@ -143,22 +143,15 @@ int grass_get_info(const grass_graph *g, grass_graph_info *info);
  * GRASS_OK.  The _host calls check it themselves. */
 int grass_check_device_error(grass_graph *g, void *stream);
 /* Device view of the resident graph (for callers that launch their own
- * kernels): the stream words (n_words + at least 16 zero guard words, each
- * word the next 32 stream bits MSB-first) and the n vertex records, 16 bytes
- * each: {P low 32 bits, P bits 32..47 | a << 16 | b << 22, degree, w}, where
- * P is the bit offset of the vertex's payload, a/b are the GT head/body or LE
- * rock/sea widths, and w is first_pos (LE degree 1: the single neighbor; GT:
- * first_pos in bits 0..15 and the skip-field extra width cx in bits 16..21).
- * The records replace the reference's uint64 bit-offset table
- * (GT/src/utils.hpp:363).  The stream is the .graph stream re-laid for random
- * access, the field values unchanged:
- *   LE: the file's stream; the payload of every vertex whose longest chunk
- *       spans at most 256 bits (2 rock_bit + its seas x (sea_bit + 1)) is in
- *       neighbor order, [rock 0][seas of chunk 0][rock 1]...[last rock],
- *       instead of all rocks then all seas (same bits, same P);
- *   GT: the payloads only, back to back in vertex order; in every block the
- *       field at each position t = 16, 32, ... holds the sum of the block's
- *       raw gaps 1..t in b + cx bits instead of gap t. */
+ * kernels): the slot words (n_words + at least 16 zero guard words, each word
+ * the next 32 bits MSB-first) and the n vertex records, 16 bytes each, which
+ * replace the reference's uint64 bit-offset table (GT/src/utils.hpp:363).
+ * The layout is the library's own, the same for GT and LE files: neighbors
+ * cT .. cT + T - 1 of a vertex share slot c,
+ *   [head n_cT - n_0 (a bits)][offsets n_i - n_cT (b bits) of i = cT+1 ..],
+ * of cb = a + (T - 1) b bits at bit P + (c / K) 256 + (c % K) cb, inside one
+ * 32-byte sector.  Record: x = P low 32 bits; y = P bits 32..39 | a << 8 |
+ * b << 14 | T << 20 | K << 26; z = degree; w = n_0 (degree 1: no slot). */
 int grass_device_view(const grass_graph *g, const uint32_t **words, uint64_t *n_words,
                       const void **records);
 
