@@ -523,33 +523,63 @@ __global__ void __launch_bounds__(256) decode_range_kernel(DevGraph g, const uin
 // A warp takes one item of the flat plan: a run of consecutive vertices
 // [v0, v1) (w == 0), or one vertex's neighbor range [z, w) (hubs, degree >=
 // kFlatHub).  It walks a run 32 vertices at a time (lane k loads vertex k's
-// record) and decodes one neighbor per lane, straight to the CSR:
-//  * vertices of degree >= 32 one after another (flat_big): everything but
-//    the lane's place in the slots is warp-uniform, and that place advances by
-//    a constant from one round of 32 neighbors to the next;
+// record) and decodes one neighbor per lane, straight to the CSR; a neighbor is
+// n_0 + head + offset, two fields of one slot, so lanes need nothing from one
+// another:
+//  * vertices of degree >= kFlatBig one after another (flat_big), from sectors
+//    staged in shared memory;
 //  * the other vertices together: their neighbors are numbered by a warp scan,
 //    and in a round of 32 each lane finds its vertex from the bit mask of the
 //    vertices that start in the round (one OR-reduction and a population
-//    count).
-// A neighbor is n_0 + head + offset, two fields of one slot, so lanes need
-// nothing from one another.  R-MAT s21 ef16, 63 M neighbors: 0.259 ms a sweep;
-// one lane per slot took 0.466 ms on this layout (slots of 3 neighbors leave
-// most of the work to per-slot set-up) and 0.340 ms on LE's own code.
-constexpr uint32_t kFlatHub = kRange;  // degree from which a vertex is split into ranges
-constexpr uint32_t kFlatBig = 32;      // degree from which a vertex is decoded by itself
-
-// Resident 256-thread blocks per SM.
-#ifndef GRASS_DECODE_FLAT_MIN_BLOCKS
-#define GRASS_DECODE_FLAT_MIN_BLOCKS 4
+//    count), and reads its fields through L1.
+// It is bound by instruction issue (67 % of the slots, 117 M warp instructions
+// on R-MAT s21 ef16, 63 M neighbors).  The whole decode there took 0.341 ms
+// with one lane per slot of LE's own code, 0.466 ms the same way on this layout
+// (its slots hold 3 neighbors, so the set-up of a slot is most of the work),
+// 0.259 ms with one neighbor per lane whose place in the slots advances by
+// wrapping counters, and takes 0.173 ms this way.
+#ifndef GRASS_FLAT_VERTEX
+#define GRASS_FLAT_VERTEX 16
 #endif
+// A vertex's share of an item beside its neighbors (32: 0.180 against 0.178 ms).
+constexpr uint32_t kFlatVertex = GRASS_FLAT_VERTEX;
+#ifndef GRASS_FLAT_BIG
+#define GRASS_FLAT_BIG 128
+#endif
+constexpr uint32_t kFlatHub = kRange;  // degree from which a vertex is split into ranges
+// Degree from which a vertex is decoded by itself: its set-up is some 250 warp
+// instructions, and a round of 32 neighbors then takes about 25, against 70 in
+// a group (0.173 ms at 128, 0.178 at 256; at most 2048, see FlatSmem::vb).
+constexpr uint32_t kFlatBig = GRASS_FLAT_BIG;
+
+// Warps per block, one item each, and resident blocks per SM (64 registers).
+// Items differ in cost, and a block's place is free only when its last warp is
+// done: two warps a block ran the sweep in 0.178 ms, eight in 0.191; 12 or 20
+// blocks in 0.196 and 0.191.
+#ifndef GRASS_FLAT_WARPS
+#define GRASS_FLAT_WARPS 2
+#endif
+#ifndef GRASS_DECODE_FLAT_MIN_BLOCKS
+#define GRASS_DECODE_FLAT_MIN_BLOCKS 16
+#endif
+constexpr int kFlatWarps = GRASS_FLAT_WARPS;
 
 // A warp's share of shared memory.
 struct FlatSmem {
   uint32_t stage[32 * 8 + 4];  // 32 sectors, and the word that a field's read may touch
-  uint4 rec[32];               // the round's small vertices with neighbors, in order:
-  uint64_t ob[32];             // record, first entry in the CSR,
-  uint32_t ex[32];             // number of the first neighbor in the group
+  // the group's small vertices with neighbors, in order:
+  uint4 va[32];  // n_0; sector; bit in it | a << 8 | b << 14 | T << 20 | K << 26; first
+                 // neighbor's number in the group
+  uint4 vb[32];  // 2^16 / T and 2^16 / K rounded up; cb; first entry in the CSR less the
+                 // number of the first neighbor, from the group's first entry
 };
+
+// Copies one word to shared memory through L1, which brings its sector there
+// and holds no register while it is on the way.
+__device__ __forceinline__ void prefetch_l1(uint32_t *dump, const uint32_t *p) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dump)), "l"(p) : "memory");
+}
+__device__ __forceinline__ void prefetch_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // The field of `width` (0..32) bits at bit `off` from word w.
 __device__ __forceinline__ uint32_t word_field(const uint32_t *w, uint32_t off, uint32_t width) {
@@ -557,65 +587,114 @@ __device__ __forceinline__ uint32_t word_field(const uint32_t *w, uint32_t off, 
   return shr_clamp(__funnelshift_l(q[1], q[0], off), 32u - width);
 }
 
+// Where the bits of one neighbor are: the shared-memory addresses of the words
+// of its slot's head and of its offset, the bits in those words, and 32 less
+// the offset's width (a slot's first neighbor has none).
+struct Place {
+  uint32_t head, head_bit, off, off_bit, drop;
+};
+__device__ __forceinline__ Place place_of(const VHdr &h, uint32_t r, uint32_t stage) {
+  const uint32_t c = div_small(r, h.T), id = r - c * h.T;  // neighbor r of a sector
+  const uint32_t hb = h.off + c * h.cb, ob = id ? hb + h.a + (id - 1) * h.b : hb;
+  return Place{stage + (hb >> 5) * 4, hb, stage + (ob >> 5) * 4, ob, id ? 32 - h.b : 32u};
+}
+__device__ __forceinline__ uint32_t lds_bits(uint32_t addr, uint32_t bit, uint32_t drop) {
+  uint32_t hi, lo;
+  asm volatile("ld.shared.u32 %0, [%2];\n\tld.shared.u32 %1, [%2+4];" : "=r"(hi), "=r"(lo) : "r"(addr));
+  return shr_clamp(__funnelshift_l(lo, hi, bit), drop);
+}
+
 // Neighbors [i0, i1) of a vertex of header h (warp-uniform, cb > 0) to
-// out[i0 .. i1).  The vertex's sectors are consecutive, so the warp copies 32
-// at a time into shared memory with two 16-byte loads a lane, the next 32
-// already on their way in registers, and reads the fields from there.
+// out[i0 .. i1); vmax: the largest value written so far.  A sector holds N = T
+// K neighbors, and the vertex's sectors are consecutive.  The warp copies up to
+// 32 of them at a time into shared memory with two 16-byte loads a lane, the
+// next ones already on their way in registers, and decodes R = 64 / N whole
+// sectors per round, two neighbors a lane: so a lane's places in the R sectors
+// stay the same from round to round, and a neighbor costs its field reads, one
+// add and the store.
 __device__ __forceinline__ void flat_big(const uint32_t *words, const VHdr &h, uint32_t i0,
-                                         uint32_t i1, uint32_t n, uint32_t *out, uint32_t *stage,
-                                         bool &bad) {
+                                         uint32_t i1, uint32_t *out, uint32_t *stage,
+                                         uint32_t &vmax) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t T = h.T, K = h.K, N = T * K;  // N neighbors a sector
-  const uint32_t q0 = div_small(div_small(i0, T), K);
-  const uint32_t nq = div_small(div_small(i1 - 1, T), K) - q0 + 1;
-  // the lane's place in a chunk of sectors, and its advance per round
-  const uint32_t dT = div_small(32u, T), rT = 32u - dT * T, dK = div_small(dT, K), rK = dT - dK * K;
-  const uint32_t c0 = div_small(lane, T), id0 = lane - c0 * T;
-  const uint32_t k0 = div_small(c0, K), s0 = c0 - k0 * K;
+  const uint32_t N = h.T * h.K;
+  const uint32_t q0 = i0 ? div_small(div_small(i0, h.T), h.K) : 0u;
+  const uint32_t nq = div_small(div_small(i1 - 1, h.T), h.K) - q0 + 1;
+  const uint32_t R = N < 64 ? div_small(64u, N) : 1u;
+  const uint32_t chunk = div_small(32u, R) * R;  // sectors staged at a time
+  const uint32_t len = i1 - i0, st = smem_u32(stage);
+  // the lane's places in a round, and its neighbors there (from i0): a lane
+  // without one (R N < 64) reads place 0 and is never inside [0, len)
+  Place pl[2];
+  uint32_t j[2];
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const uint32_t p = u * 32 + lane, k = N < 64 ? div_small(p, N) : 0u;
+    const bool ok = k < R;
+    pl[u] = place_of(h, ok ? p - k * N : 0u, st + (ok ? k * 32 : 0u));
+    j[u] = ok ? q0 * N + p - i0 : 1u << 31;
+  }
   const uint4 *src = reinterpret_cast<const uint4 *>(words + (uint64_t)(h.sec + q0) * 8) + lane;
   uint4 *dst = reinterpret_cast<uint4 *>(stage) + lane;
   const uint32_t half = lane >> 1;  // the lane's sector of 16
   uint4 x = make_uint4(0, 0, 0, 0), y = x;
   if (half < nq) x = __ldg(src);
   if (half + 16 < nq) y = __ldg(src + 32);
-  for (uint32_t q = 0; q < nq; q += 32) {  // warp-uniform
+  uint32_t *o = out + (q0 * N + lane);
+  for (uint32_t q = 0; q < nq; q += chunk) {  // warp-uniform
     dst[0] = x;
     dst[32] = y;
     __syncwarp();
-    src += 64;
-    if (q + 32 + half < nq) x = __ldg(src);
-    if (q + 48 + half < nq) y = __ldg(src + 32);
-    const uint32_t j0 = (q0 + q) * N, j1 = min(i1, j0 + 32u * N);
-    uint32_t k = k0, s = s0, id = id0;
-    for (uint32_t i = j0 + lane; i < j1; i += 32) {
-      const uint32_t *w = stage + k * 8;
-      const uint32_t at = h.off + s * h.cb;
-      uint32_t v = h.base + word_field(w, at, h.a);
-      if (T > 1) v += word_field(w, id ? at + h.a + (id - 1) * h.b : at, id ? h.b : 0u);
-      bad |= v >= n;
-      if (i >= i0) out[i] = v;
-      id += rT;
-      s += rK;
-      k += dK;
-      if (id >= T) id -= T, s++;
-      if (s >= K) s -= K, k++;
+    src += 2 * chunk;
+    if (q + chunk + half < nq) x = __ldg(src);
+    if (q + chunk + half + 16 < nq) y = __ldg(src + 32);
+    const uint32_t end = min(chunk, nq - q);
+    uint32_t at = 0;  // byte offset of the round's first sector
+    for (uint32_t e = 0; e < end; e += R) {
+      uint32_t v[2];
+#pragma unroll
+      for (int u = 0; u < 2; u++) v[u] = h.base + lds_bits(pl[u].head + at, pl[u].head_bit, 32 - h.a);
+      if (h.T > 1) {  // (warp-uniform)
+#pragma unroll
+        for (int u = 0; u < 2; u++) v[u] += lds_bits(pl[u].off + at, pl[u].off_bit, pl[u].drop);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        if (j[u] < len) {
+          o[u * 32] = v[u];
+          vmax = max(vmax, v[u]);
+        }
+        j[u] += R * N;
+      }
+      if (N > 64) {  // the rest of a sector of more than 64 neighbors
+        for (uint32_t r = 64 + lane; r < N; r += 32) {
+          const uint32_t i = (q0 + q + e) * N + r;
+          const Place p = place_of(h, r, st + at);
+          const uint32_t w = h.base + lds_bits(p.head, p.head_bit, 32 - h.a) + lds_bits(p.off, p.off_bit, p.drop);
+          if (i - i0 < len) {
+            out[i] = w;
+            vmax = max(vmax, w);
+          }
+        }
+      }
+      o += R * N;
+      at += R * 32;
     }
     __syncwarp();
   }
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(256, GRASS_DECODE_FLAT_MIN_BLOCKS) decode_flat_kernel(DevGraph g, const uint64_t *__restrict__ rowptr,
+__global__ void __launch_bounds__(32 * kFlatWarps, GRASS_DECODE_FLAT_MIN_BLOCKS) decode_flat_kernel(DevGraph g, const uint64_t *__restrict__ rowptr,
                                                           uint32_t *__restrict__ cols,
                                                           const uint4 *__restrict__ items,
                                                           uint64_t nitems, unsigned int *err) {
-  __shared__ __align__(16) FlatSmem smem[8];
+  __shared__ __align__(16) FlatSmem smem[kFlatWarps];
   FlatSmem &sm = smem[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t upto = 0xFFFFFFFFu >> (31 - lane);  // this lane and those below
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  bool bad = false;
+  uint32_t vmax = 0;
   for (uint64_t t = warp; t < nitems; t += nwarps) {
     const uint4 it = items[t];
     const bool run = it.w == 0;
@@ -637,53 +716,67 @@ __global__ void __launch_bounds__(256, GRASS_DECODE_FLAT_MIN_BLOCKS) decode_flat
         const uint32_t y = __shfl_up_sync(FULL, incl, o);
         if (lane >= (uint32_t)o) incl += y;
       }
-      const uint32_t ex = incl - d, total = __shfl_sync(FULL, incl, 31);
+      const uint32_t ex = d ? incl - d : 0xFFFFFFFFu, total = __shfl_sync(FULL, incl, 31);
       const unsigned has = __ballot_sync(FULL, d > 0);
+      const uint64_t ob0 = __shfl_sync(FULL, ob, 0);
       if (d) {
+        const VHdr h = record_header<MODE>(r);
         const uint32_t at = __popc(has & upto) - 1;
-        sm.rec[at] = r;
-        sm.ob[at] = ob;
-        sm.ex[at] = ex;
+        sm.va[at] = make_uint4(h.base, h.sec, h.off | (r.y & ~0xFFu), ex);
+        sm.vb[at] = make_uint4(65535u / h.T + 1, 65535u / h.K + 1, h.cb, (uint32_t)(ob - ob0) - ex);
+        // bring the vertex's lines into L1 (a word of each into a dump) while
+        // the others are set up
+        const uint32_t lines = h.cb ? (div_small(div_small(d - 1, h.T), h.K) + (h.sec & 3u)) / 4 + 1 : 0;
+        const uint32_t *p = g.words + (uint64_t)(h.sec & ~3u) * 8;
+#pragma unroll
+        for (uint32_t l = 0; l < kFlatBig * 32 / 1024 + 2; l++)
+          if (l < lines) prefetch_l1(&sm.stage[lane], p + l * 32);
       }
       __syncwarp();
-      uint32_t before = 0;  // vertices that start before the round
+      uint32_t *out0 = cols + ob0;
+      uint32_t before = 0xFFFFFFFFu;  // the vertices that start before the round, less one
       for (uint32_t j = 0; j < total; j += 32) {
-        const unsigned starts =
-            __reduce_or_sync(FULL, d && ex >= j && ex < j + 32 ? 1u << (ex - j) : 0u);
-        const uint32_t own = before + __popc(starts & upto) - 1;
+        const unsigned starts = __reduce_or_sync(FULL, __funnelshift_lc(0u, 1u, ex - j));
+        const uint32_t own = before + __popc(starts & upto);
         before += __popc(starts);
         if (j + lane < total) {
-          const VHdr h = record_header<MODE>(sm.rec[own]);
-          const uint32_t i = j + lane - sm.ex[own];
-          uint32_t x = h.base;
-          if (h.cb) {
-            const DrawAt at = draw_at(h, i);
-            const uint32_t *w = g.words + (uint64_t)at.sec * 8;
-            if (h.a) x += word_field(w, at.off, h.a);
-            if (at.id) x += word_field(w, at.off + h.a + (at.id - 1) * h.b, h.b);
-          }
-          bad |= x >= g.n;
-          cols[sm.ob[own] + i] = x;
+          const uint4 A = sm.va[own], B = sm.vb[own];
+          // neighbor i of its vertex: slot c, index id; exact for i < 2048
+          const uint32_t i = j + lane - A.w;
+          const uint32_t c = (i * B.x) >> 16, id = i - c * ((A.z >> 20) & 63u);
+          const uint32_t q = (c * B.y) >> 16, at = (A.z & 255u) + (c - q * (A.z >> 26)) * B.z;
+          const uint32_t *w = g.words + (uint64_t)(A.y + q) * 8;
+          const uint32_t a = (A.z >> 8) & 63u, b = (A.z >> 14) & 63u;
+          uint32_t x = A.x;
+          if (a) x += word_field(w, at, a);
+          if (id) x += word_field(w, at + a + (id - 1) * b, b);
+          vmax = max(vmax, x);
+          out0[B.w + j + lane] = x;
         }
       }
+      prefetch_wait();  // (before the dump is used again)
+      __syncwarp();
       // the large ones
       for (unsigned m = __ballot_sync(FULL, big); m; m &= m - 1) {
         const int k = __ffs(m) - 1;
         const VHdr h = record_header<MODE>(shfl_rec(r, k));
         uint32_t *out = cols + __shfl_sync(FULL, ob, k);
-        flat_big(g.words, h, run ? 0u : it.z, run ? h.d : it.w, g.n, out, sm.stage, bad);
+        flat_big(g.words, h, run ? 0u : it.z, run ? h.d : it.w, out, sm.stage, vmax);
       }
       __syncwarp();  // the group's shared memory is free
     }
   }
-  if (bad && err) atomicOr(err, 1u);
+  if (vmax >= g.n && err) atomicOr(err, 1u);
 }
 
 // Flat plan: items in vertex order.  One warp per chunk of kPlanChunk
 // vertices.  A vertex of degree >= kFlatHub becomes ceil(d / kRange) range
 // items (v, v + 1, i0, i1); the others form runs, a run starting at the
-// chunk's first vertex, after a hub, and wherever the chunk's running degree
-// sum crosses a multiple of kRange.  Runs get (v0, 0, 0, 0) here; their end
+// chunk's first vertex, after a hub, and wherever the chunk's running sum of
+// degree + kFlatVertex crosses a multiple of kRange: a group of 32 vertices
+// costs the latency of its records however few neighbors it has, and without
+// the second term the runs of low-degree vertices, which come last in
+// graph_sort's order, held most warps idle at the end of the sweep.  Runs get (v0, 0, 0, 0) here; their end
 // is the next item's first vertex (flat_plan_link_kernel).
 template <bool FILL>
 __global__ void flat_plan_kernel(const uint4 *__restrict__ recs, uint32_t n, uint32_t nchunks,
@@ -695,20 +788,21 @@ __global__ void flat_plan_kernel(const uint4 *__restrict__ recs, uint32_t n, uin
   const uint32_t v0 = warp * kPlanChunk, v1 = min(n, v0 + kPlanChunk);
   unsigned long long cur = FILL ? cursors[warp] : 0ull;
   uint32_t tot = 0;
-  uint64_t carry = 0;       // degree sum of the chunk's vertices before this sub-chunk
+  uint64_t carry = 0;       // the chunk's sum before this sub-chunk
   bool prev_hub = true;     // (the chunk's first vertex starts a run)
   uint64_t prev_win = 0;
   for (uint32_t b = v0; b < v1; b += 32) {
     const uint32_t v = b + lane;
     const uint32_t d = v < v1 ? recs[v].z : 0u;
     const bool hub = v < v1 && d >= kFlatHub;
-    uint64_t incl = d;
+    const uint32_t cost = d + kFlatVertex;
+    uint64_t incl = cost;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint64_t y = __shfl_up_sync(FULL, incl, o);
       if (lane >= o) incl += y;
     }
-    const uint64_t pre = carry + incl - d;  // chunk degree sum before v
+    const uint64_t pre = carry + incl - cost;  // the chunk's sum before v
     const uint64_t win = pre / kRange;
     const uint32_t hub_up = __shfl_up_sync(FULL, (uint32_t)hub, 1);
     const bool ph = lane ? hub_up != 0u : prev_hub;
@@ -858,9 +952,9 @@ static void launch_flat(const grass_graph *g, const uint64_t *rowptr, uint32_t *
                         unsigned int *err, cudaStream_t s) {
   if (!g->plan_nflat) return;
   const DevGraph v = g->view();
-  const unsigned grid = (unsigned)std::max<uint64_t>(
-      1, std::min<uint64_t>((g->plan_nflat + 7) / 8, (uint64_t)sm_count(g->device) * 8));
-  decode_flat_kernel<kSlots><<<grid, 256, 0, s>>>(v, rowptr, cols, g->d_plan_flat, g->plan_nflat, err);
+  const unsigned grid =
+      (unsigned)std::min<uint64_t>((g->plan_nflat + kFlatWarps - 1) / kFlatWarps, 1u << 30);
+  decode_flat_kernel<kSlots><<<grid, 32 * kFlatWarps, 0, s>>>(v, rowptr, cols, g->d_plan_flat, g->plan_nflat, err);
   count_launch();
 }
 
