@@ -809,7 +809,7 @@ int grass_mrw(const grass_graph *g, const grass_mrw_params *p, uint32_t *d_roots
     return set_error(GRASS_E_ARG, "multi-RW: bad arguments");
   DeviceGuard dg(g->device);
   if (int rc = launch_mrw(g->view(), *p, d_roots, S, d_src, d_dst, d_edge_count, g->d_err,
-                          as_stream(stream)))
+                          g->info.max_degree, as_stream(stream)))
     return rc;
   return check_launch();
 }
@@ -833,7 +833,7 @@ int grass_mrw_host(const grass_graph *g, const grass_mrw_params *p, uint32_t *h_
   GRASS_CUDA(cudaMemsetAsync(de.p, 0, 8, st));
   GRASS_CUDA(cudaMemcpyAsync(dr.p, h_roots, nr * 4, cudaMemcpyHostToDevice, st));
   if (int rc = launch_mrw(g->view(), *p, (uint32_t *)dr.p, S, (uint32_t *)dsrc.p,
-                          (uint32_t *)ddst.p, (unsigned long long *)de.p, g->d_err, st))
+                          (uint32_t *)ddst.p, (unsigned long long *)de.p, g->d_err, g->info.max_degree, st))
     return rc;
   if (int rc = check_launch()) return rc;
   GRASS_CUDA(cudaMemcpyAsync(h_roots, dr.p, nr * 4, cudaMemcpyDeviceToHost, st));

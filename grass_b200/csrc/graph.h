@@ -231,7 +231,7 @@ void launch_khop_csr(const DevCsr &c, const grass_khop_params &p, const uint32_t
                      cudaStream_t s);
 int launch_mrw(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots, uint64_t S,
                uint32_t *src, uint32_t *dst, unsigned long long *edges, unsigned int *err,
-               cudaStream_t s);
+               uint32_t max_degree, cudaStream_t s);
 
 // ---- output compaction (kernels_compact.cu) ----
 constexpr uint32_t kCompactMaxSegs = GRASS_MAX_HOPS;

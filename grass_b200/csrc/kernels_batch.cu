@@ -87,9 +87,9 @@ __global__ void __launch_bounds__(256, GRASS_BATCH_MIN_BLOCKS) batch_kernel(DevG
             jb.roots[s * jb.walkers + w] = mrw_root(g.n, jb.seed, s * jb.walkers + w);
           __syncwarp();
         }
-        mrw_warp<MODE>(g, jb.roots + s * jb.walkers,
-                       reinterpret_cast<uint4 *>(jb.mscr + s * jb.mstride), jb.walkers,
-                       jb.steps, (int)jb.select, jb.seed, s, jb.out0, jb.out1, cnt, bad);
+        mrw_degree_warp<MODE>(g, jb.roots + s * jb.walkers,
+                              reinterpret_cast<uint4 *>(jb.mscr + s * jb.mstride), jb.walkers,
+                              jb.steps, jb.seed, s, jb.out0, jb.out1, cnt, bad);
       }
     }
 #pragma unroll

@@ -383,73 +383,108 @@ __global__ void __launch_bounds__(256, GRASS_KHOP_MIN_BLOCKS) khop_csr_kernel(De
 }
 
 // ---------------------------------------------------------------------------
-// Multi random walk.  One warp per sample; the walkers' vertices, degrees and
-// a Fenwick tree of degrees (degree-proportional selection) live in shared
-// memory; lane 0 runs the step chain, which is sequential by definition.
+// Multi random walk.
 
-// Shared-memory state of one sample: vertices (16-byte padded) + records.
-struct MrwLayout {
-  uint32_t R;
-  __host__ __device__ size_t vtx_bytes() const { return ((size_t)R * 4 + 15) / 16 * 16; }
-  __host__ __device__ size_t bytes_per_warp() const { return vtx_bytes() + (size_t)R * 16; }
-};
+// Uniform selection, one warp per sample, the walkers' vertices in shared
+// memory (SMEM) or in place.
+template <int MODE, bool SMEM>
+__device__ __forceinline__ void mrw_uniform_samples(const DevGraph &g, uint32_t *roots, uint64_t S,
+                                                    uint32_t R, uint32_t T, uint64_t seed,
+                                                    uint32_t *src, uint32_t *dst,
+                                                    uint32_t *smem, uint64_t &cnt, bool &bad) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t s = warp; s < S; s += nwarps) {
+    uint32_t *rt = roots + s * R;
+    if constexpr (SMEM) {
+      for (uint32_t i = lane; i < R; i += 32) smem[i] = rt[i];
+      __syncwarp();
+      mrw_uniform_warp<MODE>(g, smem, R, T, seed, s, src, dst, cnt, bad);
+      for (uint32_t i = lane; i < R; i += 32) rt[i] = smem[i];
+      __syncwarp();
+    } else {
+      mrw_uniform_warp<MODE>(g, rt, R, T, seed, s, src, dst, cnt, bad);
+    }
+  }
+}
 
-// Multi random walk, one sample per warp, the sample's state in shared memory.
-// Resident 256-thread blocks per SM it is compiled for: each warp's step chain
-// waits on dependent record and sector reads, so resident warps pay.  On
-// 262,144 samples of 80 walkers x 100 steps (R-MAT s22 ef32) 4 blocks (64
-// registers) ran 1.6x (LE) and 1.7x (GT) faster than the unbounded build
-// (110-113 registers, 2 blocks), 1.25x faster than 3 blocks, and 1.1-1.2x
-// faster than 5 or 6 (48 / 40 registers).
+// Resident 256-thread blocks per SM: every lane waits on dependent record and
+// sector reads, so resident warps pay.
 #ifndef GRASS_MRW_MIN_BLOCKS
-#define GRASS_MRW_MIN_BLOCKS 4
+#define GRASS_MRW_MIN_BLOCKS 6
 #endif
 
 template <int MODE>
 __global__ void __launch_bounds__(256, GRASS_MRW_MIN_BLOCKS) mrw_kernel(DevGraph g, uint32_t *__restrict__ roots,
-                                                  uint64_t S, uint32_t R, uint32_t T, int select,
-                                                  uint64_t seed, uint32_t *__restrict__ src,
+                                                  uint64_t S, uint32_t R, uint32_t T, uint64_t seed,
+                                                  uint32_t *__restrict__ src,
                                                   uint32_t *__restrict__ dst,
                                                   unsigned long long *edges, unsigned int *err) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const MrwLayout lay{R};
-  const int lane = threadIdx.x & 31;
-  unsigned char *base = smem + (threadIdx.x >> 5) * lay.bytes_per_warp();
-  uint32_t *vtx = reinterpret_cast<uint32_t *>(base);
-  uint4 *rec = reinterpret_cast<uint4 *>(base + lay.vtx_bytes());
-  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  extern __shared__ uint32_t walkers[];  // R words a warp
   uint64_t cnt = 0;
   bool bad = false;
-  for (uint64_t s = warp; s < S; s += nwarps) {
-    uint32_t *rt = roots + s * R;
-    for (uint32_t i = lane; i < R; i += 32) vtx[i] = rt[i];
-    __syncwarp();
-    mrw_warp<MODE>(g, vtx, rec, R, T, select, seed, s, src, dst, cnt, bad);
-    __syncwarp();
-    for (uint32_t i = lane; i < R; i += 32) rt[i] = vtx[i];
-    __syncwarp();
-  }
+  mrw_uniform_samples<MODE, true>(g, roots, S, R, T, seed, src, dst,
+                                  walkers + (threadIdx.x >> 5) * R, cnt, bad);
   warp_add_u64(edges, cnt);
   if (bad && err) atomicOr(err, 1u);
 }
 
-// Same with the state in global memory (roots in place, rec = S*R records of
-// scratch): any number of walkers per sample.
+// The same with more walkers than shared memory holds.
 template <int MODE>
-__global__ void __launch_bounds__(256) mrw_global_kernel(DevGraph g, uint32_t *__restrict__ roots,
-                                                         uint4 *__restrict__ rec, uint64_t S,
-                                                         uint32_t R, uint32_t T, int select,
-                                                         uint64_t seed, uint32_t *__restrict__ src,
+__global__ void __launch_bounds__(256) mrw_global_kernel(DevGraph g, uint32_t *roots, uint64_t S,
+                                                         uint32_t R, uint32_t T, uint64_t seed,
+                                                         uint32_t *__restrict__ src,
                                                          uint32_t *__restrict__ dst,
                                                          unsigned long long *edges,
                                                          unsigned int *err) {
+  uint64_t cnt = 0;
+  bool bad = false;
+  mrw_uniform_samples<MODE, false>(g, roots, S, R, T, seed, src, dst, nullptr, cnt, bad);
+  warp_add_u64(edges, cnt);
+  if (bad && err) atomicOr(err, 1u);
+}
+
+// Degree-proportional selection, G lanes per sample (8, or 32 with more walkers
+// than a lane should search).  With rec == nullptr the state (R records, then R
+// vertices a sample) lives in shared memory, else (G = 32) the records in rec
+// (S R of them) and the vertices in place.
+#ifndef GRASS_MRW_DEGREE_MIN_BLOCKS
+#define GRASS_MRW_DEGREE_MIN_BLOCKS 4
+#endif
+template <int MODE, int G, class Sum>
+__global__ void __launch_bounds__(256, GRASS_MRW_DEGREE_MIN_BLOCKS)
+    mrw_degree_kernel(DevGraph g, uint32_t *roots, uint4 *rec, uint64_t S, uint32_t R, uint32_t T,
+                      uint64_t seed, uint32_t *__restrict__ src, uint32_t *__restrict__ dst,
+                      unsigned long long *edges, unsigned int *err) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  constexpr uint32_t P = 32 / G;  // samples per warp
+  const uint32_t gl = threadIdx.x & (G - 1), grp = threadIdx.x / G;
+  uint4 *srec = reinterpret_cast<uint4 *>(smem) + (uint64_t)grp * R;
+  uint32_t *svtx = reinterpret_cast<uint32_t *>(smem + (uint64_t)(blockDim.x / G) * R * 16) + (uint64_t)grp * R;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   uint64_t cnt = 0;
   bool bad = false;
-  for (uint64_t s = warp; s < S; s += nwarps)
-    mrw_warp<MODE>(g, roots + s * R, rec + s * R, R, T, select, seed, s, src, dst, cnt, bad);
+  for (uint64_t s0 = warp * P; s0 < S; s0 += nwarps * P) {  // warp-uniform
+    const uint64_t s = s0 + (threadIdx.x & 31) / G;
+    const bool live = s < S;
+    uint32_t *rt = roots + s * R;
+    if (G == 32 && rec) {
+      mrw_degree_warp<MODE>(g, rt, rec + s * R, R, T, seed, s, src, dst, cnt, bad);
+      continue;
+    }
+    if (live)
+      for (uint32_t i = gl; i < R; i += G) svtx[i] = rt[i];
+    __syncwarp();
+    if constexpr (G == 32)
+      mrw_degree_warp<MODE>(g, svtx, srec, R, T, seed, s, src, dst, cnt, bad);
+    else
+      mrw_degree_group<MODE, G, Sum>(g, live, svtx, srec, R, T, seed, s, src, dst, cnt, bad);
+    if (live)
+      for (uint32_t i = gl; i < R; i += G) rt[i] = svtx[i];
+    __syncwarp();
+  }
   warp_add_u64(edges, cnt);
   if (bad && err) atomicOr(err, 1u);
 }
@@ -719,58 +754,80 @@ void launch_khop_csr(const DevCsr &c, const grass_khop_params &p, const uint32_t
   count_launch();
 }
 
+// Warps per block (a power of two up to 8) for `warps` warps of work, each
+// with `bytes` of shared memory: at most 48 KB a block, and no more warps than
+// spread the work over the SMs.
+static int mrw_block_warps(uint64_t warps, size_t bytes) {
+  int w = 8;
+  while (w > 1 && (w * bytes > 48 * 1024 || warps < (uint64_t)sm_count(cur_dev()) * w)) w /= 2;
+  return w;
+}
+
+template <int G, class Sum>
+static int launch_mrw_degree(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots,
+                             uint64_t S, uint32_t *src, uint32_t *dst, unsigned long long *edges,
+                             unsigned int *err, cudaStream_t s) {
+  const uint64_t warps = (S + 32 / G - 1) / (32 / G);
+  size_t per_warp = (size_t)p.walkers * 20 * (32 / G);
+  uint4 *rec = nullptr;
+  if (per_warp > 48 * 1024) {  // too many walkers for shared memory (G = 32)
+    cudaError_t e =
+        scratch_alloc(reinterpret_cast<void **>(&rec), S * (uint64_t)p.walkers * sizeof(uint4), s);
+    if (e != cudaSuccess) return cuda_fail(e, "multi-RW scratch");
+    per_warp = 0;
+  }
+  const int w = mrw_block_warps(warps, per_warp);
+  mrw_degree_kernel<kSlots, G, Sum><<<grid_warps(warps, w, cur_dev(), 64 / w), w * 32, per_warp * w, s>>>(
+      g, roots, rec, S, p.walkers, p.steps, p.seed, src, dst, edges, err);
+  count_launch();
+  if (rec) scratch_free(rec, s);
+  return GRASS_OK;
+}
+
 int launch_mrw(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots, uint64_t S,
                uint32_t *src, uint32_t *dst, unsigned long long *edges, unsigned int *err,
-               cudaStream_t s) {
+               uint32_t max_degree, cudaStream_t s) {
   if (!S || !p.steps) return GRASS_OK;
   // Block per sample (walkers in parallel) for continuous-time selection, and
-  // for uniform selection when there are few samples or long chains (same
-  // output as the warp kernels).
-  if (p.select == GRASS_SELECT_DEGREE_CT ||
-      (p.select == GRASS_SELECT_UNIFORM &&
-       (p.steps >= 1024 || S < (uint64_t)sm_count(cur_dev()) * 8))) {
-    const int threads = (int)std::min<uint64_t>(
-        512, std::max<uint64_t>(128, ((uint64_t)p.walkers / 2 + 31) / 32 * 32));
-    auto kern = mrw_cta_kernel<kSlots>;
+  // for uniform selection with long chains (same output as the warp kernel):
+  // a block ends a chain sooner, a warp needs fewer threads.  With r samples
+  // resident as blocks the two cross near r (1 + steps / 2048) samples
+  // (R-MAT s22 ef32, us block / warp): 80 walkers x 1024 steps, r = 592: 148
+  // samples 46 / 73, 600 103 / 120, 1184 122 / 133, 8192 706 / 300; 2000 x
+  // 1024, r = 148: 148 36 / 59, 600 137 / 95; 2000 x 10,000: 600 527 / 723,
+  // 1184 865 / 759.  At 100 steps a warp is never slower.
+  const int threads = (int)std::min<uint64_t>(
+      512, std::max<uint64_t>(128, ((uint64_t)p.walkers / 2 + 31) / 32 * 32));
+  uint64_t resident = 0;
+  if (p.select == GRASS_SELECT_DEGREE_CT || (p.select == GRASS_SELECT_UNIFORM && p.steps >= 512)) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0);
-    const uint64_t grid =
-        std::min<uint64_t>(S, (uint64_t)sm_count(cur_dev()) * std::max(per_sm, 1));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mrw_cta_kernel<kSlots>, threads, 0);
+    resident = (uint64_t)sm_count(cur_dev()) * std::max(per_sm, 1);
+  }
+  if (p.select == GRASS_SELECT_DEGREE_CT || S <= resident + resident * p.steps / 2048) {
+    const uint64_t grid = std::min<uint64_t>(S, resident);
     const uint64_t stride = mrw_sample_scratch(p.walkers, p.steps, p.select);
     unsigned char *scr = nullptr;
     cudaError_t e = scratch_alloc(reinterpret_cast<void **>(&scr), grid * stride, s);
     if (e != cudaSuccess) return cuda_fail(e, "multi-RW scratch");
-    kern<<<(unsigned)grid, threads, 0, s>>>(g, roots, S, p.walkers, p.steps, p.select, p.seed, src,
-                                            dst, scr, stride, edges, err);
+    mrw_cta_kernel<kSlots><<<(unsigned)grid, threads, 0, s>>>(
+        g, roots, S, p.walkers, p.steps, p.select, p.seed, src, dst, scr, stride, edges, err);
     count_launch();
     scratch_free(scr, s);
     return GRASS_OK;
   }
-  const MrwLayout lay{p.walkers};
-  const size_t per_warp = lay.bytes_per_warp();
-  if (per_warp > 48 * 1024) {
-    // Too many walkers for shared memory: the state lives in global scratch.
-    uint4 *rec = nullptr;
-    cudaError_t e =
-        scratch_alloc(reinterpret_cast<void **>(&rec), S * (uint64_t)p.walkers * sizeof(uint4), s);
-    if (e != cudaSuccess) return cuda_fail(e, "multi-RW scratch");
-    auto kern = mrw_global_kernel<kSlots>;
-    kern<<<grid_warps(S, 8, cur_dev(), 8), 256, 0, s>>>(g, roots, rec, S, p.walkers, p.steps,
-                                                        (int)p.select, p.seed, src, dst, edges,
-                                                        err);
-    count_launch();
-    scratch_free(rec, s);
-    return GRASS_OK;
+  if (p.select == GRASS_SELECT_DEGREE) {
+    if (p.walkers > 256) return launch_mrw_degree<32, uint64_t>(g, p, roots, S, src, dst, edges, err, s);
+    if ((uint64_t)p.walkers * max_degree >> 32)
+      return launch_mrw_degree<8, uint64_t>(g, p, roots, S, src, dst, edges, err, s);
+    return launch_mrw_degree<8, uint32_t>(g, p, roots, S, src, dst, edges, err, s);
   }
-  const size_t budget = 200 * 1024;
-  const int warps = (int)std::min<size_t>(8, budget / per_warp);
-  const size_t smem = per_warp * warps;
-  auto kern = mrw_kernel<kSlots>;
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const unsigned grid = grid_warps(S, warps, cur_dev(), 8);
-  kern<<<grid, warps * 32, smem, s>>>(g, roots, S, p.walkers, p.steps, (int)p.select, p.seed,
-                                       src, dst, edges, err);
+  const bool fits = p.walkers <= 48 * 1024 / 4;
+  const size_t per_warp = fits ? (size_t)p.walkers * 4 : 0;
+  const int w = mrw_block_warps(S, per_warp);
+  auto kern = fits ? mrw_kernel<kSlots> : mrw_global_kernel<kSlots>;
+  kern<<<grid_warps(S, w, cur_dev(), 64 / w), w * 32, per_warp * w, s>>>(
+      g, roots, S, p.walkers, p.steps, p.seed, src, dst, edges, err);
   count_launch();
   return GRASS_OK;
 }

@@ -1,7 +1,7 @@
 // mrw_cta.cuh -- multi random walk with one thread block per sample, walkers
 // in parallel (MultiRWApp, GT/src/apps/multiRW/multiRW.cu:3-112).
 //
-// The warp version (sample_warp.cuh, mrw_warp) takes the T steps one after
+// The warp version (sample_warp.cuh, mrw_degree_warp) takes the T steps one after
 // another: ~2 dependent DRAM reads per step, ~19 ms for 10,000 steps.  Two
 // selections allow the walkers to move in parallel instead:
 //
@@ -68,7 +68,7 @@ __host__ __device__ inline uint64_t mrw_sample_scratch(uint32_t R, uint32_t T, u
   else if (select == GRASS_SELECT_DEGREE_CT)
     b = CtLayout(R, T).total;
   else
-    b = (uint64_t)R * 16;  // mrw_warp: one vertex record per walker
+    b = (uint64_t)R * 16;  // mrw_degree_warp: one vertex record per walker
   return (b + 255) & ~255ull;
 }
 
@@ -207,7 +207,7 @@ __device__ CtEvent *cta_sort_events(CtEvent *a, CtEvent *b, uint32_t n, CtaSmem<
 
 // Uniform multi-RW of one sample by the whole block.  scr: R + 1 + T words.
 // Step t: walker mulhi(word 0, R), neighbor mulhi(word 1, d) of
-// Philox(seed; t, sample, .., TAG_MRW) -- the stream of mrw_warp.
+// Philox(seed; t, sample, .., TAG_MRW) -- the stream of mrw_uniform_warp.
 template <int MODE, int NW>
 __device__ void mrw_uniform_cta(const DevGraph &g, uint32_t *roots, uint32_t *src, uint32_t *dst,
                                 uint32_t R, uint32_t T, uint64_t seed, uint64_t sample,

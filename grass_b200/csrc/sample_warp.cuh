@@ -255,44 +255,129 @@ __device__ __forceinline__ uint32_t mrw_root(uint32_t n, uint64_t seed, uint64_t
   return mulhi_u32(pick(r, (int)(i & 3)), n);
 }
 
-// Multi random walk of one sample (MultiRWApp, GT/src/apps/multiRW/multiRW.cu:3-112).
-// The sample's state is vtx[0..R), the walkers' vertices (updated in place),
-// and rec[0..R), each walker's 16-byte vertex record (all zero for a vertex
-// out of range), in shared or global memory.  Keeping the record makes a
-// step cost two dependent DRAM reads (payload, then the new vertex's record)
-// instead of three.  Lane j keeps the total degree of walkers [j*B, (j+1)*B),
-// B = ceil(R/32); a degree-proportional pick scans the 32 bucket sums with
-// shuffles, then the chosen bucket 32 entries at a time.  Step t draws from
-// Philox(seed; t, sample, .., TAG_MRW): word 0 (+ word 2 as high half) picks
-// the walker, word 1 the neighbor.  Lane k computes the block of step
-// t0 + k, so one Philox evaluation per lane serves 32 steps.
+// Multi random walk of one sample (MultiRWApp, GT/src/apps/multiRW/multiRW.cu:3-112),
+// the walker of each step picked uniformly, by one warp.  vtx[0..R) holds the
+// walkers' vertices (shared or global memory), updated in place.  Step t draws
+// from Philox(seed; t, sample, .., TAG_MRW): word 0 picks the walker, word 1
+// the neighbor.  So the walkers of 32 steps are known before any of them is
+// taken, and steps of different walkers do not depend on one another: lane k
+// takes step t0 + k, in as many rounds as one walker has steps among the 32
+// (2 or 3 with 80 walkers), where one step after the other left 31 lanes idle
+// through 32 chains of two memory reads (65,536 samples of 80 walkers x 100
+// steps, R-MAT s22 ef32: 0.25 ms against 1.70 ms).
 template <int MODE>
-__device__ __forceinline__ void mrw_warp(const DevGraph &g, uint32_t *vtx, uint4 *rec, uint32_t R,
-                                         uint32_t T, int select, uint64_t seed, uint64_t sample,
-                                         uint32_t *src, uint32_t *dst, uint64_t &cnt, bool &bad) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t B = (R + 31) / 32;
-  // Records of the start vertices: four independent loads in flight per lane.
-  for (uint32_t c0 = 0; c0 < R; c0 += 128) {
+__device__ __forceinline__ void mrw_uniform_warp(const DevGraph &g, uint32_t *vtx, uint32_t R,
+                                                 uint32_t T, uint64_t seed, uint64_t sample,
+                                                 uint32_t *src, uint32_t *dst, uint64_t &cnt,
+                                                 bool &bad) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t t0 = 0; t0 < T; t0 += 32) {
+    const uint32_t t = t0 + lane;
+    const u32x4 r = philox4x32_10(seed, t, (uint32_t)sample, (uint32_t)(sample >> 32), TAG_MRW);
+    const uint32_t x = t < T ? mulhi_u32(r.x, R) : INVALID_VERTEX;
+    const unsigned same = __match_any_sync(kFull, x);
+    const uint32_t turn = __popc(same & ((1u << lane) - 1u));
+    const uint32_t turns = __reduce_max_sync(kFull, t < T ? turn : 0u) + 1;
+    uint32_t from = INVALID_VERTEX, to = INVALID_VERTEX;
+    for (uint32_t k = 0; k < turns; k++) {  // warp-uniform
+      if (t < T && turn == k) {
+        from = vtx[x];
+        const VHdr h = record_header<MODE>(from < g.n ? graph_record<MODE>(g, from)
+                                                      : make_uint4(0u, 0u, 0u, 0u));
+        if (h.d) {
+          const uint32_t nv = neighbor<MODE>(g, h, mulhi_u32(r.y, h.d));
+          if (nv < g.n) {
+            to = vtx[x] = nv;
+            cnt++;
+          } else {
+            bad = true;
+          }
+        }
+      }
+      __syncwarp();
+    }
+    if (t < T) {
+      store_out_u32(src + sample * T + t, from);
+      store_out_u32(dst + sample * T + t, to);
+    }
+  }
+}
+
+// Records (all zero: none) of the walkers' vertices vtx[0..R) into rec[0..R),
+// lanes gl of the G that share a sample; four independent loads in flight.
+template <int MODE, int G>
+__device__ __forceinline__ void mrw_load_records(const DevGraph &g, const uint32_t *vtx,
+                                                 uint4 *rec, uint32_t R, uint32_t gl) {
+  for (uint32_t c0 = 0; c0 < R; c0 += 4 * G) {
     uint4 r[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const uint32_t i = c0 + k * 32 + lane;
+      const uint32_t i = c0 + k * G + gl;
       const uint32_t x = i < R ? vtx[i] : INVALID_VERTEX;
       r[k] = x < g.n ? graph_record<MODE>(g, x) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const uint32_t i = c0 + k * 32 + lane;
+      const uint32_t i = c0 + k * G + gl;
       if (i < R) rec[i] = r[k];
     }
   }
-  __syncwarp();
-  uint64_t bsum = 0;  // this lane's bucket
-  for (uint32_t i = lane * B; i < min(R, (lane + 1) * B); i++) bsum += rec[i].z;
-  uint64_t wsum = bsum;
+}
+
+// Inclusive sum over the lanes of groups of G.
+template <int G, class Sum>
+__device__ __forceinline__ Sum group_scan(Sum v) {
+  const uint32_t gl = threadIdx.x & (G - 1);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(kFull, wsum, o);
+  for (int o = 1; o < G; o <<= 1) {
+    const Sum y = __shfl_up_sync(kFull, v, o, G);
+    if (gl >= (uint32_t)o) v += y;
+  }
+  return v;
+}
+
+// Moves walker x along the neighbor that a random word picks: writes the edge
+// and the walker's new vertex and record, and returns the change of its degree.
+template <int MODE>
+__device__ __forceinline__ int64_t mrw_move(const DevGraph &g, uint32_t *vtx, uint4 *rec,
+                                            uint32_t x, uint32_t word, uint32_t *src, uint32_t *dst,
+                                            uint64_t &cnt, bool &bad) {
+  const VHdr h = record_header<MODE>(rec[x]);
+  const uint32_t nv = neighbor<MODE>(g, h, mulhi_u32(word, h.d));
+  store_out_u32(src, vtx[x]);
+  if (nv >= g.n) {
+    bad = true;
+    store_out_u32(dst, INVALID_VERTEX);
+    return 0;
+  }
+  const uint4 r = graph_record<MODE>(g, nv);
+  store_out_u32(dst, nv);
+  vtx[x] = nv;
+  rec[x] = r;
+  cnt++;
+  return (int64_t)r.z - h.d;
+}
+
+// Multi random walk with the walker of each step picked in proportion to its
+// degree, one sample per warp.  A step depends on the one before it through
+// two memory reads (the slot, then the new vertex's record, for its degree).
+// The sample's state is vtx[0..R) and rec[0..R), each walker's vertex and
+// record, in shared or global memory; lane j keeps the total degree of walkers
+// [j B, (j + 1) B), B = ceil(R / 32).  A pick scans the 32 sums with shuffles,
+// then the chosen B entries 32 at a time.  Step t: words 2, 0 of its Philox
+// block (see mrw_uniform_warp) pick the walker, word 1 the neighbor; lane k
+// computes the block of step t0 + k.
+template <int MODE>
+__device__ __forceinline__ void mrw_degree_warp(const DevGraph &g, uint32_t *vtx, uint4 *rec,
+                                                uint32_t R, uint32_t T, uint64_t seed,
+                                                uint64_t sample, uint32_t *src, uint32_t *dst,
+                                                uint64_t &cnt, bool &bad) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t B = (R + 31) / 32;
+  mrw_load_records<MODE, 32>(g, vtx, rec, R, lane);
+  __syncwarp();
+  uint64_t bsum = 0;  // this lane's walkers
+  for (uint32_t i = lane * B; i < min(R, (lane + 1) * B); i++) bsum += rec[i].z;
   for (uint32_t t0 = 0; t0 < T; t0 += 32) {
     const u32x4 mine =
         philox4x32_10(seed, t0 + lane, (uint32_t)sample, (uint32_t)(sample >> 32), TAG_MRW);
@@ -301,79 +386,90 @@ __device__ __forceinline__ void mrw_warp(const DevGraph &g, uint32_t *vtx, uint4
       const uint32_t rx = __shfl_sync(kFull, mine.x, k), ry = __shfl_sync(kFull, mine.y, k),
                      rz = __shfl_sync(kFull, mine.z, k);
       const uint64_t io = sample * T + t0 + k;
-      uint32_t x;
-      if (select == GRASS_SELECT_DEGREE) {
-        if (wsum == 0) {
-          if (lane == 0) {
-            src[io] = INVALID_VERTEX;
-            dst[io] = INVALID_VERTEX;
-          }
-          continue;
+      const uint64_t incl = group_scan<32>(bsum), wsum = __shfl_sync(kFull, incl, 31);
+      if (wsum == 0) {  // (warp-uniform)
+        if (lane == 0) src[io] = dst[io] = INVALID_VERTEX;
+        continue;
+      }
+      const uint64_t u = mulhi_u64(((uint64_t)rz << 32) | rx, wsum);
+      // bucket: the first lane whose inclusive sum exceeds u; then its first walker
+      const int Lb = __ffs(__ballot_sync(kFull, incl > u)) - 1;
+      uint64_t acc = __shfl_sync(kFull, incl - bsum, Lb);
+      const uint32_t b0 = (uint32_t)Lb * B, b1 = min(R, b0 + B);
+      uint32_t x = b1 - 1;
+      for (uint32_t c0 = b0; c0 < b1; c0 += 32) {  // two passes for R <= 2048
+        const uint32_t i = c0 + lane;
+        const uint64_t ci = group_scan<32>((uint64_t)(i < b1 ? rec[i].z : 0u));
+        const unsigned hit = __ballot_sync(kFull, i < b1 && acc + ci > u);
+        if (hit) {
+          x = c0 + (uint32_t)(__ffs(hit) - 1);
+          break;
         }
-        const uint64_t u = mulhi_u64(((uint64_t)rz << 32) | rx, wsum);
-        // bucket: first lane whose inclusive prefix exceeds u
-        uint64_t incl = bsum;
+        acc += __shfl_sync(kFull, ci, 31);
+      }
+      int64_t gain = 0;
+      if (lane == 0) gain = mrw_move<MODE>(g, vtx, rec, x, ry, src + io, dst + io, cnt, bad);
+      gain = __shfl_sync(kFull, gain, 0);
+      if (lane == x / B) bsum += gain;
+      __syncwarp();
+    }
+  }
+}
+
+// The same by G lanes of a warp, 32 / G samples side by side, for few walkers
+// (B = ceil(R / G) a lane) with their state in shared memory.  (Called by
+// whole warps; `live`: this group has a sample.)  The lane whose walkers hold
+// the pick finds it among them and moves it, so a step is one scan of the
+// group's sums, a short search and the two memory reads, with nothing to hand
+// round.  (8,192 samples of 80 walkers x 100 steps, R-MAT s22 ef32: 0.191 ms,
+// all of them under way at once and bound by the chain of reads, 1.9 us a
+// step; 0.216 ms with the walker found and moved by the group together, 0.370
+// ms with one sample per warp, of which 4,736 fit.)  Sum: uint32_t where no sum of R degrees reaches 2^32.
+template <int MODE, int G, class Sum>
+__device__ __forceinline__ void mrw_degree_group(const DevGraph &g, bool live, uint32_t *vtx,
+                                                 uint4 *rec, uint32_t R, uint32_t T, uint64_t seed,
+                                                 uint64_t sample, uint32_t *src, uint32_t *dst,
+                                                 uint64_t &cnt, bool &bad) {
+  const uint32_t gl = threadIdx.x & (G - 1);
+  const uint32_t B = (R + G - 1) / G, x0 = min(R, gl * B), x1 = min(R, x0 + B);
+  if (live) mrw_load_records<MODE, G>(g, vtx, rec, R, gl);
+  __syncwarp();
+  Sum bsum = 0;  // this lane's walkers [x0, x1)
+  if (live)
+    for (uint32_t i = x0; i < x1; i++) bsum += rec[i].z;
+  for (uint32_t t0 = 0; t0 < T; t0 += G) {
+    const u32x4 mine =
+        philox4x32_10(seed, t0 + gl, (uint32_t)sample, (uint32_t)(sample >> 32), TAG_MRW);
+    const uint32_t tn = min((uint32_t)G, T - t0);
+    for (uint32_t k = 0; k < tn; k++) {
+      const uint32_t rx = __shfl_sync(kFull, mine.x, k, G), ry = __shfl_sync(kFull, mine.y, k, G),
+                     rz = __shfl_sync(kFull, mine.z, k, G);
+      const uint64_t io = sample * T + t0 + k;
+      const Sum incl = group_scan<G>(bsum), wsum = __shfl_sync(kFull, incl, G - 1, G);
+      const Sum u = (Sum)mulhi_u64(((uint64_t)rz << 32) | rx, wsum), before = incl - bsum;
+      if (u >= before && u < incl) {  // the pick is among this lane's walkers
+        Sum left = u - before;
+        uint32_t x = x0;
+        for (;; x += 4) {  // four degrees at a time
+          uint32_t d[4];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint64_t y = __shfl_up_sync(kFull, incl, o);
-          if (lane >= o) incl += y;
-        }
-        const int Lb = __ffs(__ballot_sync(kFull, incl > u)) - 1;
-        uint64_t acc = __shfl_sync(kFull, incl - bsum, Lb);  // prefix before the bucket
-        const uint32_t b0 = (uint32_t)Lb * B, b1 = min(R, b0 + B);
-        x = b1 - 1;
-        for (uint32_t c0 = b0; c0 < b1; c0 += 32) {  // two passes for R <= 2048
-          const uint32_t i = c0 + lane;
-          const uint64_t d = i < b1 ? rec[i].z : 0u;
-          uint64_t ci = d;
+          for (int q = 0; q < 4; q++) d[q] = x + q < x1 ? rec[x + q].z : 0xFFFFFFFFu;
+          uint32_t past = 0;
 #pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const uint64_t y = __shfl_up_sync(kFull, ci, o);
-            if (lane >= o) ci += y;
+          for (int q = 0; q < 4; q++) {
+            if (past == (uint32_t)q && left >= d[q]) {
+              left -= d[q];
+              past++;
+            }
           }
-          const unsigned hit = __ballot_sync(kFull, i < b1 && acc + ci > u);
-          if (hit) {
-            x = c0 + (uint32_t)(__ffs(hit) - 1);
+          if (past < 4) {
+            x += past;
             break;
           }
-          acc += __shfl_sync(kFull, ci, 31);
         }
-      } else {
-        x = mulhi_u32(rx, R);
-      }
-      // lane 0 moves walker x
-      uint32_t nd = 0, od = 0;
-      bool moved = false;
-      if (lane == 0) {
-        const uint32_t v = vtx[x];
-        const uint4 r = rec[x];
-        od = r.z;
-        src[io] = v;
-        if (od == 0) {
-          dst[io] = INVALID_VERTEX;
-        } else {
-          const VHdr h = record_header<MODE>(r);
-          const uint32_t nv = neighbor<MODE>(g, h, mulhi_u32(ry, h.d));
-          if (nv >= g.n) {
-            bad = true;
-            dst[io] = INVALID_VERTEX;
-          } else {
-            dst[io] = nv;
-            cnt++;
-            const uint4 nr = graph_record<MODE>(g, nv);
-            vtx[x] = nv;
-            rec[x] = nr;
-            nd = nr.z;
-            moved = true;
-          }
-        }
-      }
-      moved = __shfl_sync(kFull, moved, 0);
-      if (moved) {
-        nd = __shfl_sync(kFull, nd, 0);
-        od = __shfl_sync(kFull, od, 0);
-        if (lane == (int)(x / B)) bsum = bsum - od + nd;
-        wsum = wsum - od + nd;
+        bsum += (Sum)mrw_move<MODE>(g, vtx, rec, x, ry, src + io, dst + io, cnt, bad);
+      } else if (wsum == 0 && live && gl == 0) {
+        src[io] = dst[io] = INVALID_VERTEX;
       }
       __syncwarp();
     }
