@@ -33,9 +33,14 @@ __global__ void __launch_bounds__(256, GRASS_BATCH_MIN_BLOCKS) batch_kernel(DevG
                                                     unsigned int *queue,
                                                     unsigned long long *total,
                                                     unsigned int *err) {
-  __shared__ SmemHdr sh[8];
+  union WarpSmem {  // a warp runs one kind of item at a time
+    SmemHdr khop;
+    uint32_t stage[kPathStageWords<DEPTH>];
+  };
+  __shared__ __align__(16) unsigned char warp_smem[8 * sizeof(WarpSmem)];
+  WarpSmem *sh = reinterpret_cast<WarpSmem *>(warp_smem);
   __shared__ CtaSmem<8> csm;
-  SmemHdr &my = sh[threadIdx.x >> 5];
+  SmemHdr &my = sh[threadIdx.x >> 5].khop;
   const int lane = threadIdx.x & 31;
   uint64_t all = 0;
   bool bad = false;
@@ -74,8 +79,15 @@ __global__ void __launch_bounds__(256, GRASS_BATCH_MIN_BLOCKS) batch_kernel(DevG
     const BatchJob &jb = jobs[tk.job];
     uint64_t cnt = 0;
     if (jb.type == GRASS_JOB_RW) {
-      rw_warp<MODE, DEPTH>(g, jb.in, jb.count, jb.length, jb.seed, 0, (int)jb.layout, jb.out0,
-                           tk.begin, tk.end, cnt, bad);
+      uint32_t *stage = sh[threadIdx.x >> 5].stage;
+      for (uint64_t wb = tk.begin; wb < tk.end; wb += 32 * DEPTH) {
+        if (jb.layout == GRASS_LAYOUT_WALK_MAJOR)
+          rw_pass<MODE, DEPTH, true>(g, jb.in, jb.count, jb.length, jb.seed, 0, jb.out0, wb, 32,
+                                     tk.end, stage, cnt, bad);
+        else
+          rw_pass<MODE, DEPTH, false>(g, jb.in, jb.count, jb.length, jb.seed, 0, jb.out0, wb, 32,
+                                      tk.end, stage, cnt, bad);
+      }
     } else if (jb.type == GRASS_JOB_KHOP) {
       const uint32_t parts = max(1u, tk.pad >> 8), part = tk.pad & 0xFFu;
       for (uint64_t s = tk.begin; s < tk.end; s++)

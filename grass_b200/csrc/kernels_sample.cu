@@ -41,38 +41,17 @@ __global__ void __launch_bounds__(512, GRASS_RW_MIN_BLOCKS) rw_kernel(DevGraph g
                                                  uint64_t w0, int layout,
                                                  uint32_t *__restrict__ paths,
                                                  unsigned long long *edges, unsigned int *err) {
+  extern __shared__ uint32_t path_stage[];  // walk-major: kPathStageWords<DEPTH> words a warp
   const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
+  uint32_t *stage = path_stage + (threadIdx.x >> 5) * kPathStageWords<DEPTH>;
   uint64_t cnt = 0;
   bool bad = false;
-  for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; base < W;
-       base += nthreads * DEPTH) {
-    uint32_t v[DEPTH];
-    u32x4 r[DEPTH];
-#pragma unroll
-    for (int k = 0; k < DEPTH; k++) {
-      const uint64_t w = base + k * nthreads;
-      v[k] = INVALID_VERTEX;
-      r[k] = u32x4{0, 0, 0, 0};
-      if (w < W) {
-        const uint32_t s0 = starts[w];
-        store_path(paths, layout, W, L, w, 0, s0);
-        v[k] = s0 < g.n ? s0 : INVALID_VERTEX;
-      }
-    }
-    for (uint32_t s = 0; s < L; s++) {
-      walk_step<MODE, DEPTH>(g, v, [&](int k) {
-        if ((s & 3) == 0) {
-          const uint64_t id = w0 + base + k * nthreads;
-          r[k] = philox4x32_10(seed, s >> 2, (uint32_t)id, (uint32_t)(id >> 32), TAG_RW);
-        }
-        return pick(r[k], s & 3);
-      }, cnt, bad);
-#pragma unroll
-      for (int k = 0; k < DEPTH; k++) {
-        const uint64_t w = base + k * nthreads;
-        if (w < W) store_path(paths, layout, W, L, w, s + 1, v[k]);
-      }
-    }
+  for (uint64_t wb = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); wb < W;
+       wb += nthreads * DEPTH) {  // warp-uniform
+    if (layout == GRASS_LAYOUT_WALK_MAJOR)
+      rw_pass<MODE, DEPTH, true>(g, starts, W, L, seed, w0, paths, wb, nthreads, W, stage, cnt, bad);
+    else
+      rw_pass<MODE, DEPTH, false>(g, starts, W, L, seed, w0, paths, wb, nthreads, W, stage, cnt, bad);
   }
   warp_add_u64(edges, cnt);
   if (bad && err) atomicOr(err, 1u);
@@ -550,11 +529,12 @@ void launch_uniform_starts(uint64_t n, uint64_t count, uint64_t seed, uint32_t *
 // attribute: the caller's stream keeps its own access policy.
 template <class... ExpTypes, class... ActTypes>
 static void launch_with_window(void (*kern)(ExpTypes...), unsigned grid, unsigned block,
-                               cudaStream_t s, const L2Window &win, ActTypes &&...args) {
+                               size_t smem, cudaStream_t s, const L2Window &win,
+                               ActTypes &&...args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   if (win.on()) {
@@ -597,11 +577,14 @@ int apply_tuning(int device, const grass_tuning &t, const void *base, size_t byt
 
 // Defaults measured on B200 (R-MAT s22 ef32, 1M walkers x 80, step-major
 // paths): the compressed walk is fastest with one walker per thread, the CSR
-// walk 0.5% faster with four.
+// walk 0.5% faster with four.  Blocks of 64 threads spread few walkers over more
+// SMs and leave a place sooner (us at 64 / 256 threads: 4,096 x 80 on s22 63 /
+// 75, on s16 54.7 / 55.1; 1M x 80 2014 / 2032); 512 resident threads a block
+// pair (64 registers) beat 1536 (40: 2.09 -> 2.15 ms).
 grass_tuning resolve_tuning(const grass_tuning &t, int kind) {
   grass_tuning r = t;
   if (!r.rw_depth) r.rw_depth = kind == 2 ? 4 : 1;
-  if (!r.rw_threads) r.rw_threads = 256;
+  if (!r.rw_threads) r.rw_threads = kind == 2 ? 256 : 64;
   return r;  // rw_blocks_per_sm == 0: as many as are resident
 }
 
@@ -609,10 +592,10 @@ grass_tuning resolve_tuning(const grass_tuning &t, int kind) {
 // what the occupancy calculator says is resident, times the SM count, and
 // no more blocks than there is work for.
 template <class K>
-static unsigned resident_grid(K kern, int threads, uint32_t want_per_sm, uint64_t units,
-                              uint64_t units_per_block) {
+static unsigned resident_grid(K kern, int threads, size_t smem, uint32_t want_per_sm,
+                              uint64_t units, uint64_t units_per_block) {
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
   if (per_sm < 1) per_sm = 1;
   if (want_per_sm && (int)want_per_sm < per_sm) per_sm = (int)want_per_sm;
   const uint64_t need = (units + units_per_block - 1) / units_per_block;
@@ -626,9 +609,12 @@ static void rw_launch_depth(const DevGraph &g, const grass_rw_params &p, const u
                             unsigned int *err, cudaStream_t s, const grass_tuning &t,
                             const L2Window &win, uint64_t w0) {
   auto kern = rw_kernel<kSlots, DEPTH>;
-  const unsigned grid =
-      resident_grid(kern, (int)t.rw_threads, t.rw_blocks_per_sm, W, (uint64_t)t.rw_threads * DEPTH);
-  launch_with_window(kern, grid, t.rw_threads, s, win, g, starts, W, p.length, p.seed, w0,
+  const size_t smem = p.layout == GRASS_LAYOUT_WALK_MAJOR
+                          ? (size_t)t.rw_threads / 32 * kPathStageWords<DEPTH> * 4 : 0;
+  static_assert(512 / 32 * kPathStageWords<DEPTH> * 4 <= 48 * 1024, "no opt-in needed");
+  const unsigned grid = resident_grid(kern, (int)t.rw_threads, smem, t.rw_blocks_per_sm, W,
+                                      (uint64_t)t.rw_threads * DEPTH);
+  launch_with_window(kern, grid, t.rw_threads, smem, s, win, g, starts, W, p.length, p.seed, w0,
                      (int)p.layout, paths, edges, err);
 }
 
@@ -680,20 +666,20 @@ void launch_rw_csr(const DevCsr &c, const grass_rw_params &p, const uint32_t *st
   const int T = (int)t.rw_threads;
   switch (t.rw_depth) {
     case 1: {
-      const unsigned grid = resident_grid(rw_csr_kernel<1>, T, t.rw_blocks_per_sm, W, T);
-      launch_with_window(rw_csr_kernel<1>, grid, T, s, win, c, starts, W, L, p.seed, w0, lay,
+      const unsigned grid = resident_grid(rw_csr_kernel<1>, T, 0, t.rw_blocks_per_sm, W, T);
+      launch_with_window(rw_csr_kernel<1>, grid, T, 0, s, win, c, starts, W, L, p.seed, w0, lay,
                          paths, edges);
       break;
     }
     case 4: {
-      const unsigned grid = resident_grid(rw_csr_kernel<4>, T, t.rw_blocks_per_sm, W, T * 4);
-      launch_with_window(rw_csr_kernel<4>, grid, T, s, win, c, starts, W, L, p.seed, w0, lay,
+      const unsigned grid = resident_grid(rw_csr_kernel<4>, T, 0, t.rw_blocks_per_sm, W, T * 4);
+      launch_with_window(rw_csr_kernel<4>, grid, T, 0, s, win, c, starts, W, L, p.seed, w0, lay,
                          paths, edges);
       break;
     }
     default: {
-      const unsigned grid = resident_grid(rw_csr_kernel<2>, T, t.rw_blocks_per_sm, W, T * 2);
-      launch_with_window(rw_csr_kernel<2>, grid, T, s, win, c, starts, W, L, p.seed, w0, lay,
+      const unsigned grid = resident_grid(rw_csr_kernel<2>, T, 0, t.rw_blocks_per_sm, W, T * 2);
+      launch_with_window(rw_csr_kernel<2>, grid, T, 0, s, win, c, starts, W, L, p.seed, w0, lay,
                          paths, edges);
     }
   }
