@@ -151,9 +151,6 @@ void launch_bswap(uint32_t *w, uint64_t n_words, cudaStream_t s);
 uint64_t scan_tmp_words(uint64_t n);
 void launch_unpack_scan(const uint32_t *payload, uint64_t n, uint32_t ubl, uint64_t *out,
                         uint64_t *tmp, cudaStream_t s);
-// u32 counts -> u64 exclusive scan into out[0..n]
-void launch_scan_u32(const uint32_t *counts, uint64_t n, uint64_t *out, uint64_t *tmp,
-                     cudaStream_t s);
 // Header validation: stats[0] = sum of degrees, stats[1] = max degree,
 // stats[2] = first bad vertex + 1 (0 if none). deg may be null.
 void launch_validate(const DevGraph &g, uint32_t *deg, unsigned long long *stats,

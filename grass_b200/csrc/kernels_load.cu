@@ -52,11 +52,6 @@ struct DegreeLoader {  // degrees from the vertex records
   __device__ __forceinline__ uint64_t operator()(uint64_t u) const { return __ldg(&recs[u].z); }
 };
 
-struct CountLoader {
-  const uint32_t *counts;
-  __device__ __forceinline__ uint64_t operator()(uint64_t u) const { return counts[u]; }
-};
-
 template <class Loader>
 __global__ void __launch_bounds__(kScanThreads) tile_reduce(Loader ld, uint64_t n,
                                                               uint64_t *tile_sums) {
@@ -423,11 +418,6 @@ uint64_t scan_tmp_words(uint64_t n) { return (n + kTile - 1) / kTile + 1; }
 void launch_unpack_scan(const uint32_t *payload, uint64_t n, uint32_t ubl, uint64_t *out,
                         uint64_t *tmp, cudaStream_t s) {
   scan_impl(FieldLoader{payload, ubl}, n, out, tmp, s);
-}
-
-void launch_scan_u32(const uint32_t *counts, uint64_t n, uint64_t *out, uint64_t *tmp,
-                     cudaStream_t s) {
-  scan_impl(CountLoader{counts}, n, out, tmp, s);
 }
 
 void launch_scan_degrees(const uint4 *recs, uint64_t n, uint64_t *rowptr, uint64_t *tmp,
