@@ -311,17 +311,21 @@ __global__ void __launch_bounds__(512, GRASS_RW_CSR_MIN_BLOCKS) rw_csr_kernel(De
 }
 
 // ---------------------------------------------------------------------------
-// Draws a lane of the standalone k-hop has in flight at once (the batched
-// kernel keeps one: its register budget is shared with the walks), and the
-// k-hop kernels' resident blocks per SM (256 threads each).  Measured on
-// R-MAT s22 ef32, 65,536 seeds x (25, 10): (2, 4) beat (4, 2), (4, 3), (2, 3)
-// and (1, 4) for GT, LE and the CSR.
+// Draws a lane of the standalone k-hop has in flight at once, and the k-hop
+// kernels' resident blocks per SM (256 threads each).  Measured on R-MAT s22
+// ef32, 65,536 seeds x (25, 10), us: one draw, 4 blocks 232, 5 blocks 253; two
+// draws, 4 blocks 249 (they spill), 3 blocks 244; four draws, 2 blocks 240.  The
+// CSR's draws need no sector in registers: two.
 #ifndef GRASS_KHOP_INFLIGHT
-#define GRASS_KHOP_INFLIGHT 2
+#define GRASS_KHOP_INFLIGHT 1
+#endif
+#ifndef GRASS_KHOP_CSR_INFLIGHT
+#define GRASS_KHOP_CSR_INFLIGHT 2
 #endif
 #ifndef GRASS_KHOP_MIN_BLOCKS
 #define GRASS_KHOP_MIN_BLOCKS 4
 #endif
+
 // k-hop.  One warp per seed (khop_seed_warp).
 
 template <int MODE>
@@ -357,7 +361,7 @@ __global__ void __launch_bounds__(256, GRASS_KHOP_MIN_BLOCKS) khop_csr_kernel(De
   uint64_t cnt = 0;
   bool bad = false;
   for (uint64_t s = warp; s < S; s += nwarps)
-    khop_seed_warp<kCsr, GRASS_KHOP_INFLIGHT>(g, seeds, A, s, my, cnt, bad);
+    khop_seed_warp<kCsr, GRASS_KHOP_CSR_INFLIGHT>(g, seeds, A, s, my, cnt, bad);
   warp_add_u64(edges, cnt);
 }
 

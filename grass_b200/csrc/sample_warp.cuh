@@ -148,9 +148,8 @@ __device__ __forceinline__ void rw_pass(const DevGraph &g, const uint32_t *start
 
 // ---------------------------------------------------------------------------
 // k-hop of one seed (KHopApp, GT/src/apps/khop/khop.cu:1-79, with runtime
-// fanouts).  For each hop the frontier is taken in chunks of 32 transits:
-// lane p decodes the header of transit p into the warp's shared-memory slot,
-// then the chunk's f*32 draws are spread over the lanes.
+// fanouts).  For each hop the frontier is taken in groups of 32 transits, and a
+// group's f * 32 draws are spread over the lanes.
 
 struct KhopArgs {
   uint32_t hops;
@@ -160,17 +159,15 @@ struct KhopArgs {
   uint64_t seed;
 };
 
-// A warp's frontier group: transit i's record (degree 0: none) and first
-// output slot (parent index * fanout).
+// A warp's share of shared memory.
+constexpr uint32_t kFrontier = 64;
 struct SmemHdr {
-  uint4 rec[32];
-  uint64_t ob[32];
+  uint4 kept[2][kFrontier];  // records of a frontier of up to kFrontier vertices (degree 0:
+                             // none), for this hop and the next
+  uint4 rec[32];             // a group's records, where the frontier is in global memory
+  uint64_t ob[32];           // and its transits' first output slots, with parts > 1
+  uint32_t words[128];       // random words of 128 draws
 };
-
-// Word k (0..3) of a Philox block held as four values.
-__device__ __forceinline__ uint32_t pick4(uint32_t x, uint32_t y, uint32_t z, uint32_t w, int k) {
-  return k == 0 ? x : k == 1 ? y : k == 2 ? z : w;
-}
 
 // With parts > 1, `parts` warps share the seed: warp `part` takes the subtrees
 // of the first hop's children part, part + parts, ... for every later hop.
@@ -181,117 +178,149 @@ __device__ __forceinline__ uint32_t pick4(uint32_t x, uint32_t y, uint32_t z, ui
 // Draw slot k of hop h (its index in the seed's hop-h output row) uses word
 // k & 3 of Philox(seed; k >> 2, s, s >> 32, TAG_KHOP | h).  The frontier is
 // taken G transits at a time (G = 32, fewer only for fanouts above 2^27, so
-// that a group's draw count fits 32 bits): lane p loads the header of transit
-// p, then the group's G f draws are spread over the lanes.  With one part and
-// G = 32 a group's slots are contiguous (pc f + j, pc a multiple of 32), so the
-// lanes compute the group's Philox blocks once per 128 draws, lane l block l of
-// the window, and hand the words out by shuffles; otherwise each draw
-// computes its own block.  INFLIGHT: draws a lane has in flight at once (every
-// load is issued before any is decoded).  On a CSR a draw is one column load.
+// that a group's draw count fits 32 bits).  With one part and G = 32 a group's
+// slots are contiguous (pc f + j, pc a multiple of 32), so the lanes compute the
+// group's Philox blocks once per 128 draws and hand the words out through
+// shared memory; otherwise each draw computes its own block.  INFLIGHT: draws a
+// lane has in flight at once (every load is issued before any is decoded).  On a
+// CSR a draw is one column load.
+//
+// A frontier of up to kFrontier vertices stays in shared memory as records,
+// loaded by the lanes that drew the vertices: the next hop then starts with its
+// slot loads, where it would first read the vertices back and then their
+// records.  A lane's place (transit, draw under it) advances by 32 / f and
+// 32 % f.  65,536 seeds x (25, 10) on R-MAT s22 ef32: 0.232 ms, of which the 8.9
+// M sectors that miss L2 take 0.19 at the rate of random reads; 0.251 with
+// 64-bit divisions for the place and the parent, words by shuffle, every
+// frontier read back and two draws in flight.
 template <int MODE, int INFLIGHT = 1>
 __device__ __forceinline__ void khop_seed_warp(const DevGraph &g, const uint32_t *seeds,
                                                const KhopArgs &A, uint64_t s, SmemHdr &my,
-                                               uint64_t &cnt, bool &bad,
-                                               uint32_t part = 0, uint32_t parts = 1) {
+                                               uint64_t &cnt, bool &bad, uint32_t part = 0,
+                                               uint32_t parts = 1) {
   static_assert(INFLIGHT == 1 || INFLIGHT == 2 || INFLIGHT == 4, "INFLIGHT in {1, 2, 4}");
-  const int lane = threadIdx.x & 31;
+  const uint32_t lane = threadIdx.x & 31;
+  const bool whole = parts == 1;
+  auto record = [&](uint32_t v) {
+    return v < g.n ? graph_record<MODE>(g, v) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  __syncwarp();  // (an earlier seed's reads of the shared memory are done)
+  if (lane == 0) my.kept[0][0] = record(seeds[s]);
+  __syncwarp();
+  uint32_t buf = 0;  // which of my.kept holds this hop's frontier
+  bool kept = true;  // ... if it does
   for (uint32_t hop = 0; hop < A.hops; hop++) {
     const uint32_t f = A.fan[hop];
-    const uint64_t Mf = div_magic(f);
-    const uint64_t Pall = hop ? A.width[hop - 1] : 1;
-    // this part's parents: Q consecutive ones under each of its first-hop children
-    const uint64_t Q = hop ? Pall / A.fan[0] : 1;
-    const uint64_t mine = hop ? (part < A.fan[0] ? (A.fan[0] - part + parts - 1) / parts : 0) : 1;
-    const uint64_t P = mine * Q;
-    auto parent = [&](uint64_t k) -> uint64_t {
-      return hop ? (part + (k / Q) * parts) * Q + k % Q : 0;
-    };
+    const uint64_t width = A.width[hop];
+    uint64_t P = 1, Q = 1;  // this part's parents: Q consecutive ones under each of its
+    if (hop) {              // first-hop children
+      P = A.width[hop - 1];
+      if (!whole) {
+        Q = P / A.fan[0];
+        P = part < A.fan[0] ? (uint64_t)((A.fan[0] - part + parts - 1) / parts) * Q : 0;
+      }
+    }
     const bool count = hop || part == 0;
     const bool last_hop = hop + 1 == A.hops;
+    const bool keep = whole && !last_hop && width <= kFrontier;
     const uint32_t G = f < (1u << 27) ? 32u : (uint32_t)max(1ull, 0xFFFFFFFFull / f);
-    const bool contig = parts == 1 && G == 32;
-    uint32_t *out = A.out[hop] + s * A.width[hop];
+    const bool contig = whole && G == 32;
+    const uint32_t dp = f < 32 ? 32 / f : f == 32 ? 1u : 0u, dk = f < 32 ? 32 - dp * f : f == 32 ? 0u : 32u;
+    const uint32_t p0 = f < 32 ? lane / f : 0u, k0 = lane - p0 * f;
+    uint32_t *out = A.out[hop] + s * width;
     const uint32_t *prev = hop ? A.out[hop - 1] + s * A.width[hop - 1] : nullptr;
+    uint32_t drawn = 0;
     for (uint64_t pc = 0; pc < P; pc += G) {
-      const uint64_t p = pc + lane;
-      uint32_t t = INVALID_VERTEX;
-      uint64_t ob = 0;
-      if (lane < (int)G && p < P) {
-        const uint64_t par = parent(p);
-        ob = par * f;
-        t = hop ? prev[par] : seeds[s];
+      const uint4 *rec = kept ? my.kept[buf] + pc : my.rec;
+      if (!kept) {
+        __syncwarp();
+        if (lane < G && pc + lane < P) {
+          uint64_t par = pc + lane;
+          if (!whole && hop) par = (part + par / Q * parts) * Q + par % Q;
+          my.ob[lane] = par * f;
+          my.rec[lane] = record(prev[par]);
+        }
+        __syncwarp();
+      } else if (!whole) {
+        if (lane == 0) my.ob[0] = 0;  // (the seed, the only frontier that parts keep)
+        __syncwarp();
       }
-      my.rec[lane] = t < g.n ? graph_record<MODE>(g, t) : make_uint4(0u, 0u, 0u, 0u);
-      my.ob[lane] = ob;
-      __syncwarp();
-      const uint32_t nP = (uint32_t)min((uint64_t)G, P - pc);
-      const uint32_t total = nP * f;  // < 2^32 by the choice of G
-      const uint64_t sbase = pc * f;  // contiguous groups: slot = sbase + j
-      u32x4 rw = u32x4{0, 0, 0, 0};
-      for (uint64_t j0 = 0; j0 < total; j0 += 32 * INFLIGHT) {  // warp-uniform
-        if (contig && (j0 & 127u) == 0)
-          rw = philox4x32_10(A.seed, (uint32_t)(((sbase + j0) >> 2) + (uint64_t)lane), (uint32_t)s,
-                             (uint32_t)(s >> 32), TAG_KHOP | hop);
-        uint32_t rnd[INFLIGHT];
-#pragma unroll
-        for (int u = 0; u < INFLIGHT; u++) {
-          rnd[u] = 0;
-          if (contig) {  // warp-uniform
-            // block ((j0 mod 128) + 32 u + lane) / 4 of the window, word lane & 3
-            const int src = (int)((((uint32_t)j0 & 127u) + 32u * u + (uint32_t)lane) >> 2);
-            const uint32_t x = __shfl_sync(kFull, rw.x, src), y = __shfl_sync(kFull, rw.y, src);
-            const uint32_t z = __shfl_sync(kFull, rw.z, src), w = __shfl_sync(kFull, rw.w, src);
-            rnd[u] = pick4(x, y, z, w, lane & 3);
-          }
+      const uint32_t total = (uint32_t)min((uint64_t)G, P - pc) * f;  // < 2^32 by the choice of G
+      const uint64_t sbase = pc * f;  // with one part: slot = sbase + j
+      uint32_t pl = p0, k = k0;       // the lane's draw: transit of the group, draw under it
+      for (uint32_t j0 = 0;; j0 += 32 * INFLIGHT) {  // warp-uniform
+        if (contig && (j0 & 127u) == 0) {
+          __syncwarp();
+          const u32x4 r = philox4x32_10(A.seed, (uint32_t)((sbase + j0) >> 2) + lane, (uint32_t)s,
+                                        (uint32_t)(s >> 32), TAG_KHOP | hop);
+          reinterpret_cast<uint4 *>(my.words)[lane] = make_uint4(r.x, r.y, r.z, r.w);
+          __syncwarp();
         }
         // phase 1: each draw's load; phase 2: its value, stored
         Sec S[INFLIGHT];
         DrawAt at[INFLIGHT];
-        uint32_t col[INFLIGHT];
+        uint32_t nv[INFLIGHT], y[INFLIGHT], d[INFLIGHT];
+        uint64_t slot[INFLIGHT];
 #pragma unroll
         for (int u = 0; u < INFLIGHT; u++) {
-          const uint64_t j = j0 + (uint64_t)u * 32 + lane;
-          if (j >= total) continue;
-          const uint32_t pl = div_by((uint32_t)j, f, Mf);
-          const VHdr h = record_header<MODE>(my.rec[pl]);
-          col[u] = h.base;  // (degree 1)
-          if (MODE == kCsr ? h.d == 0 : h.cb == 0) continue;
-          if (!contig) {
-            const uint64_t slot = my.ob[pl] + ((uint32_t)j - pl * f);
-            rnd[u] = pick(philox4x32_10(A.seed, (uint32_t)(slot >> 2), (uint32_t)s,
-                                        (uint32_t)(s >> 32), TAG_KHOP | hop),
-                          (int)(slot & 3));
+          const uint32_t j = j0 + u * 32 + lane;
+          d[u] = y[u] = 0;
+          nv[u] = INVALID_VERTEX;
+          slot[u] = ~0ull;
+          if (j < total && j >= j0) {  // (j may pass 2^32)
+            const uint4 r = rec[pl];
+            const VHdr h = record_header<MODE>(r);
+            slot[u] = whole ? sbase + j : my.ob[pl] + k;
+            uint32_t word;
+            if (contig)
+              word = my.words[j & 127u];
+            else
+              word = pick(philox4x32_10(A.seed, (uint32_t)(slot[u] >> 2), (uint32_t)s,
+                                        (uint32_t)(s >> 32), TAG_KHOP | hop), (int)(slot[u] & 3));
+            const uint32_t i = mulhi_u32(word, h.d);
+            d[u] = h.d;
+            nv[u] = h.base;
+            if constexpr (MODE == kCsr) {
+              if (h.d) nv[u] = load_cold_u32(g.cols + h.P + i);
+            } else if (h.cb) {
+              y[u] = r.y;
+              at[u] = draw_at(h, i);
+              S[u] = load_sector(g.words, at[u].sec);
+            }
           }
-          const uint32_t i = mulhi_u32(rnd[u], h.d);
-          if constexpr (MODE == kCsr) {
-            col[u] = load_cold_u32(g.cols + h.P + i);
-          } else {
-            at[u] = draw_at(h, i);
-            S[u] = load_sector(g.words, at[u].sec);
+          k += dk;
+          pl += dp;
+          if (k >= f) {
+            k -= f;
+            pl++;
           }
         }
 #pragma unroll
         for (int u = 0; u < INFLIGHT; u++) {
-          const uint64_t j = j0 + (uint64_t)u * 32 + lane;
-          if (j >= total) continue;
-          const uint32_t pl = div_by((uint32_t)j, f, Mf);
-          const VHdr h = record_header<MODE>(my.rec[pl]);
-          const uint64_t slot = contig ? sbase + j : my.ob[pl] + ((uint32_t)j - pl * f);
-          uint32_t nv = col[u];
-          if constexpr (MODE != kCsr)
-            if (h.cb) nv = draw_value(S[u], at[u], h);
-          const bool ok = nv < g.n;
-          if (h.d) {
+          if (slot[u] == ~0ull) continue;
+          if constexpr (MODE != kCsr) {
+            if (y[u]) {  // (a slot has bits, so its record's y is not 0)
+              VHdr h = record_header<MODE>(make_uint4(0u, y[u], 0u, nv[u]));
+              nv[u] = draw_value(S[u], at[u], h);
+            }
+          }
+          const bool ok = nv[u] < g.n;
+          if (d[u]) {
             bad |= !ok;
-            if (ok && count) cnt++;
+            drawn += ok;
           }
-          nv = h.d && ok ? nv : INVALID_VERTEX;
-          if (last_hop) store_out_u32(out + slot, nv);
-          else out[slot] = nv;  // read back by the next hop
+          const uint32_t v = d[u] && ok ? nv[u] : INVALID_VERTEX;
+          if (last_hop) store_out_u32(out + slot[u], v);
+          else out[slot[u]] = v;  // (read back by the next hop if it is not kept)
+          if (keep) my.kept[buf ^ 1][slot[u]] = record(v);
         }
+        if (total - j0 <= 32 * INFLIGHT) break;
       }
-      __syncwarp();
     }
+    if (count) cnt += drawn;
+    __syncwarp();
+    kept = keep;
+    buf ^= 1;
   }
 }
 
