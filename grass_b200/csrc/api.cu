@@ -466,6 +466,7 @@ int grass_close(grass_graph *g) {
   cudaFree(g->d_plan_big);
   cudaFree(g->d_plan_small);
   cudaFree(g->d_plan_flat);
+  cudaFree(g->d_fences);
   delete g;
   return GRASS_OK;
 }
@@ -645,6 +646,31 @@ static int node2vec_args(const grass_node2vec_params *p, grass_node2vec_params &
   return GRASS_OK;
 }
 
+// The graph's fences, or null: while the stream is being captured (nothing can
+// be allocated or waited for) or without memory the search goes without them,
+// with the same results.
+static const uint32_t *graph_fences(const grass_graph *g, cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(g->fence_mu);
+  if (g->d_fences || g->fences_tried) return g->d_fences;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  g->fences_tried = true;
+  uint32_t *f = nullptr;
+  if (cudaMalloc(&f, fence_words(g->n_words) * 4) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  launch_build_fences(g->view(), f, st);
+  if (cudaStreamSynchronize(st) != cudaSuccess) {  // (reported by the caller's own launch)
+    cudaFree(f);
+    return nullptr;
+  }
+  return g->d_fences = f;
+}
+
 int grass_node2vec(const grass_graph *g, const grass_node2vec_params *p,
                    const uint32_t *d_starts, uint64_t W, uint32_t *d_paths,
                    unsigned long long *d_edge_count, void *stream) {
@@ -656,8 +682,9 @@ int grass_node2vec(const grass_graph *g, const grass_node2vec_params *p,
   if (int rc = node2vec_args(p, r, t)) return rc;
   if (W && (!d_starts || !d_paths)) return set_error(GRASS_E_ARG, "node2vec: null buffers");
   DeviceGuard dg(g->device);
-  launch_node2vec(g->view(), r, t, d_starts, W, d_paths, d_edge_count, g->d_err,
-                  as_stream(stream));
+  DevGraph v = g->view();
+  if (W && t[1] != t[2]) v.fences = graph_fences(g, as_stream(stream));  // (else nothing is searched)
+  launch_node2vec(v, r, t, d_starts, W, d_paths, d_edge_count, g->d_err, as_stream(stream));
   return check_launch();
 }
 

@@ -27,6 +27,7 @@ struct DevGraph {
   int32_t mode;
   const uint64_t *__restrict__ rowptr;   // mode 2
   const uint32_t *__restrict__ cols;     // mode 2
+  const uint32_t *__restrict__ fences;   // node2vec: a head per 128-byte line (or null)
 };
 constexpr int GRASS_MODE_CSR_INTERNAL = 2;
 // Sampler template argument MODE.

@@ -69,6 +69,12 @@ struct grass_graph {
   mutable uint4 *d_plan_flat = nullptr;
   mutable uint64_t plan_nflat = 0;
   mutable bool plan_flat_ok = false;
+  // Fences of the node2vec membership search (kernels_sample.cu), built by the
+  // first grass_node2vec that is not being captured; null until then, and for
+  // good where there is no memory for them.
+  mutable std::mutex fence_mu;
+  mutable uint32_t *d_fences = nullptr;
+  mutable bool fences_tried = false;
   grass::DevGraph view() const {
     grass::DevGraph g;
     g.words = d_words;
@@ -78,6 +84,7 @@ struct grass_graph {
     g.mode = mode;
     g.rowptr = nullptr;
     g.cols = nullptr;
+    g.fences = nullptr;
     return g;
   }
 };
@@ -223,6 +230,9 @@ void launch_node2vec(const DevGraph &g, const grass_node2vec_params &p, const ui
                      const uint32_t *starts, uint64_t W, uint32_t *paths,
                      unsigned long long *edges, unsigned int *err, cudaStream_t s,
                      uint64_t w0 = 0);
+// Fences of a graph's slots: fence_words(n_words) words.
+uint64_t fence_words(uint64_t n_words);
+void launch_build_fences(const DevGraph &g, uint32_t *fences, cudaStream_t s);
 void launch_khop_csr(const DevCsr &c, const grass_khop_params &p, const uint32_t *seeds,
                      uint64_t S, uint32_t *const *hop_out, unsigned long long *edges,
                      cudaStream_t s);

@@ -70,15 +70,10 @@ struct N2vArgs {
   uint64_t t_ret, t_in, t_out;  // acceptance thresholds in [0, 2^32]
 };
 
-// The head of slot c (its first neighbor less n_0): one field of at most 32
-// bits, read as one or two 32-bit words (the second only when the field
-// crosses into it).
-__device__ __forceinline__ uint32_t slot_head(const DevGraph &g, const VHdr &h, uint32_t c) {
-  const DrawAt at = slot_at(h, c);
-  const uint32_t *q = g.words + (uint64_t)at.sec * 8 + (at.off >> 5);
-  const uint32_t s = at.off & 31u;
-  const uint32_t hi = ldw(q), lo = s + h.a > 32u ? ldw(q + 1) : 0u;
-  return shr_clamp(__funnelshift_l(lo, hi, s), 32u - h.a);
+// The head of the first slot of sector q (from the vertex's first): one field
+// of at most 32 bits at the sector's first bit.
+__device__ __forceinline__ uint32_t sector_head(const DevGraph &g, const VHdr &h, uint32_t q) {
+  return shr_clamp(ldw(g.words + (uint64_t)(h.sec + q) * 8), 32u - h.a);
 }
 
 // The last index in [lo, hi] whose key is <= x, given key(lo) <= x, for
@@ -95,10 +90,10 @@ __device__ __forceinline__ uint32_t last_le(uint32_t lo, uint32_t hi, uint32_t x
   return lo;
 }
 
-// Whether x is a neighbor of the vertex of header h.  Compressed: a search
-// over the slots' heads for the one slot that can hold x, then a search of
-// that slot's offsets inside its sector, in registers.  CSR: a search of the
-// row.
+// Whether x is a neighbor of the vertex of header h.  Compressed: a search for
+// the one sector that can hold x, over the fences (see build_fences_kernel) for
+// its line and over the line's sectors' first heads, then for the slot and the
+// neighbor inside that sector, in registers.  CSR: a search of the row.
 template <int MODE>
 __device__ __forceinline__ bool has_neighbor(const DevGraph &g, const VHdr &h, uint32_t x) {
   if (h.d == 0) return false;
@@ -109,27 +104,51 @@ __device__ __forceinline__ bool has_neighbor(const DevGraph &g, const VHdr &h, u
   } else {
     if (x <= h.base || h.cb == 0) return x == h.base;
     const uint32_t y = x - h.base;
-    const uint32_t c = last_le(0u, div_small(h.d - 1, h.T), y,
-                               [&](uint32_t k) { return slot_head(g, h, k); });
-    const DrawAt at = slot_at(h, c);
-    const Sec A = load_sector(g.words, at.sec);
-    const uint32_t z = y - sec_field(A, at.off, h.a);  // the offset looked for
+    const uint32_t slots = div_small(h.d - 1, h.T) + 1;
+    uint32_t q = 0, last = div_small(slots - 1, h.K);  // sectors, from the vertex's first
+    const uint32_t l0 = h.sec / 4, l1 = (h.sec + last) / 4;
+    if (g.fences && l1 > l0) {
+      // (fence l0 is the line's owner's, never read: the probes are above it)
+      const uint32_t l = last_le(l0, l1, y, [&](uint32_t k) { return ldw(g.fences + k); });
+      q = l > l0 ? l * 4 - h.sec : 0;
+      last = min(last, l * 4 + 3 - h.sec);
+    }
+    q = last_le(q, last, y, [&](uint32_t k) { return sector_head(g, h, k); });
+    const Sec A = load_sector(g.words, h.sec + q);
+    const uint32_t c0 = q * h.K, n = min(h.K, slots - c0);
+    auto head = [&](uint32_t c) { return sec_field(A, h.off + c * h.cb, h.a); };
+    const uint32_t c = last_le(0u, n - 1, y, head);
+    const uint32_t at = h.off + c * h.cb, z = y - sec_field(A, at, h.a);  // the offset looked for
     if (z == 0) return true;
-    const uint32_t last = min(h.T, h.d - c * h.T) - 1;
     auto offset = [&](uint32_t id) {  // of index id in the slot
-      return sec_field(A, at.off + h.a + (id - 1) * h.b, id ? h.b : 0u);
+      return sec_field(A, at + h.a + (id - 1) * h.b, id ? h.b : 0u);
     };
-    return offset(last_le(0u, last, z, offset)) == z;
+    return offset(last_le(0u, min(h.T, h.d - (c0 + c) * h.T) - 1, z, offset)) == z;
   }
 }
 
-// Resident 256-thread blocks per SM the node2vec kernels are compiled for.
-// The walk is latency-bound (dependent sector reads, divergent tries), so
-// resident warps matter more than registers: on the 1M x 80 walk the
-// compressed kernels at 4 blocks (64 registers) ran 1.6x faster than at 118
-// registers (2 blocks; unbounded builds also came out at 134, 1 block), 1.2x
-// faster than at 3 blocks, and 1.1-1.2x faster than at 5 or 6, where spills
-// grow.  The CSR kernel needs no cap (69 registers, 3 blocks).
+// Fences for the membership search: word l is the head of the first slot in
+// 128-byte line l where that line begins inside a vertex of several sectors
+// (other words are not written).  A search over a hub's heads took 3.6 reads
+// that missed L2, 12 in all; the fences are 1/32 of the slots' size, a hub's
+// lie side by side, and what they leave is one line.  Built by the first
+// node2vec call on a graph; one warp per vertex.
+__global__ void __launch_bounds__(256) build_fences_kernel(DevGraph g, uint32_t *fences) {
+  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t v = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; v < g.n; v += nwarps) {
+    const VHdr h = record_header<kSlots>(load_record(g.recs + v));
+    if (h.d < 2) continue;
+    const uint32_t last = div_small(div_small(h.d - 1, h.T), h.K);
+    for (uint32_t l = h.sec / 4 + 1 + (threadIdx.x & 31); l <= (h.sec + last) / 4; l += 32)
+      fences[l] = sector_head(g, h, l * 4 - h.sec);
+  }
+}
+
+// Resident 256-thread blocks per SM the node2vec kernels are compiled for: the
+// walk waits on dependent sector reads, so resident warps matter more than
+// registers until those spill.  262,144 walkers x 80, p = 1, q = 0.5, R-MAT s22
+// ef32: 1.45 ms at 4 blocks (53 registers), 1.56 at 5, 1.86 at 6.  The CSR
+// kernel needs no cap (42 registers).
 #ifndef GRASS_N2V_MIN_BLOCKS
 #define GRASS_N2V_MIN_BLOCKS 4
 #endif
@@ -137,6 +156,12 @@ __device__ __forceinline__ bool has_neighbor(const DevGraph &g, const VHdr &h, u
 #define GRASS_N2V_CSR_MIN_BLOCKS 1
 #endif
 
+// A lane goes its own way through tries, steps and walkers: a turn of the loop
+// is one candidate for every lane, a first try for most, and the lanes that
+// search do so together.  (With the tries of a step in a loop of their own, all
+// lanes waited for the last one's: 2.43 against 2.14 ms, and 1.45 with the
+// fences.  41 M of its reads miss L2; at the rate of random reads they take
+// 0.9.)
 template <int MODE>
 __global__ void __launch_bounds__(256, MODE == kCsr ? GRASS_N2V_CSR_MIN_BLOCKS : GRASS_N2V_MIN_BLOCKS) n2v_kernel(DevGraph g, const uint32_t *__restrict__ starts,
                                                   uint64_t W, N2vArgs a,
@@ -146,49 +171,61 @@ __global__ void __launch_bounds__(256, MODE == kCsr ? GRASS_N2V_CSR_MIN_BLOCKS :
   const uint64_t t_lo = min(a.t_in, a.t_out), t_hi = max(a.t_in, a.t_out);
   uint64_t cnt = 0;
   bool bad = false;
-  for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < W; w += nthreads) {
-    const uint64_t id = a.w0 + w;
-    const uint32_t s0 = starts[w];
-    store_path(paths, a.layout, W, a.L, w, 0, s0);
-    uint32_t v = s0 < g.n ? s0 : INVALID_VERTEX, u = INVALID_VERTEX;
-    VHdr hu;  // the previous vertex's header (kept from the step that left it)
-    hu.d = 0;
-    for (uint32_t s = 0; s < a.L; s++) {
-      if (v != INVALID_VERTEX) {
-        const VHdr h = header<MODE>(g, v);
-        if (h.d == 0) {
-          v = INVALID_VERTEX;
-        } else {
-          uint32_t x = INVALID_VERTEX;
-          for (uint32_t k = 0; k < a.max_tries; k++) {
-            const u32x4 r =
-                philox4x32_10(a.seed, s, (uint32_t)id, (uint32_t)(id >> 32), TAG_N2V | k);
-            x = neighbor<MODE>(g, h, mulhi_u32(r.x, h.d));
-            if (s == 0 || k + 1 == a.max_tries) break;  // first step: uniform
-            const uint64_t y = r.y;
-            if (x == u) {
-              if (y < a.t_ret) break;
-              continue;
-            }
-            // below both thresholds the candidate is taken, at or above both it
-            // is not, whether or not it is a neighbor of u: only in between does
-            // the membership search run (never when t_in == t_out, i.e. q = 1)
-            if (y < t_lo) break;
-            if (y >= t_hi) continue;
-            if (y < (has_neighbor<MODE>(g, hu, x) ? a.t_in : a.t_out)) break;
-          }
-          if (x >= g.n) {
-            bad = true;
-            v = INVALID_VERTEX;
-          } else {
-            u = v;
-            hu = h;
-            v = x;
-            cnt++;
-          }
-        }
+  uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;  // the lane's walker
+  uint32_t s = a.L, k = 0;  // its step and try (s == L: take the next walker)
+  uint32_t v = INVALID_VERTEX, u = INVALID_VERTEX;
+  uint4 rv = make_uint4(0, 0, 0, 0), ru = rv;  // records of v and of the vertex before it
+  bool fresh = false;  // v's record is not loaded yet
+  bool first = true;
+  for (;;) {  // warp-uniform: one candidate for every lane
+    while (s == a.L && w < W) {  // (a loop for walks of no steps)
+      if (!first) w += nthreads;
+      first = false;
+      if (w >= W) break;
+      const uint32_t s0 = starts[w];
+      store_path(paths, a.layout, W, a.L, w, 0, s0);
+      v = s0 < g.n ? s0 : INVALID_VERTEX;
+      u = INVALID_VERTEX;
+      s = k = 0;
+      fresh = true;
+    }
+    const bool live = w < W;
+    if (!__any_sync(kFull, live)) break;
+    if (live && fresh) {
+      rv = walk_record<MODE>(g, v);
+      fresh = false;
+      if (rv.z == 0) {  // the walk stops
+        for (; s < a.L; s++) store_path(paths, a.layout, W, a.L, w, s + 1, INVALID_VERTEX);
       }
-      store_path(paths, a.layout, W, a.L, w, s + 1, v);
+    }
+    if (live && s < a.L) {
+      const uint64_t id = a.w0 + w;
+      const u32x4 r = philox4x32_10(a.seed, s, (uint32_t)id, (uint32_t)(id >> 32), TAG_N2V | k);
+      const VHdr h = record_header<MODE>(rv);
+      const uint32_t x = neighbor<MODE>(g, h, mulhi_u32(r.x, h.d));
+      const uint64_t y = r.y;
+      // below both thresholds the candidate is taken, at or above both it is
+      // not, whether or not it is a neighbor of u: only in between does the
+      // membership search run (never when t_in == t_out, i.e. q = 1)
+      bool take = s == 0 || k + 1 == a.max_tries;  // (first step: uniform)
+      if (!take) {
+        if (x == u) take = y < a.t_ret;
+        else if (y < t_lo) take = true;
+        else if (y < t_hi) take = y < (has_neighbor<MODE>(g, record_header<MODE>(ru), x) ? a.t_in : a.t_out);
+      }
+      k++;
+      if (take) {
+        const bool ok = x < g.n;
+        bad |= !ok;
+        cnt += ok;
+        u = v;
+        ru = rv;
+        v = ok ? x : INVALID_VERTEX;
+        store_path(paths, a.layout, W, a.L, w, s + 1, v);
+        s++;
+        k = 0;
+        fresh = true;
+      }
     }
   }
   warp_add_u64(edges, cnt);
@@ -711,6 +748,13 @@ void launch_khop(const DevGraph &g, const grass_khop_params &p, const uint32_t *
   const KhopArgs A = khop_args(p, hop_out);
   const unsigned grid = grid_warps(S, 8, cur_dev(), 8);
   khop_kernel<kSlots><<<grid, 256, 0, s>>>(g, seeds, S, A, edges, err);
+  count_launch();
+}
+
+uint64_t fence_words(uint64_t n_words) { return n_words / 32 + 1; }
+
+void launch_build_fences(const DevGraph &g, uint32_t *fences, cudaStream_t s) {
+  build_fences_kernel<<<grid_warps(g.n, 8, cur_dev(), 8), 256, 0, s>>>(g, fences);
   count_launch();
 }
 
