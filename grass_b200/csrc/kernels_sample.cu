@@ -511,8 +511,8 @@ __global__ void __launch_bounds__(256, GRASS_MRW_DEGREE_MIN_BLOCKS)
 
 // Multi random walk, one block per sample, walkers in parallel (mrw_cta.cuh);
 // scratch holds `stride` bytes per block, reused for its samples.
-template <int MODE>
-__global__ void __launch_bounds__(512) mrw_cta_kernel(DevGraph g, uint32_t *__restrict__ roots,
+template <int MODE, int NW>
+__global__ void __launch_bounds__(32 * NW) mrw_cta_kernel(DevGraph g, uint32_t *__restrict__ roots,
                                                       uint64_t S, uint32_t R, uint32_t T,
                                                       uint32_t select, uint64_t seed,
                                                       uint32_t *__restrict__ src,
@@ -520,12 +520,12 @@ __global__ void __launch_bounds__(512) mrw_cta_kernel(DevGraph g, uint32_t *__re
                                                       unsigned char *scratch, uint64_t stride,
                                                       unsigned long long *edges,
                                                       unsigned int *err) {
-  __shared__ CtaSmem<16> sm;
+  __shared__ CtaSmem<NW> sm;
   unsigned char *scr = scratch + blockIdx.x * stride;
   uint64_t cnt = 0;
   bool bad = false;
   for (uint64_t s = blockIdx.x; s < S; s += gridDim.x)
-    mrw_cta_sample<MODE, 16>(g, roots + s * R, src + s * T, dst + s * T, R, T, select, seed, s,
+    mrw_cta_sample<MODE, NW>(g, roots + s * R, src + s * T, dst + s * T, R, T, select, seed, s,
                              scr, sm, cnt, bad);
   warp_add_u64(edges, cnt);
   if (bad && err) atomicOr(err, 1u);
@@ -830,21 +830,27 @@ int launch_mrw(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots, ui
   // samples 46 / 73, 600 103 / 120, 1184 122 / 133, 8192 706 / 300; 2000 x
   // 1024, r = 148: 148 36 / 59, 600 137 / 95; 2000 x 10,000: 600 527 / 723,
   // 1184 865 / 759.  At 100 steps a warp is never slower.
-  const int threads = (int)std::min<uint64_t>(
-      512, std::max<uint64_t>(128, ((uint64_t)p.walkers / 2 + 31) / 32 * 32));
+  // Continuous time with many walkers: 1024 threads at 64 registers (2000 walkers
+  // x 10,000 steps, 1 / 51 samples: 246 / 320 us, 512 threads 279 / 400); with
+  // few, the 116 registers pay (80 x 100, 2000 samples: 279 us against 331).
+  const bool ct = p.select == GRASS_SELECT_DEGREE_CT, wide = ct && p.walkers > 512;
+  const uint64_t want = ct ? p.walkers : p.walkers / 2;
+  const int threads = (int)std::min<uint64_t>(wide ? 1024 : 512,
+                                              std::max<uint64_t>(128, (want + 31) / 32 * 32));
+  auto cta = wide ? mrw_cta_kernel<kSlots, 32> : mrw_cta_kernel<kSlots, 16>;
   uint64_t resident = 0;
-  if (p.select == GRASS_SELECT_DEGREE_CT || (p.select == GRASS_SELECT_UNIFORM && p.steps >= 512)) {
+  if (ct || (p.select == GRASS_SELECT_UNIFORM && p.steps >= 512)) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mrw_cta_kernel<kSlots>, threads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cta, threads, 0);
     resident = (uint64_t)sm_count(cur_dev()) * std::max(per_sm, 1);
   }
-  if (p.select == GRASS_SELECT_DEGREE_CT || S <= resident + resident * p.steps / 2048) {
+  if (ct || S <= resident + resident * p.steps / 2048) {
     const uint64_t grid = std::min<uint64_t>(S, resident);
     const uint64_t stride = mrw_sample_scratch(p.walkers, p.steps, p.select);
     unsigned char *scr = nullptr;
     cudaError_t e = scratch_alloc(reinterpret_cast<void **>(&scr), grid * stride, s);
     if (e != cudaSuccess) return cuda_fail(e, "multi-RW scratch");
-    mrw_cta_kernel<kSlots><<<(unsigned)grid, threads, 0, s>>>(
+    cta<<<(unsigned)grid, threads, 0, s>>>(
         g, roots, S, p.walkers, p.steps, p.select, p.seed, src, dst, scr, stride, edges, err);
     count_launch();
     scratch_free(scr, s);

@@ -36,6 +36,36 @@ struct CtWalker {
   double t;               // time of event k (+inf when the walker cannot move)
 };
 
+// The next vertices of G walkers at once: go[q] walkers at records r[q] draw
+// with word[q].  All slot loads are issued before any is decoded.
+template <int MODE, int G>
+__device__ __forceinline__ void draw_all(const DevGraph &g, const bool (&go)[G], const uint4 (&r)[G],
+                                         const uint32_t (&word)[G], uint32_t (&nv)[G]) {
+  DrawAt at[G];
+  Sec S[G];
+#pragma unroll
+  for (int q = 0; q < G; q++) {
+    nv[q] = r[q].w;  // (degree 1)
+    if (!go[q]) continue;
+    const VHdr h = record_header<MODE>(r[q]);
+    const uint32_t i = mulhi_u32(word[q], h.d);
+    if constexpr (MODE == kCsr) {
+      nv[q] = load_cold_u32(g.cols + h.P + i);
+    } else if (h.cb) {
+      at[q] = draw_at(h, i);
+      S[q] = load_sector(g.words, at[q].sec);
+    }
+  }
+  if constexpr (MODE != kCsr) {
+#pragma unroll
+    for (int q = 0; q < G; q++) {
+      if (!go[q]) continue;
+      const VHdr h = record_header<MODE>(r[q]);
+      if (h.cb) nv[q] = draw_value(S[q], at[q], h);
+    }
+  }
+}
+
 // Block workspace; NW = most warps per block.
 template <int NW>
 struct CtaSmem {
@@ -205,6 +235,53 @@ __device__ CtEvent *cta_sort_events(CtEvent *a, CtEvent *b, uint32_t n, CtaSmem<
   return a;
 }
 
+// Orders a[0..n), events at times in [0, H], by (time, walker): copies them to
+// b grouped by bucket of time, and writes ord[r] = the place in b of the event
+// of rank r.  The total rate of events changes little, so their times spread
+// evenly: a few events a bucket, and an event's rank in its bucket is a count
+// over it.  One pass where the radix sort takes one per differing byte of the
+// time (2000 walkers x 10,000 events: 177 us of a sample's 415; with this 250).
+// False, with nothing usable written, where the buckets would be too full.
+template <int NW>
+__device__ bool cta_bucket_order(const CtEvent *a, CtEvent *b, uint32_t *ord, uint32_t n, double H,
+                                 CtaSmem<NW> &sm) {
+  constexpr uint32_t kBuckets = NW * 256;
+  constexpr uint32_t kFull32 = 32;  // most events of a bucket
+  const uint32_t tid = threadIdx.x, nt = blockDim.x;
+  if (n > 8 * kBuckets) return false;
+  uint32_t *cnt = &sm.hist[0][0];
+  const double scale = kBuckets / H;
+  auto bucket = [&](uint64_t t) {  // (does not decrease with the time)
+    return min(kBuckets - 1, (uint32_t)(bits_f64(t) * scale));
+  };
+  for (uint32_t i = tid; i < kBuckets; i += nt) cnt[i] = 0;
+  __syncthreads();
+  for (uint32_t i = tid; i < n; i += nt) atomicAdd(&cnt[bucket(a[i].t)], 1u);
+  __syncthreads();
+  bool full = false;
+  for (uint32_t i = tid; i < kBuckets; i += nt) full |= cnt[i] > kFull32;
+  if (__syncthreads_or(full)) return false;
+  cta_exclusive_scan(cnt, kBuckets, sm);
+  for (uint32_t i = tid; i < n; i += nt) {
+    const CtEvent e = a[i];
+    b[atomicAdd(&cnt[bucket(e.t)], 1u)] = e;  // cnt: first place of the bucket, then its end
+  }
+  __syncthreads();
+  for (uint32_t i = tid; i < n; i += nt) {
+    const uint64_t t = b[i].t;
+    const uint32_t w = b[i].w, k = bucket(t), end = cnt[k];
+    const uint32_t first = k ? cnt[k - 1] : 0u;
+    uint32_t r = first;
+    for (uint32_t j = first; j < end; j++) {
+      const uint64_t tj = b[j].t;
+      r += tj < t || (tj == t && b[j].w < w);
+    }
+    ord[r] = i;
+  }
+  __syncthreads();
+  return true;
+}
+
 // Uniform multi-RW of one sample by the whole block.  scr: R + 1 + T words.
 // Step t: walker mulhi(word 0, R), neighbor mulhi(word 1, d) of
 // Philox(seed; t, sample, .., TAG_MRW) -- the stream of mrw_uniform_warp.
@@ -224,8 +301,9 @@ __device__ void mrw_uniform_cta(const DevGraph &g, uint32_t *roots, uint32_t *sr
   for (uint32_t t = tid; t < T; t += nt)
     list[atomicAdd(&cur[mulhi_u32(philox4x32_10(seed, t, s_lo, s_hi, TAG_MRW).x, R)], 1u)] = t;
   __syncthreads();
-  // Walker w's steps are list[cur[w-1] .. cur[w]) (cur[-1] = 0); two walkers
-  // per thread advance together so their DRAM reads overlap.
+  // Walker w's steps are list[cur[w-1] .. cur[w]) (cur[-1] = 0); two walkers per
+  // thread advance together so that their reads overlap (2000 walkers x 10,000
+  // steps, 600 samples: 0.484 ms, one at a time 0.541, three 0.540).
   constexpr int G = 2;
   for (uint32_t w0 = tid; w0 < R; w0 += G * nt) {
     uint32_t pos[G], end[G], v[G];
@@ -253,31 +331,36 @@ __device__ void mrw_uniform_cta(const DevGraph &g, uint32_t *roots, uint32_t *sr
       }
     }
     for (;;) {
-      bool any = false;
+      bool any = false, go[G];
+      uint32_t t[G], word[G], nv[G];
 #pragma unroll
       for (int q = 0; q < G; q++) {
-        if (pos[q] >= end[q]) continue;
-        any = true;
-        const uint32_t t = list[pos[q]++];
-        src[t] = v[q];
+        go[q] = pos[q] < end[q];
+        any |= go[q];
+        word[q] = 0;
+        if (!go[q]) continue;
+        t[q] = list[pos[q]++];
+        src[t[q]] = v[q];
         if (rc[q].z == 0) {
-          dst[t] = INVALID_VERTEX;
+          dst[t[q]] = INVALID_VERTEX;
+          go[q] = false;
           continue;
         }
-        const uint32_t ry = philox4x32_10(seed, t, s_lo, s_hi, TAG_MRW).y;
-        const VHdr h = record_header<MODE>(rc[q]);
-        const uint32_t nv = neighbor<MODE>(g, h, mulhi_u32(ry, h.d));
-        if (nv >= g.n) {
-          bad = true;
-          dst[t] = INVALID_VERTEX;
-          continue;
-        }
-        dst[t] = nv;
-        cnt++;
-        v[q] = nv;
-        rc[q] = graph_record<MODE>(g, nv);
+        word[q] = philox4x32_10(seed, t[q], s_lo, s_hi, TAG_MRW).y;
       }
       if (!any) break;
+      draw_all<MODE, G>(g, go, rc, word, nv);
+#pragma unroll
+      for (int q = 0; q < G; q++) {
+        if (!go[q]) continue;
+        const bool ok = nv[q] < g.n;
+        dst[t[q]] = ok ? nv[q] : INVALID_VERTEX;
+        bad |= !ok;
+        if (!ok) continue;
+        cnt++;
+        v[q] = nv[q];
+        rc[q] = graph_record<MODE>(g, nv[q]);
+      }
     }
 #pragma unroll
     for (int q = 0; q < G; q++)
@@ -317,7 +400,7 @@ __device__ void mrw_ct_cta(const DevGraph &g, uint32_t *roots, uint32_t *src, ui
   CtEvent *B = A + cap;
   uint32_t N = 0;
   bool done = false;
-  double frac = 0.5, ext = 0.75;
+  double frac = 0.5, ext = 0.75, H = 0.0;
   for (int attempt = 0; attempt < 6 && !done; attempt++) {
     uint64_t dsum = 0;
     for (uint32_t w = tid; w < R; w += nt) {
@@ -339,55 +422,32 @@ __device__ void mrw_ct_cta(const DevGraph &g, uint32_t *roots, uint32_t *src, ui
       done = true;
       break;
     }
-    double H = frac * (double)T / (double)dsum;
+    H = frac * (double)T / (double)dsum;
     bool overflow = false;
     for (int phase = 0; phase < 512; phase++) {
-      // Every walker runs its events with time <= H; two per thread together.
-      constexpr int G = 2;
-      for (uint32_t w0 = tid; w0 < R; w0 += G * nt) {
-        CtWalker s[G];
-        uint4 r[G];
-#pragma unroll
-        for (int q = 0; q < G; q++) {
-          const uint32_t w = w0 + q * nt;
-          if (w < R) {
-            s[q] = W[w];
-            r[q] = rec[w];
-          } else {
-            s[q].t = ct_inf();
+      // Every walker runs its events with time <= H.  (One walker per thread at
+      // a time: two or four side by side took 286 and 371 us a sample, not 250;
+      // few walkers have many events in a phase.)
+      for (uint32_t w = tid; w < R; w += nt) {
+        CtWalker s = W[w];
+        if (!(s.t <= H)) continue;
+        uint4 r = rec[w];
+        do {
+          const uint32_t nv = neighbor<MODE>(g, record_header<MODE>(r), mulhi_u32(s.z, r.z));
+          if (nv >= g.n) {  // corrupt payload: the walker stops
+            bad = true;
+            s.t = ct_inf();
+            break;
           }
-        }
-        for (;;) {
-          bool any = false;
-#pragma unroll
-          for (int q = 0; q < G; q++) {
-            if (!(s[q].t <= H)) continue;
-            any = true;
-            const uint32_t w = w0 + q * nt;
-            const VHdr h = record_header<MODE>(r[q]);
-            const uint32_t nv = neighbor<MODE>(g, h, mulhi_u32(s[q].z, h.d));
-            if (nv >= g.n) {  // corrupt payload: the walker stops
-              bad = true;
-              s[q].t = ct_inf();
-              continue;
-            }
-            const uint32_t idx = atomicAdd(&sm.n_events, 1u);
-            if (idx < cap) A[idx] = CtEvent{f64_bits(s[q].t), w, s[q].v, nv, 0u};
-            r[q] = graph_record<MODE>(g, nv);
-            s[q].v = nv;
-            s[q].k++;
-            ct_arm(s[q], r[q], seed, s_lo, w, s[q].t);
-          }
-          if (!any) break;
-        }
-#pragma unroll
-        for (int q = 0; q < G; q++) {
-          const uint32_t w = w0 + q * nt;
-          if (w < R) {
-            W[w] = s[q];
-            rec[w] = r[q];
-          }
-        }
+          r = graph_record<MODE>(g, nv);
+          const uint32_t idx = atomicAdd(&sm.n_events, 1u);
+          if (idx < cap) A[idx] = CtEvent{f64_bits(s.t), w, s.v, nv, 0u};
+          s.v = nv;
+          s.k++;
+          ct_arm(s, r, seed, s_lo, w, s.t);
+        } while (s.t <= H);
+        W[w] = s;
+        rec[w] = r;
       }
       __syncthreads();
       N = sm.n_events;
@@ -421,23 +481,32 @@ __device__ void mrw_ct_cta(const DevGraph &g, uint32_t *roots, uint32_t *src, ui
     bad = true;
     N = 0;
   }
-  const CtEvent *E = cta_sort_events(A, B, N, sm);
+  // Event of rank r: E[ord[r]], or E[r] after the sort.
+  uint32_t *ord = reinterpret_cast<uint32_t *>(A);
+  const CtEvent *E = B;
+  if (!cta_bucket_order(A, B, ord, N, H, sm)) {
+    E = cta_sort_events(A, B, N, sm);
+    ord = nullptr;
+  }
   for (uint32_t r = tid; r < T; r += nt) {
+    uint32_t from = INVALID_VERTEX, to = INVALID_VERTEX;
     if (r < N) {
-      src[r] = E[r].src;
-      dst[r] = E[r].dst;
-    } else {
-      src[r] = INVALID_VERTEX;
-      dst[r] = INVALID_VERTEX;
+      const CtEvent &e = E[ord ? ord[r] : r];
+      from = e.src;
+      to = e.dst;
     }
+    src[r] = from;
+    dst[r] = to;
   }
   // Final vertices: before each walker's first event past the T-th.
   for (uint32_t w = tid; w < R; w += nt) first[w] = 0xFFFFFFFFu;
   __syncthreads();
-  for (uint32_t r = T + tid; r < N; r += nt) atomicMin(&first[E[r].w], r);
+  for (uint32_t r = T + tid; r < N; r += nt) atomicMin(&first[E[ord ? ord[r] : r].w], r);
   __syncthreads();
-  for (uint32_t w = tid; w < R; w += nt)
-    roots[w] = first[w] != 0xFFFFFFFFu ? E[first[w]].src : W[w].v;
+  for (uint32_t w = tid; w < R; w += nt) {
+    const uint32_t r = first[w];
+    roots[w] = r != 0xFFFFFFFFu ? E[ord ? ord[r] : r].src : W[w].v;
+  }
   if (tid == 0) cnt += min(N, T);
   __syncthreads();
 }
