@@ -28,6 +28,15 @@ struct BatchTask {
   uint64_t begin, end;
 };
 
+// The work items by kind, in this order: ends of the block-level multi-RW
+// samples, the sequential multi-RW samples, the k-hop seeds and the walker
+// tiles.  parts: warps per k-hop seed.
+struct BatchRanges {
+  uint32_t cta, mrw, khop, rw, parts;
+};
+// Words of the device queue: a counter per kind, zero before a run.
+constexpr uint32_t kQueueWords = 4;
+
 // Zero fields of a config take the defaults for this decode mode.
 grass_batch_config resolve_batch_config(const grass_batch_config &c, int mode);
 
@@ -65,12 +74,34 @@ void split_job(const grass_job &j, uint32_t ji, const grass_batch_config &c,
                std::vector<BatchTask> &cta, std::vector<BatchTask> &mrw,
                std::vector<BatchTask> &khop, std::vector<BatchTask> &rw);
 
-// Launches the persistent kernel on graph `dg` (compressed or CSR) of device
-// `device` over ntasks work items, the first ncta of them block-level.
-// d_queue: two zeroed counters.  Corrupt payloads set bit 0 of *d_err.
+inline BatchRanges batch_ranges(const std::vector<BatchTask> &cta, const std::vector<BatchTask> &mrw,
+                                const std::vector<BatchTask> &khop,
+                                const std::vector<BatchTask> &rw, const grass_batch_config &c) {
+  BatchRanges r;
+  r.cta = (uint32_t)cta.size();
+  r.mrw = r.cta + (uint32_t)mrw.size();
+  r.khop = r.mrw + (uint32_t)khop.size();
+  r.rw = r.khop + (uint32_t)rw.size();
+  r.parts = c.warps_per_vertex;
+  return r;
+}
+
+// A stream and events beside a batch's stream, for its block-level items.
+struct BatchSide {
+  cudaStream_t st = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  cudaError_t create();  // once; a second call does nothing
+  void destroy();
+};
+
+// Launches the persistent kernels on graph `dg` (compressed or CSR) of device
+// `device` over the work items of `ranges`: block-level and warp-level items
+// have a kernel each, which run side by side where both kinds are present
+// (side, created here, joins stream s again).  d_queue: kQueueWords zeroed
+// words.  Corrupt payloads set bit 0 of *d_err.
 int launch_batch(const DevGraph &dg, int device, const BatchJob *d_jobs, const BatchTask *d_tasks,
-                 uint32_t ncta, uint32_t ntasks, unsigned int *d_queue,
-                 unsigned long long *d_total, unsigned int *d_err, cudaStream_t s,
+                 const BatchRanges &ranges, unsigned int *d_queue, unsigned long long *d_total,
+                 unsigned int *d_err, cudaStream_t s, BatchSide &side,
                  const grass_batch_config &c);
 
 }  // namespace grass

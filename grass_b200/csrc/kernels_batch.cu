@@ -4,11 +4,11 @@
 // pipeline per step (GT/src/grass.cu:1417-2037).  Here a batch holds any mix
 // of RW, k-hop and multi-RW jobs with their own sizes, parameters and seeds.
 // The host splits them into work items -- one multi-RW sample, a few k-hop
-// seeds, or a tile of walkers -- ordered longest first (multi-RW chains are
-// sequential by definition), and a persistent kernel's warps pull items from
-// a device counter until the queue is empty.  The queue reset, the restore of
-// the multi-RW start vertices and the kernel are captured once into a CUDA
-// graph and replayed by every run.
+// seeds, or a tile of walkers -- and a persistent kernel's warps pull items from
+// device counters, one kind after the other, until the queues are empty;
+// multi-RW samples that take a whole block have a kernel of their own beside
+// it.  The queue reset, the restore of the multi-RW start vertices and the
+// kernels are captured once into a CUDA graph and replayed by every run.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -16,9 +16,9 @@
 
 #include "batch.h"
 
-// Resident blocks per SM the compiler must allow for (the register budget):
-// the batched-jobs workload waits on memory, so more resident warps pay until
-// spills cost more.
+// Resident 256-thread blocks per SM the compiler must allow for: the items wait
+// on memory, so more resident warps pay until spills cost more (the 256-job mix
+// on R-MAT s22 ef32: 1.25 ms at 4, 1.33 at 3).
 #ifndef GRASS_BATCH_MIN_BLOCKS
 #define GRASS_BATCH_MIN_BLOCKS 4
 #endif
@@ -26,31 +26,49 @@
 namespace grass {
 namespace {
 
-template <int MODE, int DEPTH>
-__global__ void __launch_bounds__(256, GRASS_BATCH_MIN_BLOCKS) batch_kernel(DevGraph g, const BatchJob *__restrict__ jobs,
-                                                    const BatchTask *__restrict__ tasks,
-                                                    uint32_t ncta, uint32_t ntasks,
-                                                    unsigned int *queue,
-                                                    unsigned long long *total,
-                                                    unsigned int *err) {
-  union WarpSmem {  // a warp runs one kind of item at a time
-    SmemHdr khop;
-    uint32_t stage[kPathStageWords<DEPTH>];
-  };
-  __shared__ __align__(16) unsigned char warp_smem[8 * sizeof(WarpSmem)];
-  WarpSmem *sh = reinterpret_cast<WarpSmem *>(warp_smem);
-  __shared__ CtaSmem<8> csm;
-  SmemHdr &my = sh[threadIdx.x >> 5].khop;
-  const int lane = threadIdx.x & 31;
+// Runs `body` on the items [first, end) that the calling warp takes from the
+// counter `queue`, `grab` at a time.
+template <class Body>
+__device__ __forceinline__ void take_items(const BatchTask *tasks, uint32_t first, uint32_t end,
+                                           uint32_t grab, unsigned int *queue, Body body) {
+  while (first < end) {
+    uint32_t t = 0;
+    if ((threadIdx.x & 31) == 0) t = atomicAdd(queue, grab);
+    t = __shfl_sync(kFull, t, 0);
+    if (t >= end - first) break;
+    for (uint32_t i = first + t; i < min(end, first + t + grab); i++) body(tasks[i]);
+  }
+}
+
+// Adds a warp's edges of an item to its job's counter and to lane 0's total.
+__device__ __forceinline__ void count_item(const BatchJob &jb, uint64_t cnt, uint64_t &all) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(kFull, cnt, o);
+  if ((threadIdx.x & 31) == 0 && cnt) {
+    if (jb.edges) atomicAdd(jb.edges, (unsigned long long)cnt);
+    all += cnt;
+  }
+}
+
+// Multi-RW samples whose walkers move in parallel, a block each, in a kernel of
+// their own: they want more threads a sample (51 samples of 2000 walkers x
+// 10,000 events alone: 0.50 ms, with 8 warps 0.75), and their workspace would
+// come out of the other items' L1.
+constexpr int kBatchCtaWarps = 16;
+template <int MODE>
+__global__ void __launch_bounds__(32 * kBatchCtaWarps, 2)
+    batch_cta_kernel(DevGraph g, const BatchJob *__restrict__ jobs,
+                     const BatchTask *__restrict__ tasks, uint32_t ntasks, unsigned int *queue,
+                     unsigned long long *total, unsigned int *err) {
+  __shared__ CtaSmem<kBatchCtaWarps> csm;
   uint64_t all = 0;
   bool bad = false;
-  // Block-level items first: multi-RW samples whose walkers move in parallel.
-  while (ncta) {
-    if (threadIdx.x == 0) csm.task = atomicAdd(queue + 1, 1u);
+  for (;;) {
+    if (threadIdx.x == 0) csm.task = atomicAdd(queue, 1u);
     __syncthreads();
     const uint32_t c = csm.task;
     __syncthreads();
-    if (c >= ncta) break;
+    if (c >= ntasks) break;
     const BatchTask tk = tasks[c];
     const BatchJob &jb = jobs[tk.job];
     const uint64_t s = tk.begin;
@@ -60,62 +78,93 @@ __global__ void __launch_bounds__(256, GRASS_BATCH_MIN_BLOCKS) batch_kernel(DevG
         jb.roots[s * jb.walkers + w] = mrw_root(g.n, jb.seed, s * jb.walkers + w);
       __syncthreads();
     }
-    mrw_cta_sample<MODE, 8>(g, jb.roots + s * jb.walkers, jb.out0 + s * jb.steps,
-                            jb.out1 + s * jb.steps, jb.walkers, jb.steps, jb.select, jb.seed, s,
-                            jb.mscr + s * jb.mstride, csm, cnt, bad);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(kFull, cnt, o);
-    if (lane == 0 && cnt) {
-      if (jb.edges) atomicAdd(jb.edges, (unsigned long long)cnt);
-      all += cnt;
-    }
+    mrw_cta_sample<MODE, kBatchCtaWarps>(g, jb.roots + s * jb.walkers, jb.out0 + s * jb.steps,
+                                         jb.out1 + s * jb.steps, jb.walkers, jb.steps, jb.select,
+                                         jb.seed, s, jb.mscr + s * jb.mstride, csm, cnt, bad);
+    count_item(jb, cnt, all);
   }
-  for (;;) {
-    uint32_t t = 0;
-    if (lane == 0) t = ncta + atomicAdd(queue, 1u);
-    t = __shfl_sync(kFull, t, 0);
-    if (t >= ntasks) break;
-    const BatchTask tk = tasks[t];
+  if ((threadIdx.x & 31) == 0 && total && all) atomicAdd(total, (unsigned long long)all);
+  if (bad && err) atomicOr(err, 1u);
+}
+
+// One kind of item after the other, each with a counter of its own: a warp goes
+// on to the next kind when the last items of one are taken, so the kinds
+// overlap, and each kind's loop has the registers to itself.  (In one loop over
+// items of any kind, block-level ones too, the walks and k-hops spilled 200-360
+// bytes and had 38 KB less L1 an SM: the walks of the 256-job mix on R-MAT s22
+// ef32 took 0.675 ms alone and now 0.571, its k-hops 0.715 and 0.627, all of it
+// 1.61 and 1.25.)
+// The kinds come in the order of how long an item takes (a chain, 100 steps of
+// a tile of walkers, a seed), so that the last items are short.
+template <int MODE, int DEPTH>
+__global__ void __launch_bounds__(256, GRASS_BATCH_MIN_BLOCKS) batch_kernel(DevGraph g, const BatchJob *__restrict__ jobs,
+                                                    const BatchTask *__restrict__ tasks,
+                                                    BatchRanges R, uint32_t khop_grab,
+                                                    unsigned int *queue,
+                                                    unsigned long long *total,
+                                                    unsigned int *err) {
+  union WarpSmem {  // a warp runs one kind of item at a time
+    SmemHdr khop;
+    uint32_t stage[kPathStageWords<DEPTH>];
+  };
+  __shared__ __align__(16) unsigned char warp_smem[8 * sizeof(WarpSmem)];
+  WarpSmem &my = reinterpret_cast<WarpSmem *>(warp_smem)[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  uint64_t all = 0;
+  bool bad = false;
+  // sequential multi-RW samples
+  take_items(tasks, R.cta, R.mrw, 1, queue + 1, [&](const BatchTask &tk) {
     const BatchJob &jb = jobs[tk.job];
     uint64_t cnt = 0;
-    if (jb.type == GRASS_JOB_RW) {
-      uint32_t *stage = sh[threadIdx.x >> 5].stage;
-      for (uint64_t wb = tk.begin; wb < tk.end; wb += 32 * DEPTH) {
-        if (jb.layout == GRASS_LAYOUT_WALK_MAJOR)
-          rw_pass<MODE, DEPTH, true>(g, jb.in, jb.count, jb.length, jb.seed, 0, jb.out0, wb, 32,
-                                     tk.end, stage, cnt, bad);
-        else
-          rw_pass<MODE, DEPTH, false>(g, jb.in, jb.count, jb.length, jb.seed, 0, jb.out0, wb, 32,
-                                      tk.end, stage, cnt, bad);
+    for (uint64_t s = tk.begin; s < tk.end; s++) {
+      if (jb.gen_roots) {
+        for (uint32_t w = lane; w < jb.walkers; w += 32)
+          jb.roots[s * jb.walkers + w] = mrw_root(g.n, jb.seed, s * jb.walkers + w);
+        __syncwarp();
       }
-    } else if (jb.type == GRASS_JOB_KHOP) {
-      const uint32_t parts = max(1u, tk.pad >> 8), part = tk.pad & 0xFFu;
+      mrw_degree_warp<MODE>(g, jb.roots + s * jb.walkers,
+                            reinterpret_cast<uint4 *>(jb.mscr + s * jb.mstride), jb.walkers,
+                            jb.steps, jb.seed, s, jb.out0, jb.out1, cnt, bad);
+    }
+    count_item(jb, cnt, all);
+  });
+  // walker tiles
+  take_items(tasks, R.khop, R.rw, 1, queue + 3, [&](const BatchTask &tk) {
+    const BatchJob &jb = jobs[tk.job];
+    uint64_t cnt = 0;
+    for (uint64_t wb = tk.begin; wb < tk.end; wb += 32 * DEPTH) {
+      if (jb.layout == GRASS_LAYOUT_WALK_MAJOR)
+        rw_pass<MODE, DEPTH, true>(g, jb.in, jb.count, jb.length, jb.seed, 0, jb.out0, wb, 32,
+                                   tk.end, my.stage, cnt, bad);
+      else
+        rw_pass<MODE, DEPTH, false>(g, jb.in, jb.count, jb.length, jb.seed, 0, jb.out0, wb, 32,
+                                    tk.end, my.stage, cnt, bad);
+    }
+    count_item(jb, cnt, all);
+  });
+  // k-hop seeds (whole, or split over several warps)
+  if (R.parts == 1) {
+    take_items(tasks, R.mrw, R.khop, khop_grab, queue + 2, [&](const BatchTask &tk) {
+      const BatchJob &jb = jobs[tk.job];
+      uint64_t cnt = 0;
       for (uint64_t s = tk.begin; s < tk.end; s++)
-        khop_seed_warp<MODE>(g, jb.in, jb.khop, s, my, cnt, bad, part, parts);
-    } else {
-      for (uint64_t s = tk.begin; s < tk.end; s++) {
-        if (jb.gen_roots) {
-          for (uint32_t w = lane; w < jb.walkers; w += 32)
-            jb.roots[s * jb.walkers + w] = mrw_root(g.n, jb.seed, s * jb.walkers + w);
-          __syncwarp();
-        }
-        mrw_degree_warp<MODE>(g, jb.roots + s * jb.walkers,
-                              reinterpret_cast<uint4 *>(jb.mscr + s * jb.mstride), jb.walkers,
-                              jb.steps, jb.seed, s, jb.out0, jb.out1, cnt, bad);
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(kFull, cnt, o);
-    if (lane == 0 && cnt) {
-      if (jb.edges) atomicAdd(jb.edges, (unsigned long long)cnt);
-      all += cnt;
-    }
+        khop_seed_warp<MODE>(g, jb.in, jb.khop, s, my.khop, cnt, bad);
+      count_item(jb, cnt, all);
+    });
+  } else {
+    take_items(tasks, R.mrw, R.khop, khop_grab, queue + 2, [&](const BatchTask &tk) {
+      const BatchJob &jb = jobs[tk.job];
+      uint64_t cnt = 0;
+      for (uint64_t s = tk.begin; s < tk.end; s++)
+        khop_seed_warp<MODE>(g, jb.in, jb.khop, s, my.khop, cnt, bad, tk.pad & 0xFFu, R.parts);
+      count_item(jb, cnt, all);
+    });
   }
   if (lane == 0 && total && all) atomicAdd(total, (unsigned long long)all);
   if (bad && err) atomicOr(err, 1u);
 }
 
-using BatchKernel = void (*)(DevGraph, const BatchJob *, const BatchTask *, uint32_t, uint32_t,
+using BatchKernel = void (*)(DevGraph, const BatchJob *, const BatchTask *, BatchRanges, uint32_t,
                              unsigned int *, unsigned long long *, unsigned int *);
 
 BatchKernel pick_kernel(int mode, uint32_t depth) {
@@ -207,9 +256,28 @@ void split_job(const grass_job &j, uint32_t ji, const grass_batch_config &c,
 }
 
 int launch_batch(const DevGraph &dg, int device, const BatchJob *d_jobs, const BatchTask *d_tasks,
-                 uint32_t ncta, uint32_t ntasks, unsigned int *d_queue,
-                 unsigned long long *d_total, unsigned int *d_err, cudaStream_t s,
+                 const BatchRanges &ranges, unsigned int *d_queue, unsigned long long *d_total,
+                 unsigned int *d_err, cudaStream_t s, BatchSide &side,
                  const grass_batch_config &c) {
+  const bool warps = ranges.rw > ranges.cta;
+  if (ranges.cta) {
+    cudaStream_t cs = s;
+    if (warps) {
+      cudaError_t e = side.create();
+      if (e == cudaSuccess) e = cudaEventRecord(side.fork, s);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(side.st, side.fork, 0);
+      if (e != cudaSuccess) return cuda_fail(e, "batch side stream");
+      cs = side.st;
+    }
+    auto k = dg.mode == GRASS_MODE_CSR_INTERNAL ? batch_cta_kernel<kCsr> : batch_cta_kernel<kSlots>;
+    const unsigned grid = std::min<unsigned>(ranges.cta, (unsigned)sm_count(device) * 2);
+    k<<<grid, 32 * kBatchCtaWarps, 0, cs>>>(dg, d_jobs, d_tasks, ranges.cta, d_queue, d_total,
+                                             d_err);
+    cudaError_t e = cudaGetLastError();
+    if (warps && e == cudaSuccess) e = cudaEventRecord(side.join, cs);
+    if (e != cudaSuccess) return cuda_fail(e, "batch kernel launch");
+  }
+  if (!warps) return GRASS_OK;
   BatchKernel k = pick_kernel(dg.mode, c.depth);
   const int threads = 32 * (int)c.warps_per_block;
   // Resident blocks per SM, once per (kernel, block size): the query costs
@@ -228,13 +296,32 @@ int launch_batch(const DevGraph &dg, int device, const BatchJob *d_jobs, const B
     }
   }
   if (per_sm < 1) per_sm = 1;
-  const uint64_t need =
-      std::max<uint64_t>(ncta, (ntasks - ncta + c.warps_per_block - 1) / c.warps_per_block);
+  const uint64_t need = (ranges.rw - ranges.cta + c.warps_per_block - 1) / c.warps_per_block;
   const unsigned grid = (unsigned)std::max<uint64_t>(
       1, std::min<uint64_t>(need, (uint64_t)sm_count(device) * per_sm));
-  k<<<grid, threads, 0, s>>>(dg, d_jobs, d_tasks, ncta, ntasks, d_queue, d_total, d_err);
-  const cudaError_t e = cudaGetLastError();
+  // A seed takes some 10 us; one counter serves about one take a nanosecond.
+  const uint64_t takes = (uint64_t)grid * c.warps_per_block * 8;
+  const uint32_t grab =
+      (uint32_t)std::min<uint64_t>(8, std::max<uint64_t>(1, (ranges.khop - ranges.mrw) / takes));
+  k<<<grid, threads, 0, s>>>(dg, d_jobs, d_tasks, ranges, grab, d_queue, d_total, d_err);
+  cudaError_t e = cudaGetLastError();
+  if (ranges.cta && e == cudaSuccess) e = cudaStreamWaitEvent(s, side.join, 0);
   return e == cudaSuccess ? GRASS_OK : cuda_fail(e, "batch kernel launch");
+}
+
+cudaError_t BatchSide::create() {
+  if (join) return cudaSuccess;
+  cudaError_t e = st ? cudaSuccess : cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e == cudaSuccess && !fork) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
+  return e;
+}
+
+void BatchSide::destroy() {
+  if (st) cudaStreamDestroy(st);
+  if (fork) cudaEventDestroy(fork);
+  if (join) cudaEventDestroy(join);
+  *this = BatchSide();
 }
 
 }  // namespace grass
@@ -256,7 +343,8 @@ struct grass_batch {
   grass_batch_config built_cfg{};
   BatchJob *d_jobs = nullptr;
   BatchTask *d_tasks = nullptr;
-  uint32_t ntasks = 0, ncta = 0;
+  uint32_t ntasks = 0;
+  BatchRanges ranges{};
   unsigned int *d_queue = nullptr;
   std::vector<void *> owned;                      // MRW record scratch (per build)
   std::vector<uint32_t *> snap;                   // per job: MRW start vertices as added
@@ -264,6 +352,7 @@ struct grass_batch {
   std::vector<uint64_t> restore_n;
   // captured graph
   cudaStream_t cap = nullptr;
+  BatchSide side;
   cudaGraphExec_t exec = nullptr;
   unsigned long long *exec_total = nullptr;
 
@@ -280,7 +369,7 @@ struct grass_batch {
     owned.clear();
     restore.clear();
     restore_n.clear();
-    ntasks = ncta = 0;
+    ntasks = 0;
   }
   void free_snapshots() {
     for (uint32_t *p : snap) cudaFree(p);
@@ -290,6 +379,7 @@ struct grass_batch {
     free_device();
     free_snapshots();
     if (cap) cudaStreamDestroy(cap);
+    side.destroy();
   }
 };
 
@@ -320,10 +410,10 @@ int build(grass_batch *b) {
   tasks.insert(tasks.end(), rw.begin(), rw.end());
   if (tasks.size() > 0xFFFFFFF0ull) return set_error(GRASS_E_ARG, "batch: too many work items");
   b->ntasks = (uint32_t)tasks.size();
-  b->ncta = (uint32_t)cta.size();
+  b->ranges = batch_ranges(cta, mrw, khop, rw, c);
   GRASS_CUDA(cudaMalloc(&b->d_jobs, std::max<size_t>(hj.size(), 1) * sizeof(BatchJob)));
   GRASS_CUDA(cudaMalloc(&b->d_tasks, std::max<size_t>(tasks.size(), 1) * sizeof(BatchTask)));
-  GRASS_CUDA(cudaMalloc(&b->d_queue, 2 * sizeof(unsigned int)));
+  GRASS_CUDA(cudaMalloc(&b->d_queue, kQueueWords * sizeof(unsigned int)));
   if (!hj.empty())
     GRASS_CUDA(cudaMemcpy(b->d_jobs, hj.data(), hj.size() * sizeof(BatchJob),
                           cudaMemcpyHostToDevice));
@@ -341,10 +431,10 @@ int enqueue(grass_batch *b, cudaStream_t s, unsigned long long *total) {
   for (size_t i = 0; i < b->restore.size(); i++)
     GRASS_CUDA(cudaMemcpyAsync(b->restore[i].first, b->restore[i].second, b->restore_n[i] * 4,
                                cudaMemcpyDeviceToDevice, s));
-  GRASS_CUDA(cudaMemsetAsync(b->d_queue, 0, 2 * sizeof(unsigned int), s));
+  GRASS_CUDA(cudaMemsetAsync(b->d_queue, 0, kQueueWords * sizeof(unsigned int), s));
   if (!b->ntasks) return GRASS_OK;
-  return launch_batch(b->dg, b->device, b->d_jobs, b->d_tasks, b->ncta, b->ntasks, b->d_queue,
-                      total, b->d_err, s, c);
+  return launch_batch(b->dg, b->device, b->d_jobs, b->d_tasks, b->ranges, b->d_queue, total, b->d_err,
+                      s, b->side, c);
 }
 
 int check_job(const grass_job *j) {
@@ -487,6 +577,7 @@ int grass_batch_run(grass_batch *b, void *stream, unsigned long long *d_total_ed
     if (b->exec) cudaGraphExecDestroy(b->exec);
     b->exec = nullptr;
     if (!b->cap) GRASS_CUDA(cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking));
+    if (b->ranges.cta && b->ranges.rw > b->ranges.cta) GRASS_CUDA(b->side.create());
     GRASS_CUDA(cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal));
     const int rc = enqueue(b, b->cap, d_total_edges);
     cudaGraph_t graph = nullptr;

@@ -204,6 +204,7 @@ struct grass_server {
   grass_server_config cfg{};
   grass_batch_config bcfg{};
   cudaStream_t streams[grass::kMaxSlots] = {nullptr};
+  grass::BatchSide sides[grass::kMaxSlots];  // made when a batch needs it
   bool slot_busy[grass::kMaxSlots] = {false};
   grass::Arena staging, scratch;  // pinned host, device
   grass::PinnedPool pinned;
@@ -475,6 +476,7 @@ void grass_server::launch(Batch *b) {
   const uint64_t tasks_off = off;
   off += align_up(ntasks * sizeof(BatchTask));
   const uint64_t queue_off = off;
+  static_assert(kQueueWords * 4 <= kAlign, "queue");
   off += kAlign;
   for (size_t i = 0; i < nj; i++) {
     in_off[i] = off;
@@ -567,10 +569,10 @@ void grass_server::launch(Batch *b) {
     }
     if (!rc && ntasks)
       rc = launch_batch(g->view(), g->device, reinterpret_cast<const BatchJob *>(d + jobs_off),
-                        reinterpret_cast<const BatchTask *>(d + tasks_off), (uint32_t)cta.size(),
-                        (uint32_t)ntasks,
+                        reinterpret_cast<const BatchTask *>(d + tasks_off),
+                        batch_ranges(cta, mrw, khop, rw, bcfg),
                         reinterpret_cast<unsigned int *>(d + queue_off), nullptr,
-                        reinterpret_cast<unsigned int *>(d + err_off), s, bcfg);
+                        reinterpret_cast<unsigned int *>(d + err_off), s, sides[b->slot], bcfg);
     if (!rc && ntasks) count_launch();
     lap(3);
     if (!rc) {
@@ -593,6 +595,7 @@ void grass_server::launch(Batch *b) {
   if (rc) {
     // Nothing will call back: wait for what was queued, then fail the batch.
     cudaStreamSynchronize(s);
+    if (sides[b->slot].st) cudaStreamSynchronize(sides[b->slot].st);
     cudaGetLastError();
     finish(b, rc);
   }
@@ -916,6 +919,7 @@ int grass_server_destroy(grass_server *s, uint32_t timeout_ms) {
     if (s->streams[i]) {
       cudaStreamSynchronize(s->streams[i]);
       cudaStreamDestroy(s->streams[i]);
+      s->sides[i].destroy();
     }
   for (auto &kv : s->reqs) {
     Batch *b = kv.second->batch;
