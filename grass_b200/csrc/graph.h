@@ -21,7 +21,15 @@ struct HostPipe {
   uint32_t *d_paths[2] = {nullptr, nullptr};
   size_t cap_starts = 0, cap_paths = 0;  // elements per slot
   unsigned long long *d_edges = nullptr;
+  // Small calls: starts and results in one pinned buffer (the kernel reads the
+  // starts there), results on the device as [edge counter][paths]; the counter
+  // runs on from call to call (edges_seen: its value after the last one).
+  uint8_t *h_small = nullptr, *d_small = nullptr;
+  size_t cap_small = 0;
+  uint64_t edges_seen = 0;
   ~HostPipe() {
+    cudaFreeHost(h_small);
+    cudaFree(d_small);
     for (int i = 0; i < 2; i++) {
       cudaFree(d_starts[i]);
       cudaFree(d_paths[i]);
