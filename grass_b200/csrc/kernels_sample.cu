@@ -90,6 +90,33 @@ __device__ __forceinline__ uint32_t last_le(uint32_t lo, uint32_t hi, uint32_t x
   return lo;
 }
 
+// The same with P independent probes a round, for keys that lie side by side
+// in memory: with 3 for the fences and for a line's sectors the walk below took
+// 1.28 ms instead of 1.43; with 5, 7 and 15 for the fences 1.28, 1.29 and 1.46.
+template <int P, class Key>
+__device__ __forceinline__ uint32_t last_le_wide(uint32_t lo, uint32_t hi, uint32_t x, Key key) {
+  while (lo < hi) {
+    const uint32_t n = hi - lo;  // candidates above lo, cut into P + 1 parts
+    uint32_t nlo = lo, nhi = hi;
+    bool le[P];
+#pragma unroll
+    for (int i = 1; i <= P; i++) le[i - 1] = key(lo + (n * i + P) / (P + 1)) <= x;
+#pragma unroll
+    for (int i = 1; i <= P; i++) {
+      const uint32_t p = lo + (n * i + P) / (P + 1);
+      if (le[i - 1]) nlo = p;
+    }
+#pragma unroll
+    for (int i = P; i >= 1; i--) {
+      const uint32_t p = lo + (n * i + P) / (P + 1);
+      if (!le[i - 1]) nhi = p - 1;
+    }
+    lo = nlo;
+    hi = nhi;
+  }
+  return lo;
+}
+
 // Whether x is a neighbor of the vertex of header h.  Compressed: a search for
 // the one sector that can hold x, over the fences (see build_fences_kernel) for
 // its line and over the line's sectors' first heads, then for the slot and the
@@ -109,11 +136,11 @@ __device__ __forceinline__ bool has_neighbor(const DevGraph &g, const VHdr &h, u
     const uint32_t l0 = h.sec / 4, l1 = (h.sec + last) / 4;
     if (g.fences && l1 > l0) {
       // (fence l0 is the line's owner's, never read: the probes are above it)
-      const uint32_t l = last_le(l0, l1, y, [&](uint32_t k) { return ldw(g.fences + k); });
+      const uint32_t l = last_le_wide<3>(l0, l1, y, [&](uint32_t k) { return ldw(g.fences + k); });
       q = l > l0 ? l * 4 - h.sec : 0;
       last = min(last, l * 4 + 3 - h.sec);
     }
-    q = last_le(q, last, y, [&](uint32_t k) { return sector_head(g, h, k); });
+    q = last_le_wide<3>(q, last, y, [&](uint32_t k) { return sector_head(g, h, k); });
     const Sec A = load_sector(g.words, h.sec + q);
     const uint32_t c0 = q * h.K, n = min(h.K, slots - c0);
     auto head = [&](uint32_t c) { return sec_field(A, h.off + c * h.cb, h.a); };
@@ -147,8 +174,8 @@ __global__ void __launch_bounds__(256) build_fences_kernel(DevGraph g, uint32_t 
 // Resident 256-thread blocks per SM the node2vec kernels are compiled for: the
 // walk waits on dependent sector reads, so resident warps matter more than
 // registers until those spill.  262,144 walkers x 80, p = 1, q = 0.5, R-MAT s22
-// ef32: 1.45 ms at 4 blocks (53 registers), 1.56 at 5, 1.86 at 6.  The CSR
-// kernel needs no cap (42 registers).
+// ef32: 1.45 ms at 4 blocks, 1.56 at 5, 1.86 at 6 (now 1.28 at 4, 54
+// registers).  The CSR kernel needs no cap (42 registers).
 #ifndef GRASS_N2V_MIN_BLOCKS
 #define GRASS_N2V_MIN_BLOCKS 4
 #endif
@@ -159,9 +186,9 @@ __global__ void __launch_bounds__(256) build_fences_kernel(DevGraph g, uint32_t 
 // A lane goes its own way through tries, steps and walkers: a turn of the loop
 // is one candidate for every lane, a first try for most, and the lanes that
 // search do so together.  (With the tries of a step in a loop of their own, all
-// lanes waited for the last one's: 2.43 against 2.14 ms, and 1.45 with the
-// fences.  41 M of its reads miss L2; at the rate of random reads they take
-// 0.9.)
+// lanes waited for the last one's: 2.43 against 2.14 ms; 1.45 with the fences and
+// 1.28 with three probes a round.  41 M of its reads miss L2; at the rate of
+// random reads they take 0.9.)
 template <int MODE>
 __global__ void __launch_bounds__(256, MODE == kCsr ? GRASS_N2V_CSR_MIN_BLOCKS : GRASS_N2V_MIN_BLOCKS) n2v_kernel(DevGraph g, const uint32_t *__restrict__ starts,
                                                   uint64_t W, N2vArgs a,
