@@ -457,9 +457,11 @@ __device__ __forceinline__ void mrw_uniform_samples(const DevGraph &g, uint32_t 
 }
 
 // Resident 256-thread blocks per SM: every lane waits on dependent record and
-// sector reads, so resident warps pay.
+// sector reads, so resident warps pay (65,536 samples of 80 x 100 on R-MAT s22
+// ef32: 246 us at 4 blocks, 251 at 6, 212 at 8, 32 registers; the 7 M reads that miss L2
+// take 155 at the rate of random reads).
 #ifndef GRASS_MRW_MIN_BLOCKS
-#define GRASS_MRW_MIN_BLOCKS 6
+#define GRASS_MRW_MIN_BLOCKS 8
 #endif
 
 template <int MODE>

@@ -341,7 +341,7 @@ __device__ __forceinline__ uint32_t mrw_root(uint32_t n, uint64_t seed, uint64_t
 // takes step t0 + k, in as many rounds as one walker has steps among the 32
 // (2 or 3 with 80 walkers), where one step after the other left 31 lanes idle
 // through 32 chains of two memory reads (65,536 samples of 80 walkers x 100
-// steps, R-MAT s22 ef32: 0.25 ms against 1.70 ms).
+// steps, R-MAT s22 ef32: 0.21 ms against 1.70 ms).
 template <int MODE>
 __device__ __forceinline__ void mrw_uniform_warp(const DevGraph &g, uint32_t *vtx, uint32_t R,
                                                  uint32_t T, uint64_t seed, uint64_t sample,
