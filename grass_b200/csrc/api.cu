@@ -7,8 +7,10 @@
 #include <algorithm>
 #include <cmath>
 #include <chrono>
+#include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "graph.h"
@@ -80,6 +82,21 @@ int sm_count(int device) {
     cache[device] = v;
   }
   return cache[device];
+}
+
+int resident_blocks(const void *kern, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void *, int, size_t, int>, int> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(mu);
+  int &per_sm = known[{kern, threads, smem, dev}];
+  if (per_sm < 1) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess)
+      cudaGetLastError();
+    per_sm = std::max(per_sm, 1);
+  }
+  return per_sm;
 }
 
 namespace {

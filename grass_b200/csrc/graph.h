@@ -153,6 +153,10 @@ int cuda_fail(cudaError_t e, const char *what);
 
 // Streaming SM count of the current device (cached per device).
 int sm_count(int device);
+// Resident blocks per SM of a kernel on the current device, at least 1; asked of
+// the runtime once per kernel, block size, shared memory and device (the query
+// is microseconds of a small call's host time).
+int resident_blocks(const void *kern, int threads, size_t smem);
 // Stream-ordered scratch on the current device from the library's own pool
 // (freed memory stays mapped for reuse).
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s);

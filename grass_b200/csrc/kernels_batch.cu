@@ -10,7 +10,6 @@
 // it.  The queue reset, the restore of the multi-RW start vertices and the
 // kernels are captured once into a CUDA graph and replayed by every run.
 #include <algorithm>
-#include <map>
 #include <mutex>
 #include <vector>
 
@@ -280,22 +279,7 @@ int launch_batch(const DevGraph &dg, int device, const BatchJob *d_jobs, const B
   if (!warps) return GRASS_OK;
   BatchKernel k = pick_kernel(dg.mode, c.depth);
   const int threads = 32 * (int)c.warps_per_block;
-  // Resident blocks per SM, once per (kernel, block size): the query costs
-  // tens of microseconds and the serving loop launches thousands of batches.
-  static std::mutex occ_mu;
-  static std::map<std::pair<const void *, int>, int> occ;
-  int per_sm = 0;
-  {
-    std::lock_guard<std::mutex> lk(occ_mu);
-    auto it = occ.find({(const void *)k, threads});
-    if (it != occ.end()) {
-      per_sm = it->second;
-    } else {
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, 0);
-      occ[{(const void *)k, threads}] = per_sm;
-    }
-  }
-  if (per_sm < 1) per_sm = 1;
+  const int per_sm = resident_blocks((const void *)k, threads, 0);
   const uint64_t need = (ranges.rw - ranges.cta + c.warps_per_block - 1) / c.warps_per_block;
   const unsigned grid = (unsigned)std::max<uint64_t>(
       1, std::min<uint64_t>(need, (uint64_t)sm_count(device) * per_sm));

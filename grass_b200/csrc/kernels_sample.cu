@@ -664,9 +664,7 @@ grass_tuning resolve_tuning(const grass_tuning &t, int kind) {
 template <class K>
 static unsigned resident_grid(K kern, int threads, size_t smem, uint32_t want_per_sm,
                               uint64_t units, uint64_t units_per_block) {
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
-  if (per_sm < 1) per_sm = 1;
+  int per_sm = resident_blocks((const void *)kern, threads, smem);
   if (want_per_sm && (int)want_per_sm < per_sm) per_sm = (int)want_per_sm;
   const uint64_t need = (units + units_per_block - 1) / units_per_block;
   const uint64_t cap = (uint64_t)sm_count(cur_dev()) * per_sm;
@@ -868,11 +866,8 @@ int launch_mrw(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots, ui
                                               std::max<uint64_t>(128, (want + 31) / 32 * 32));
   auto cta = wide ? mrw_cta_kernel<kSlots, 32> : mrw_cta_kernel<kSlots, 16>;
   uint64_t resident = 0;
-  if (ct || (p.select == GRASS_SELECT_UNIFORM && p.steps >= 512)) {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cta, threads, 0);
-    resident = (uint64_t)sm_count(cur_dev()) * std::max(per_sm, 1);
-  }
+  if (ct || (p.select == GRASS_SELECT_UNIFORM && p.steps >= 512))
+    resident = (uint64_t)sm_count(cur_dev()) * resident_blocks((const void *)cta, threads, 0);
   if (ct || S <= resident + resident * p.steps / 2048) {
     const uint64_t grid = std::min<uint64_t>(S, resident);
     const uint64_t stride = mrw_sample_scratch(p.walkers, p.steps, p.select);
