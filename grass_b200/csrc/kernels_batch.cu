@@ -404,6 +404,8 @@ int build(grass_batch *b) {
   if (!tasks.empty())
     GRASS_CUDA(cudaMemcpy(b->d_tasks, tasks.data(), tasks.size() * sizeof(BatchTask),
                           cudaMemcpyHostToDevice));
+  // (now, not in launch_batch: a later run may be under capture)
+  if (b->ranges.cta && b->ranges.rw > b->ranges.cta) GRASS_CUDA(b->side.create());
   b->built_cfg = c;
   b->dirty = false;
   return GRASS_OK;
@@ -561,7 +563,6 @@ int grass_batch_run(grass_batch *b, void *stream, unsigned long long *d_total_ed
     if (b->exec) cudaGraphExecDestroy(b->exec);
     b->exec = nullptr;
     if (!b->cap) GRASS_CUDA(cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking));
-    if (b->ranges.cta && b->ranges.rw > b->ranges.cta) GRASS_CUDA(b->side.create());
     GRASS_CUDA(cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal));
     const int rc = enqueue(b, b->cap, d_total_edges);
     cudaGraph_t graph = nullptr;
