@@ -665,6 +665,14 @@ static int node2vec_args(const grass_node2vec_params *p, grass_node2vec_params &
   return GRASS_OK;
 }
 
+// While it lives, this thread may allocate although another stream is being
+// captured (by this or another thread, in global mode).
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // The graph's fences, or null: while the stream is being captured (nothing can
 // be allocated or waited for) or without memory the search goes without them,
 // with the same results.
@@ -677,6 +685,7 @@ static const uint32_t *graph_fences(const grass_graph *g, cudaStream_t st) {
     return nullptr;
   }
   g->fences_tried = true;
+  RelaxedCapture relaxed;
   uint32_t *f = nullptr;
   if (cudaMalloc(&f, fence_words(g->n_words) * 4) != cudaSuccess) {
     cudaGetLastError();
@@ -743,6 +752,7 @@ int rw_host_small(const grass_graph *g, const grass_rw_params &p, const uint32_t
   const size_t in = (W * 4 + 15) & ~15ull, paths = W * ((uint64_t)p.length + 1) * 4;
   const size_t out = 16 + paths;  // the counter, then the paths
   if (hp.cap_small < in + out + 16) {
+    RelaxedCapture relaxed;
     cudaFreeHost(hp.h_small);
     cudaFree(hp.d_small);
     hp.h_small = hp.d_small = nullptr;

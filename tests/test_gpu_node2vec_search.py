@@ -46,3 +46,27 @@ def test_search_with_and_without_fences(oracle_mod, tmp_path, mode, spread):
         torch.cuda.synchronize()
         np.testing.assert_array_equal(paths.cpu().numpy().view(np.uint32), ref)
         assert int(count) == total
+
+
+def test_first_call_beside_a_capture(oracle_mod, tmp_path):
+    """The first call builds the fences; another stream's capture goes on."""
+    import torch
+    n, d = 400, 150
+    rows = [np.sort(np.random.default_rng(v).choice(n, d, replace=False)).astype(np.uint32) for v in range(n)]
+    rp = (np.arange(n + 1) * d).astype(np.uint64)
+    G.compress_to_files(rp, np.concatenate(rows), "LE", str(tmp_path / "g"))
+    g, og = G.Graph(str(tmp_path / "g"), "LE"), oracle_mod.OracleGraph(str(tmp_path / "g"))
+    W, L = 500, 10
+    starts = np.arange(W, dtype=np.uint32) % n
+    ref, _ = og.node2vec("LE", starts, L, 5, 1.0, 0.5)
+    dev = torch.from_numpy(starts.view(np.int32)).cuda()
+    captured, beside = (torch.zeros(W, L + 1, dtype=torch.int32, device="cuda") for _ in range(2))
+    graph, stream, other = torch.cuda.CUDAGraph(), torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        g.node2vec_device(dev, W, L, 5, 1.0, 0.5, captured, stream=stream)
+        g.node2vec_device(dev, W, L, 5, 1.0, 0.5, beside, stream=other)
+    graph.replay()
+    torch.cuda.synchronize()
+    for paths in (captured, beside):
+        np.testing.assert_array_equal(paths.cpu().numpy().view(np.uint32), ref)
