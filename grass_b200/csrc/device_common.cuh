@@ -465,47 +465,6 @@ __device__ __forceinline__ uint32_t draw_value(const Sec &A, const DrawAt &at, c
          sec_field(A, at.off + h.a + (at.id - 1u) * h.b, at.id ? h.b : 0u);
 }
 
-// ---- slot decoder on 32-bit words (shared or global memory) ----
-// w points at the slot's sector as stream words, with three more readable
-// words after it; off is the bit offset of the slot in it.
-// Fields of up to 32 bits read in order from words: a two-word window, one
-// funnel shift per field, the next word loaded one ahead.  Reads up to three
-// words past the last field's word.
-struct WordStream {
-  const uint32_t *w;
-  uint32_t q, pos, lo, hi, nx;
-  __device__ __forceinline__ void init(const uint32_t *words, uint32_t at) {
-    w = words;
-    q = at >> 5;
-    pos = at & 31u;
-    lo = w[q];
-    hi = w[q + 1];
-    nx = w[q + 2];
-  }
-  __device__ __forceinline__ uint32_t get(uint32_t width) {  // width 0..32
-    const uint32_t x = __funnelshift_l(hi, lo, pos);
-    pos += width;
-    if (pos >= 32) {
-      pos -= 32;
-      lo = hi;
-      hi = nx;
-      nx = w[q + 3];
-      q++;
-    }
-    return shr_clamp(x, 32u - width);
-  }
-};
-
-// Neighbors 0..L-1 of a slot into o.
-__device__ __forceinline__ void slot_decode_w(const uint32_t *w, uint32_t off, const VHdr &h,
-                                              uint32_t L, uint32_t *o) {
-  WordStream S;
-  S.init(w, off);
-  const uint32_t x = h.base + S.get(h.a);
-  o[0] = x;
-  for (uint32_t t = 1; t < L; t++) o[t] = x + S.get(h.b);
-}
-
 // [rowptr[v], rowptr[v+1]) of a CSR with one 32-byte load (two when the pair
 // straddles a sector, v % 4 == 3).  rowptr must be allocated in whole
 // sectors with one spare sector (see grass_csr allocation).

@@ -280,20 +280,102 @@ __global__ void plan_fill_kernel(const uint4 *__restrict__ recs, uint32_t n, uin
   }
 }
 
-// ---- slot staging for the range sweep ----
-// Lane 0 of a warp copies the sectors that hold each group of 32 chunk slots
-// into one of the warp's D shared-memory buffers with one bulk copy
-// (cp.async.bulk, completion counted on that buffer's mbarrier), D - 1 groups
-// ahead of the group being decoded (D = 1: copy, then decode), and the lanes
-// read their fields from shared memory, one funnel shift per field.  Every
-// wait is bounded: a copy that has not landed after kStagePolls polls is
-// reported (error word bit 2, GRASS_E_TIMEOUT) and the warp reads global
-// memory from then on, waiting once more, bounded, for its copies in flight
-// before it exits.
+// ---- whole sectors from shared memory, a neighbor per lane ----
+// Where the bits of one neighbor are: the shared-memory addresses of the words
+// of its slot's head and of its offset, the bits in those words, and 32 less
+// the offset's width (a slot's first neighbor has none).
+struct Place {
+  uint32_t head, head_bit, off, off_bit, drop;
+};
+__device__ __forceinline__ Place place_of(const VHdr &h, uint32_t r, uint32_t stage) {
+  const uint32_t c = div_small(r, h.T), id = r - c * h.T;  // neighbor r of a sector
+  const uint32_t hb = h.off + c * h.cb, ob = id ? hb + h.a + (id - 1) * h.b : hb;
+  return Place{stage + (hb >> 5) * 4, hb, stage + (ob >> 5) * 4, ob, id ? 32 - h.b : 32u};
+}
+__device__ __forceinline__ uint32_t lds_bits(uint32_t addr, uint32_t bit, uint32_t drop) {
+  uint32_t hi, lo;
+  asm volatile("ld.shared.u32 %0, [%2];\n\tld.shared.u32 %1, [%2+4];" : "=r"(hi), "=r"(lo) : "r"(addr));
+  return shr_clamp(__funnelshift_l(lo, hi, bit), drop);
+}
+
+// The decoding of a vertex's staged sectors by a warp, R = 64 / N whole sectors
+// (N = T K neighbors each) a round, two neighbors a lane: the lane's places in
+// the R sectors stay the same from round to round, and a neighbor costs its
+// field reads, one add and the store.
+struct SectorLanes {
+  uint32_t N, R, chunk;  // chunk: sectors staged at a time, rounds of R
+  Place pl[2];           // the lane's places in a round, in shared memory from address 0
+  uint32_t j[2];         // its neighbors there (from i0): a lane without one
+                         // (R N < 64) reads place 0 and is never inside [0, len)
+  uint32_t *o;           // the lane's first neighbor of the round in the output
+
+  __device__ __forceinline__ void size(const VHdr &h) {
+    N = h.T * h.K;
+    R = N < 64 ? div_small(64u, N) : 1u;
+    chunk = div_small(32u, R) * R;
+  }
+  // (q0: the first sector, which holds neighbor i0; after size())
+  __device__ __forceinline__ void start(const VHdr &h, uint32_t q0, uint32_t i0, uint32_t *out) {
+    const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const uint32_t p = u * 32 + lane, k = N < 64 ? div_small(p, N) : 0u;
+      const bool ok = k < R;
+      pl[u] = place_of(h, ok ? p - k * N : 0u, ok ? k * 32 : 0u);
+      j[u] = ok ? q0 * N + p - i0 : 1u << 31;
+    }
+    o = out + (q0 * N + lane);
+  }
+  // Sectors q .. q + end - 1 of the vertex, staged at shared address st; its
+  // neighbors i0 .. i0 + len - 1 go to out.
+  __device__ __forceinline__ void decode(const VHdr &h, uint32_t st, uint32_t q, uint32_t end,
+                                         uint32_t i0, uint32_t len, uint32_t *out,
+                                         uint32_t &vmax) {
+    uint32_t at = st;  // address of the round's first sector
+    for (uint32_t e = 0; e < end; e += R) {
+      uint32_t v[2];
+#pragma unroll
+      for (int u = 0; u < 2; u++) v[u] = h.base + lds_bits(pl[u].head + at, pl[u].head_bit, 32 - h.a);
+      if (h.T > 1) {  // (warp-uniform)
+#pragma unroll
+        for (int u = 0; u < 2; u++) v[u] += lds_bits(pl[u].off + at, pl[u].off_bit, pl[u].drop);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        if (j[u] < len) {
+          o[u * 32] = v[u];
+          vmax = max(vmax, v[u]);
+        }
+        j[u] += R * N;
+      }
+      if (N > 64) {  // the rest of a sector of more than 64 neighbors
+        for (uint32_t r = 64 + (threadIdx.x & 31); r < N; r += 32) {
+          const uint32_t i = (q + e) * N + r;
+          const Place p = place_of(h, r, at);
+          const uint32_t w = h.base + lds_bits(p.head, p.head_bit, 32 - h.a) + lds_bits(p.off, p.off_bit, p.drop);
+          if (i - i0 < len) {
+            out[i] = w;
+            vmax = max(vmax, w);
+          }
+        }
+      }
+      o += R * N;
+      at += R * 32;
+    }
+  }
+};
+
+// ---- sector staging for the range sweep ----
+// Lane 0 of a warp copies each group of up to 32 sectors into one of the warp's
+// D shared-memory buffers with one bulk copy (cp.async.bulk, completion counted
+// on that buffer's mbarrier), D - 1 groups ahead of the group being decoded (D =
+// 1: copy, then decode).  Every wait is bounded: a copy that has not landed
+// after kStagePolls polls is reported (error word bit 2, GRASS_E_TIMEOUT) and
+// the warp loads the sectors itself from then on, waiting once more, bounded,
+// for its copies in flight before it exits.
 constexpr int kDecodeWarps = 8;          // warps per range block
-constexpr uint32_t kGroupBytes = 1056;   // 32 slots lie in at most 32 sectors; + one
-                                         // sector that field reads may touch
-constexpr uint32_t kOutWords = 32 * 32;  // a group's neighbors (32 slots of <= 32)
+constexpr uint32_t kGroupBytes = 1088;   // 32 sectors, and two that the reads of
+                                         // lanes without a neighbor may touch
 // Polls of the copy's mbarrier before the warp gives up (far beyond the
 // microseconds one copy takes).
 #ifndef GRASS_STAGE_POLLS
@@ -359,29 +441,26 @@ struct RangeMeta {
 
 // Shared memory of one range warp, in a block of its own that starts on a
 // 128-byte boundary: DEPTH staging buffers (each a multiple of 16 bytes, as
-// cp.async.bulk requires of its destination), the group's decoded neighbors,
-// the item metadata, then the buffers' mbarriers (8-byte aligned).
-template <int DEPTH>  // DEPTH 0: no staging buffers, no barriers
+// cp.async.bulk requires of its destination) and one for the loads after a
+// timeout, the item metadata, then the buffers' mbarriers (8-byte aligned).
+template <int DEPTH>
 struct WarpSmem {
-  static constexpr uint32_t stage_off() { return 0; }
-  static constexpr uint32_t out_off() { return DEPTH * kGroupBytes; }
-  static constexpr uint32_t meta_off() { return out_off() + kOutWords * 4; }
+  static constexpr uint32_t meta_off() { return (DEPTH + 1) * kGroupBytes; }
   static constexpr uint32_t bar_off() { return meta_off() + (uint32_t)sizeof(RangeMeta); }
   static constexpr uint32_t bytes() { return (bar_off() + DEPTH * 8 + 127) / 128 * 128; }
 };
-static_assert(kGroupBytes % 16 == 0 && (kOutWords * 4) % 16 == 0 && sizeof(RangeMeta) % 16 == 0,
+static_assert(kGroupBytes % 16 == 0 && sizeof(RangeMeta) % 16 == 0,
               "staging alignment");
 
-// Range sweep: one lane per chunk slot.  A
-// warp takes 32 range items at a time: lane k loads item k's record and row
-// start, and a scan over the lanes numbers the items' groups of 32 slots
-// 0 .. total-1 in item order.  The warp then walks that sequence: each lane
-// decodes its chunk's neighbors into shared memory, and the warp writes the
-// group's neighbors to the CSR with coalesced stores.  DEPTH 0 (the default)
-// reads the slot words from global memory through L1; DEPTH 1, 2 or 4 stages
-// each group's sectors in shared memory DEPTH - 1 groups ahead (across item
-// boundaries, see above).  Measured on R-MAT s22 ef32, the unstaged sweep is
-// the fastest: 7 % (LE) and 23 % (GT) faster than staging at depth 1.
+// Range sweep: a warp takes 32 range items at a time: lane k loads item k's
+// record and row start, and a scan over the lanes numbers the items' groups of
+// up to 32 sectors 0 .. total-1 in item order.  The warp then walks that
+// sequence, a neighbor per lane, straight to the CSR.  Each group's sectors are
+// staged in shared memory DEPTH - 1 groups ahead (1, 2 or 4; across item
+// boundaries, see above).  A lane per slot, its neighbors brought into order
+// through shared memory, took 1.54 ms at depth 1 on R-MAT s22 ef32 (250 M
+// neighbors; slots hold 3 neighbors there); this takes 0.90 ms, and 0.77 at
+// depths 2 and 4 (the flat sweep: 0.52).
 template <int DEPTH>
 __global__ void __launch_bounds__(256) decode_range_kernel(DevGraph g, const uint64_t *rowptr,
                                                            uint32_t *cols,
@@ -395,32 +474,35 @@ __global__ void __launch_bounds__(256) decode_range_kernel(DevGraph g, const uin
   static_assert(WS::bytes() % 128 == 0 && WS::bar_off() % 8 == 0 && WS::meta_off() % 16 == 0,
                 "warp block alignment");
   unsigned char *mine = le_smem + (threadIdx.x >> 5) * WS::bytes();
-  unsigned char *stage = mine + WS::stage_off();
-  uint32_t *out = reinterpret_cast<uint32_t *>(mine + WS::out_off());
   RangeMeta &m = *reinterpret_cast<RangeMeta *>(mine + WS::meta_off());
   uint64_t *bars = reinterpret_cast<uint64_t *>(mine + WS::bar_off());
+  const uint32_t st = smem_u32(mine);
   uint32_t phase = 0;    // bit b: parity of buffer b's next completion
   uint32_t pending = 0;  // bit b: buffer b has a copy issued and not yet waited for
-  constexpr uint32_t D = DEPTH > 0 ? DEPTH : 1;  // ring size (DEPTH 0: unstaged)
-  bool stage_ok = DEPTH > 0;
+  bool stage_ok = true;
   if (lane < DEPTH) stage_bar_init(bars + lane);
   __syncwarp();
-  bool bad = false;
+  uint32_t vmax = 0;
   for (uint64_t tb = warp * 32; tb < nitems; tb += nwarps * 32) {
-    // lane k: item tb + k, its slots [c0, c1] and their group count
+    // lane k: item tb + k, its sectors qs .. qs + qn - 1 of the layout, in
+    // groups of gs
     const uint64_t t = tb + lane;
-    uint32_t c0 = 0, c1 = 0, ng = 0;
+    uint32_t qs = 0, qn = 0, gs = 1, ng = 0;
     if (t < nitems) {
       const uint4 it = items[t];
       const uint4 r = load_record(g.recs + it.x);
       const VHdr h = record_header<kSlots>(r);
+      const uint32_t q = div_small(div_small(it.y, h.T), h.K);
       m.rec[lane] = r;
       m.base[lane] = rowptr[it.x];
       m.i0[lane] = it.y;
       m.i1[lane] = it.z;
-      c0 = div_small(it.y, h.T);
-      c1 = div_small(it.z - 1, h.T);
-      ng = (c1 - c0) / 32 + 1;
+      SectorLanes sl;
+      sl.size(h);
+      gs = sl.chunk;
+      qs = h.sec + q;
+      qn = div_small(div_small(it.z - 1, h.T), h.K) - q + 1;
+      ng = div_small(qn - 1, gs) + 1;
     }
     uint32_t incl = ng;
 #pragma unroll
@@ -435,88 +517,73 @@ __global__ void __launch_bounds__(256) decode_range_kernel(DevGraph g, const uin
     auto item_of = [&](uint32_t s) -> int {
       return __popc(__ballot_sync(FULL, ng > 0 && excl <= s)) - 1;
     };
-    // sectors [qa, qb] of group s
-    auto group_sectors = [&](uint32_t s, uint64_t &qa, uint64_t &qb) {
+    // the layout's sectors [qa, qa + n) of group s
+    auto group_sectors = [&](uint32_t s, uint32_t &qa, uint32_t &n) {
       const int k = item_of(s);
-      const uint32_t j = s - __shfl_sync(FULL, excl, k);
-      const uint32_t kc0 = __shfl_sync(FULL, c0, k), kc1 = __shfl_sync(FULL, c1, k);
-      const VHdr hk = record_header<kSlots>(m.rec[k]);
-      const uint32_t ca = kc0 + 32 * j, cz = min(kc1, ca + 31);
-      qa = slot_at(hk, ca).sec;
-      qb = slot_at(hk, cz).sec;
+      const uint32_t kgs = __shfl_sync(FULL, gs, k);
+      const uint32_t at = (s - __shfl_sync(FULL, excl, k)) * kgs;
+      qa = __shfl_sync(FULL, qs, k) + at;
+      n = min(kgs, __shfl_sync(FULL, qn, k) - at);
     };
     auto issue = [&](uint32_t s) {
-      if (DEPTH == 0 || !stage_ok) return;
-      const uint32_t b = s % D;
-      uint64_t qa, qb;
-      group_sectors(s, qa, qb);
+      if (!stage_ok) return;
+      const uint32_t b = s % DEPTH;
+      uint32_t qa, n;
+      group_sectors(s, qa, n);
       if (lane == 0)
-        stage_copy(stage + b * kGroupBytes, g.words + qa * 8, (uint32_t)(qb - qa + 1) * 32u,
-                   bars + b);
+        stage_copy(mine + b * kGroupBytes, g.words + (uint64_t)qa * 8, n * 32u, bars + b);
       pending |= 1u << b;
     };
     if constexpr (DEPTH > 1)
       for (uint32_t s = 0; s + 1 < (uint32_t)DEPTH && s < total; s++) issue(s);
     int kcur = -1;
     VHdr h;
-    uint64_t base = 0;
-    uint32_t i0 = 0, i1 = 0, kc0 = 0, kc1 = 0, kex = 0;
+    SectorLanes sl;
+    uint32_t *out = nullptr;
+    uint32_t i0 = 0, len = 0, q = 0, left = 0;  // the next sector of the vertex, the sectors left
     for (uint32_t s = 0; s < total; s++) {  // warp-uniform
-      if (DEPTH > 0 && s + DEPTH - 1 < total) issue(s + DEPTH - 1);
+      if (s + DEPTH - 1 < total) issue(s + DEPTH - 1);
       const int k = item_of(s);
       if (k != kcur) {  // the next item: its header and range from the metadata
         kcur = k;
         h = record_header<kSlots>(m.rec[k]);
-        base = m.base[k];
         i0 = m.i0[k];
-        i1 = m.i1[k];
-        kc0 = __shfl_sync(FULL, c0, k);
-        kc1 = __shfl_sync(FULL, c1, k);
-        kex = __shfl_sync(FULL, excl, k);
+        len = m.i1[k] - i0;
+        out = cols + m.base[k];
+        q = __shfl_sync(FULL, qs, k) - h.sec;
+        left = __shfl_sync(FULL, qn, k);
+        sl.size(h);
+        sl.start(h, q, i0, out);
       }
-      const uint32_t T = h.T, j = s - kex;
-      bool staged = false;
-      const uint32_t b = s % D;
-      if (DEPTH > 0 && stage_ok) {
+      uint32_t b = s % DEPTH;
+      if (stage_ok) {
         if (__all_sync(FULL, stage_wait(bars + b, (phase >> b) & 1u))) {
           phase ^= 1u << b;
           pending &= ~(1u << b);
-          staged = true;
         } else {  // the copy did not land in time: report, go on from global memory
           if (lane == 0 && err) atomicOr(err, 2u);
           stage_ok = false;
         }
       }
-      const uint32_t cg = kc0 + 32 * j, c = cg + lane;
-      if (c <= kc1) {
-        const DrawAt at = slot_at(h, c);
-        // the slot's sector as words: from the staged group, or (after a
-        // timeout) from global memory
-        const uint32_t *w;
-        if (staged) {
-          const uint32_t qa = slot_at(h, cg).sec;
-          w = reinterpret_cast<const uint32_t *>(stage + b * kGroupBytes + (at.sec - qa) * 32u);
-        } else {
-          w = g.words + (uint64_t)at.sec * 8;
-        }
-        slot_decode_w(w, at.off, h, min(T, h.d - c * T), out + (c - cg) * T);
+      const uint32_t n = min(sl.chunk, left);
+      if (!stage_ok) {  // into the buffer that no copy writes
+        b = DEPTH;
+        uint4 *dst = reinterpret_cast<uint4 *>(mine + DEPTH * kGroupBytes);
+        const uint4 *src = reinterpret_cast<const uint4 *>(g.words + (uint64_t)(h.sec + q) * 8);
+        for (uint32_t w = lane; w < 2 * n; w += 32) dst[w] = __ldg(src + w);
+        __syncwarp();
       }
-      __syncwarp();
-      const uint32_t nb0 = cg * T, nhi = min(h.d, (cg + 32) * T);
-      const uint32_t lo = max(i0, nb0), hi = min(i1, nhi);
-      for (uint32_t q = lo + lane; q < hi; q += 32) {
-        const uint32_t val = out[q - nb0];
-        bad |= val >= g.n;
-        cols[base + q] = val;
-      }
-      __syncwarp();  // the group's buffers are free for the next group
+      sl.decode(h, st + b * kGroupBytes, q, n, i0, len, out, vmax);
+      q += n;
+      left -= n;
+      __syncwarp();  // the group's buffer is free for the next group
     }
     __syncwarp();  // the metadata is free for the next batch
   }
   // copies still in flight after a timeout: one more bounded wait each
   for (int b = 0; b < DEPTH; b++)
     if ((pending >> b) & 1u) stage_wait(bars + b, (phase >> b) & 1u);
-  if (bad && err) atomicOr(err, 1u);
+  if (vmax >= g.n && err) atomicOr(err, 1u);
 }
 
 // ---- the flat sweep (the default) ----
@@ -587,98 +654,35 @@ __device__ __forceinline__ uint32_t word_field(const uint32_t *w, uint32_t off, 
   return shr_clamp(__funnelshift_l(q[1], q[0], off), 32u - width);
 }
 
-// Where the bits of one neighbor are: the shared-memory addresses of the words
-// of its slot's head and of its offset, the bits in those words, and 32 less
-// the offset's width (a slot's first neighbor has none).
-struct Place {
-  uint32_t head, head_bit, off, off_bit, drop;
-};
-__device__ __forceinline__ Place place_of(const VHdr &h, uint32_t r, uint32_t stage) {
-  const uint32_t c = div_small(r, h.T), id = r - c * h.T;  // neighbor r of a sector
-  const uint32_t hb = h.off + c * h.cb, ob = id ? hb + h.a + (id - 1) * h.b : hb;
-  return Place{stage + (hb >> 5) * 4, hb, stage + (ob >> 5) * 4, ob, id ? 32 - h.b : 32u};
-}
-__device__ __forceinline__ uint32_t lds_bits(uint32_t addr, uint32_t bit, uint32_t drop) {
-  uint32_t hi, lo;
-  asm volatile("ld.shared.u32 %0, [%2];\n\tld.shared.u32 %1, [%2+4];" : "=r"(hi), "=r"(lo) : "r"(addr));
-  return shr_clamp(__funnelshift_l(lo, hi, bit), drop);
-}
-
 // Neighbors [i0, i1) of a vertex of header h (warp-uniform, cb > 0) to
-// out[i0 .. i1); vmax: the largest value written so far.  A sector holds N = T
-// K neighbors, and the vertex's sectors are consecutive.  The warp copies up to
-// 32 of them at a time into shared memory with two 16-byte loads a lane, the
-// next ones already on their way in registers, and decodes R = 64 / N whole
-// sectors per round, two neighbors a lane: so a lane's places in the R sectors
-// stay the same from round to round, and a neighbor costs its field reads, one
-// add and the store.
+// out[i0 .. i1); vmax: the largest value written so far.  The vertex's sectors
+// are consecutive: the warp copies up to 32 of them at a time into shared
+// memory with two 16-byte loads a lane, the next ones already on their way in
+// registers.
 __device__ __forceinline__ void flat_big(const uint32_t *words, const VHdr &h, uint32_t i0,
                                          uint32_t i1, uint32_t *out, uint32_t *stage,
                                          uint32_t &vmax) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t N = h.T * h.K;
   const uint32_t q0 = i0 ? div_small(div_small(i0, h.T), h.K) : 0u;
   const uint32_t nq = div_small(div_small(i1 - 1, h.T), h.K) - q0 + 1;
-  const uint32_t R = N < 64 ? div_small(64u, N) : 1u;
-  const uint32_t chunk = div_small(32u, R) * R;  // sectors staged at a time
   const uint32_t len = i1 - i0, st = smem_u32(stage);
-  // the lane's places in a round, and its neighbors there (from i0): a lane
-  // without one (R N < 64) reads place 0 and is never inside [0, len)
-  Place pl[2];
-  uint32_t j[2];
-#pragma unroll
-  for (int u = 0; u < 2; u++) {
-    const uint32_t p = u * 32 + lane, k = N < 64 ? div_small(p, N) : 0u;
-    const bool ok = k < R;
-    pl[u] = place_of(h, ok ? p - k * N : 0u, st + (ok ? k * 32 : 0u));
-    j[u] = ok ? q0 * N + p - i0 : 1u << 31;
-  }
+  SectorLanes sl;
+  sl.size(h);
+  sl.start(h, q0, i0, out);
   const uint4 *src = reinterpret_cast<const uint4 *>(words + (uint64_t)(h.sec + q0) * 8) + lane;
   uint4 *dst = reinterpret_cast<uint4 *>(stage) + lane;
   const uint32_t half = lane >> 1;  // the lane's sector of 16
   uint4 x = make_uint4(0, 0, 0, 0), y = x;
   if (half < nq) x = __ldg(src);
   if (half + 16 < nq) y = __ldg(src + 32);
-  uint32_t *o = out + (q0 * N + lane);
-  for (uint32_t q = 0; q < nq; q += chunk) {  // warp-uniform
+  for (uint32_t q = 0; q < nq; q += sl.chunk) {  // warp-uniform
     dst[0] = x;
     dst[32] = y;
     __syncwarp();
-    src += 2 * chunk;
-    if (q + chunk + half < nq) x = __ldg(src);
-    if (q + chunk + half + 16 < nq) y = __ldg(src + 32);
-    const uint32_t end = min(chunk, nq - q);
-    uint32_t at = 0;  // byte offset of the round's first sector
-    for (uint32_t e = 0; e < end; e += R) {
-      uint32_t v[2];
-#pragma unroll
-      for (int u = 0; u < 2; u++) v[u] = h.base + lds_bits(pl[u].head + at, pl[u].head_bit, 32 - h.a);
-      if (h.T > 1) {  // (warp-uniform)
-#pragma unroll
-        for (int u = 0; u < 2; u++) v[u] += lds_bits(pl[u].off + at, pl[u].off_bit, pl[u].drop);
-      }
-#pragma unroll
-      for (int u = 0; u < 2; u++) {
-        if (j[u] < len) {
-          o[u * 32] = v[u];
-          vmax = max(vmax, v[u]);
-        }
-        j[u] += R * N;
-      }
-      if (N > 64) {  // the rest of a sector of more than 64 neighbors
-        for (uint32_t r = 64 + lane; r < N; r += 32) {
-          const uint32_t i = (q0 + q + e) * N + r;
-          const Place p = place_of(h, r, st + at);
-          const uint32_t w = h.base + lds_bits(p.head, p.head_bit, 32 - h.a) + lds_bits(p.off, p.off_bit, p.drop);
-          if (i - i0 < len) {
-            out[i] = w;
-            vmax = max(vmax, w);
-          }
-        }
-      }
-      o += R * N;
-      at += R * 32;
-    }
+    src += 2 * sl.chunk;
+    if (q + sl.chunk + half < nq) x = __ldg(src);
+    if (q + sl.chunk + half + 16 < nq) y = __ldg(src + 32);
+    sl.decode(h, st, q0 + q, min(sl.chunk, nq - q), i0, len, out, vmax);
     __syncwarp();
   }
 }
@@ -893,8 +897,7 @@ static void launch_range_depth(const DevGraph &v, const uint64_t *rowptr, uint32
   switch (g->tuning.decode_stage_depth) {
     case 1: launch_range<1>(v, rowptr, cols, g, grid, err, s); break;
     case 2: launch_range<2>(v, rowptr, cols, g, grid, err, s); break;
-    case 4: launch_range<4>(v, rowptr, cols, g, grid, err, s); break;
-    default: launch_range<0>(v, rowptr, cols, g, grid, err, s);  // unstaged
+    default: launch_range<4>(v, rowptr, cols, g, grid, err, s);
   }
 }
 

@@ -57,3 +57,16 @@ def test_slots_hold_the_lists(oracle_mod, tmp_path, mode, gap):
     for a, b in zip(hops, refs):
         np.testing.assert_array_equal(a, b)
     assert e == re_
+
+
+@pytest.mark.parametrize("depth", [1, 2, 4])
+@pytest.mark.parametrize("gap", [1, 9, 0])
+def test_staged_sectors_hold_the_lists(tmp_path, depth, gap):
+    rp, cols = _csr(gap)
+    G.compress_to_files(rp, cols, "LE", str(tmp_path / "LE"))
+    g = G.Graph(str(tmp_path / "LE"), "LE")
+    g.set_tuning(decode_stage_depth=depth)
+    r, c = g.decode_all()
+    np.testing.assert_array_equal(r, rp)
+    np.testing.assert_array_equal(c, cols)
+    g.check_device_error()
