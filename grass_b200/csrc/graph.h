@@ -205,7 +205,7 @@ int launch_decode_planned(const grass_graph *g, const uint64_t *rowptr, uint32_t
 bool launch_decode_if_planned(const grass_graph *g, const uint64_t *rowptr, uint32_t *cols,
                               unsigned int *err, cudaStream_t s);
 // Decode sweep without a plan: warps over fixed 2048-neighbor tasks of the
-// CSR being written (no allocation, no set-up; about 2.4x slower).
+// CSR being written (no allocation, no set-up; about 3x slower).
 void launch_decode_all(const DevGraph &g, const uint64_t *rowptr, uint32_t *cols, uint64_t E,
                        unsigned int *err, cudaStream_t s);
 

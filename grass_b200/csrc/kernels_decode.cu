@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(256) decode_range_kernel(DevGraph g, const uin
 // with one lane per slot of LE's own code, 0.466 ms the same way on this layout
 // (its slots hold 3 neighbors, so the set-up of a slot is most of the work),
 // 0.259 ms with one neighbor per lane whose place in the slots advances by
-// wrapping counters, and takes 0.173 ms this way.
+// wrapping counters, and takes 0.166 ms this way.
 #ifndef GRASS_FLAT_VERTEX
 #define GRASS_FLAT_VERTEX 16
 #endif

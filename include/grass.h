@@ -168,10 +168,10 @@ typedef struct {
                                  access-policy window                               */
   uint32_t l2_fetch_bytes;    /* 0 = leave as is; 32/64/128: this process's
                                  cudaLimitMaxL2FetchGranularity hint                 */
-  uint32_t decode_stage_depth;/* decode sweep: 0 (default) reads chunk slots
-                                 through L1; 1, 2 or 4 copies groups of 32 slots into
-                                 shared memory (cp.async.bulk) that many groups ahead
-                                 of the one being decoded (measured slower)          */
+  uint32_t decode_stage_depth;/* decode sweep: 0 (default) decodes a neighbor per
+                                 lane; 1, 2 or 4 does so from groups of sectors
+                                 copied into shared memory (cp.async.bulk) that many
+                                 groups ahead less one (measured slower)             */
   uint32_t reserved[2];
 } grass_tuning;
 int grass_set_tuning(grass_graph *g, const grass_tuning *t);
@@ -199,7 +199,7 @@ int grass_decode_all(const grass_graph *g, uint64_t *d_rowptr, uint32_t *d_cols,
  * them.  Speed: once a grass_decode_all on the same graph has built its
  * decode plan (that call allocates, once), this call runs the same planned
  * sweep; before that it runs an unplanned sweep that needs no set-up, about
- * 3x slower (3.1 ms against 0.94 ms for 250 M neighbors on one B200). */
+ * 3x slower (1.74 ms against 0.54 ms for 250 M neighbors on one B200). */
 int grass_decode_all_noalloc(const grass_graph *g, uint64_t *d_rowptr, uint32_t *d_cols,
                              void *stream);
 
@@ -230,9 +230,9 @@ int grass_rw_host(const grass_graph *g, const grass_rw_params *p, const uint32_t
 /* Traffic accounting for a walk (no reference counterpart; the reference
  * reports only wall times, GT/src/grass.cu:2127-2130).  Replays the walk of
  * grass_rw without writing paths and adds to d_out[0] the algorithmic bytes
- * (per draw: 8 offset + ceil(stream bits read / 8) + 4 path entry; 4 per
- * start entry), to d_out[1] the 32-byte sectors the reads span (+1 per draw
- * for the offset) and to d_out[2] the number of draws. */
+ * (per draw: 16 record + ceil(slot bits read / 8) + 4 path entry; 4 per start
+ * entry), to d_out[1] the 32-byte sectors the reads span (+1 per draw for the
+ * record) and to d_out[2] the number of draws. */
 int grass_rw_account(const grass_graph *g, const grass_rw_params *p, const uint32_t *d_starts,
                      uint64_t W, unsigned long long *d_out, void *stream);
 /* Second-order (node2vec) walk: a biased walk beyond the reference, whose
@@ -246,8 +246,11 @@ int grass_rw_account(const grass_graph *g, const grass_rw_params *p, const uint3
  * taken.  Try k of step s of walker w draws Philox(seed; s, w, w >> 32,
  * GRASS_N2V tag | k): word 0 picks the candidate ((r * d) >> 32), word 1 is
  * compared with the integer threshold floor(alpha / alpha_max * 2^32).
- * Membership in N(u) is a binary search of u's sorted neighbor list.  Paths
- * as grass_rw. */
+ * Membership in N(u) is a search of u's sorted neighbor list.  Paths as
+ * grass_rw.  The first call on a graph whose stream is not being captured
+ * builds an index for the search (a word per 128 bytes of slots, kept with the
+ * graph) and waits for it once; without memory for it, or while captured
+ * before, the search goes without, with the same results. */
 typedef struct {
   uint32_t length;     /* steps per walk                                      */
   uint32_t layout;     /* GRASS_LAYOUT_*                                      */
@@ -315,11 +318,10 @@ int grass_mrw_roots(uint64_t n, uint64_t S, uint32_t R, uint64_t seed, uint32_t 
  * GT/src/grass.cu:1085-1117, launched :1641).  The samplers here write
  * fixed-shape outputs with GRASS_INVALID_VERTEX in empty slots; these calls
  * write the valid edges (src, dst) in output order -- an edge is valid when
- * its dst is not GRASS_INVALID_VERTEX -- using per-warp ballot/popc ranks and
- * one scan over 4096-entry tile counts.  Edges past `capacity` are not
- * written; *d_count (a device word) receives the total number of valid
+ * its dst is not GRASS_INVALID_VERTEX -- in two launches, a count and a fill.
+ * Edges past `capacity` are not written; *d_count (a device word) receives the total number of valid
  * edges, which equals the sampler's edge count.  The buffers must be on the
- * current device; each call takes its tile counts from a stream-ordered
+ * current device; each call takes its counts from a stream-ordered
  * memory pool private to this library.
  * ========================================================================= */
 
