@@ -616,7 +616,7 @@ constexpr uint32_t kFlatVertex = GRASS_FLAT_VERTEX;
 constexpr uint32_t kFlatHub = kRange;  // degree from which a vertex is split into ranges
 // Degree from which a vertex is decoded by itself: its set-up is some 250 warp
 // instructions, and a round of 32 neighbors then takes about 25, against 70 in
-// a group (0.173 ms at 128, 0.178 at 256; at most 2048, see FlatSmem::vb).
+// a group (0.166 ms at 96, 128 and 192, 0.174 at 64; at most 2048, see FlatSmem::vb).
 constexpr uint32_t kFlatBig = GRASS_FLAT_BIG;
 
 // Warps per block, one item each, and resident blocks per SM (64 registers).
