@@ -747,6 +747,16 @@ namespace {
 // against 80).
 constexpr uint64_t kSmallHostBytes = 1u << 20;
 
+// Brings a small call's results and the error word to the host.
+int small_results(const grass_graph *g, uint8_t *h_out, size_t out, unsigned int *h_err,
+                  HostPipe &hp) {
+  if (int rc = check_launch()) return rc;
+  GRASS_CUDA(cudaMemcpyAsync(h_out, hp.d_small, out, cudaMemcpyDeviceToHost, hp.st[0]));
+  GRASS_CUDA(cudaMemcpyAsync(h_err, g->d_err, sizeof *h_err, cudaMemcpyDeviceToHost, hp.st[0]));
+  GRASS_CUDA(cudaStreamSynchronize(hp.st[0]));
+  return GRASS_OK;
+}
+
 int rw_host_small(const grass_graph *g, const grass_rw_params &p, const uint32_t *h_starts,
                   uint64_t W, uint32_t *h_paths, uint64_t *edges_out, HostPipe &hp) {
   const size_t in = (W * 4 + 15) & ~15ull, paths = W * ((uint64_t)p.length + 1) * 4;
@@ -771,10 +781,12 @@ int rw_host_small(const grass_graph *g, const grass_rw_params &p, const uint32_t
             reinterpret_cast<uint32_t *>(hp.d_small + 16),
             reinterpret_cast<unsigned long long *>(hp.d_small), g->d_err, hp.st[0], g->tuning,
             g->l2win);
-  if (int rc = check_launch()) return rc;
-  GRASS_CUDA(cudaMemcpyAsync(h_out, hp.d_small, out, cudaMemcpyDeviceToHost, hp.st[0]));
-  GRASS_CUDA(cudaMemcpyAsync(h_err, g->d_err, sizeof *h_err, cudaMemcpyDeviceToHost, hp.st[0]));
-  GRASS_CUDA(cudaStreamSynchronize(hp.st[0]));
+  const int rc = small_results(g, h_out, out, h_err, hp);
+  if (rc) {  // the walk may have run all the same: wait for it, and start over with a new counter
+    cudaStreamSynchronize(hp.st[0]);
+    hp.cap_small = 0;
+    return rc;
+  }
   uint64_t edges;
   memcpy(&edges, h_out, sizeof edges);
   memcpy(h_paths, h_out + 16, paths);
