@@ -486,6 +486,7 @@ int grass_close(grass_graph *g) {
   cudaFree(g->d_plan_small);
   cudaFree(g->d_plan_flat);
   cudaFree(g->d_fences);
+  if (g->fences_done) cudaEventDestroy(g->fences_done);
   delete g;
   return GRASS_OK;
 }
@@ -673,30 +674,61 @@ struct RelaxedCapture {
   ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
 
-// The graph's fences, or null: while the stream is being captured (nothing can
-// be allocated or waited for) or without memory the search goes without them,
-// with the same results.
+// Starts building a graph's fences on a stream of their own: the slots do not
+// change after opening, so the build waits for no other work, and no host
+// thread waits for it.
+static void start_fences(const grass_graph *g) {
+  RelaxedCapture relaxed;
+  cudaStream_t st = nullptr;
+  void *f = nullptr;
+  cudaEvent_t done = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaMallocAsync(&f, fence_words(g->n_words) * 4, st);
+  if (e == cudaSuccess) {
+    launch_build_fences(g->view(), static_cast<uint32_t *>(f), st);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaEventRecord(done, st);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    if (f) cudaFreeAsync(f, st);
+    if (done) cudaEventDestroy(done);
+    f = nullptr;
+    done = nullptr;
+  }
+  if (st) cudaStreamDestroy(st);  // (its work goes on)
+  g->d_fences = static_cast<uint32_t *>(f);
+  g->fences_done = done;
+}
+
+// The graph's fences for work on stream st, or null: without memory, or while
+// st is being captured before they are complete (a capture cannot wait for work
+// outside it), the search goes without them, with the same results.
 static const uint32_t *graph_fences(const grass_graph *g, cudaStream_t st) {
   std::lock_guard<std::mutex> lk(g->fence_mu);
-  if (g->d_fences || g->fences_tried) return g->d_fences;
+  if (g->fences_ready) return g->d_fences;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return nullptr;
+  const bool captured =
+      cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+  if (captured) cudaGetLastError();
+  if (!g->fences_tried) {
+    if (captured) return nullptr;
+    g->fences_tried = true;
+    start_fences(g);
   }
-  g->fences_tried = true;
+  if (!g->d_fences) return nullptr;
   RelaxedCapture relaxed;
-  uint32_t *f = nullptr;
-  if (cudaMalloc(&f, fence_words(g->n_words) * 4) != cudaSuccess) {
+  const cudaError_t q = cudaEventQuery(g->fences_done);
+  if (q == cudaSuccess) {
+    g->fences_ready = true;
+    return g->d_fences;
+  }
+  if (q != cudaErrorNotReady || captured || cudaStreamWaitEvent(st, g->fences_done, 0) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  launch_build_fences(g->view(), f, st);
-  if (cudaStreamSynchronize(st) != cudaSuccess) {  // (reported by the caller's own launch)
-    cudaFree(f);
-    return nullptr;
-  }
-  return g->d_fences = f;
+  return g->d_fences;
 }
 
 int grass_node2vec(const grass_graph *g, const grass_node2vec_params *p,

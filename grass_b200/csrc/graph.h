@@ -77,12 +77,14 @@ struct grass_graph {
   mutable uint4 *d_plan_flat = nullptr;
   mutable uint64_t plan_nflat = 0;
   mutable bool plan_flat_ok = false;
-  // Fences of the node2vec membership search (kernels_sample.cu), built by the
-  // first grass_node2vec that is not being captured; null until then, and for
-  // good where there is no memory for them.
+  // Fences of the node2vec membership search (kernels_sample.cu), whose build is
+  // started by the first grass_node2vec that is not being captured and complete
+  // at fences_done; null until then, and for good where there is no memory for
+  // them.
   mutable std::mutex fence_mu;
   mutable uint32_t *d_fences = nullptr;
-  mutable bool fences_tried = false;
+  mutable cudaEvent_t fences_done = nullptr;
+  mutable bool fences_tried = false, fences_ready = false;  // (ready: seen to be complete)
   grass::DevGraph view() const {
     grass::DevGraph g;
     g.words = d_words;

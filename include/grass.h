@@ -248,9 +248,10 @@ int grass_rw_account(const grass_graph *g, const grass_rw_params *p, const uint3
  * compared with the integer threshold floor(alpha / alpha_max * 2^32).
  * Membership in N(u) is a search of u's sorted neighbor list.  Paths as
  * grass_rw.  The first call on a graph whose stream is not being captured
- * builds an index for the search (a word per 128 bytes of slots, kept with the
- * graph) and waits for it once; without memory for it, or while captured
- * before, the search goes without, with the same results. */
+ * starts building an index for the search on a stream of the library's (a word
+ * per 128 bytes of slots, kept with the graph); `stream` waits for it, the
+ * calling thread does not.  Without memory for it, or while captured before it
+ * is complete, the search goes without, with the same results. */
 typedef struct {
   uint32_t length;     /* steps per walk                                      */
   uint32_t layout;     /* GRASS_LAYOUT_*                                      */
