@@ -858,7 +858,7 @@ int grass_rw_host(const grass_graph *g, const grass_rw_params *p, const uint32_t
     GRASS_CUDA(cudaEventCreateWithFlags(&hp.ev, cudaEventDisableTiming));
     GRASS_CUDA(cudaMalloc(&hp.d_edges, sizeof(unsigned long long)));
   }
-  if (W && W * (L1 + 1) * 4 <= kSmallHostBytes)
+  if (W && W <= kSmallHostBytes / 4 / (L1 + 1))  // (W (L1 + 1) may pass 2^64)
     return rw_host_small(g, *p, h_starts, W, h_paths, edges_out, hp);
   // Chunks of walkers alternate between two streams: while one chunk's paths
   // are copied out, the next chunk is copied in and walked.  Walker ids stay

@@ -1,5 +1,7 @@
 """Small walks on host buffers (one pinned buffer, a running edge counter) when
 something around them fails."""
+import contextlib
+import ctypes as C
 import os
 
 import numpy as np
@@ -35,3 +37,15 @@ def test_edges_after_a_failed_small_call(oracle_mod):
         paths, e = g.rw(starts, 20, 3)
         np.testing.assert_array_equal(paths, ref)
         assert e == edges
+
+
+def test_a_call_too_large_for_64_bits_is_refused(oracle_mod):
+    """Sizes whose product in bytes is a multiple of 2^64: no memory, not a small call."""
+    g, og, starts = _graphs(oracle_mod)
+    many = np.zeros(1 << 31, np.uint32)  # (never written: takes no memory)
+    p, e = G.RwParams((1 << 31) - 2, G.LAYOUT_WALK_MAJOR, 3), C.c_uint64()
+    assert len(many) * (p.length + 2) * 4 == 1 << 64
+    assert G.lib.grass_rw_host(g.handle, C.byref(p), G._p(many), len(many), G._p(many), C.byref(e)) == G.E_OOM
+    with contextlib.suppress(G.GrassError):  # (takes the refused allocation's error)
+        g.rw(starts, 20, 3)
+    np.testing.assert_array_equal(g.rw(starts, 20, 3)[0], og.rw("LE", starts, 20, 3)[0])
