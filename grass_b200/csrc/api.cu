@@ -779,6 +779,35 @@ namespace {
 // against 80).
 constexpr uint64_t kSmallHostBytes = 1u << 20;
 
+// Test hook, off in the library: pinned memory cannot be had.
+#ifndef GRASS_NO_PINNED
+#define GRASS_NO_PINNED 0
+#endif
+
+size_t small_in(uint64_t W) { return (W * 4 + 15) & ~15ull; }
+
+// Room for a small call of W walkers and `steps` columns of paths; false where
+// there is no memory for it.
+bool small_room(uint64_t W, uint64_t steps, HostPipe &hp) {
+  const size_t need = small_in(W) + 16 + W * steps * 4;
+  if (hp.cap_small >= need + 16) return true;
+  RelaxedCapture relaxed;
+  cudaFreeHost(hp.h_small);
+  cudaFree(hp.d_small);
+  hp.h_small = hp.d_small = nullptr;
+  hp.cap_small = 0;
+  hp.edges_seen = 0;
+  const size_t cap = std::max<size_t>(2 * need, 64 << 10);
+  if (!GRASS_NO_PINNED && cudaMallocHost(&hp.h_small, cap) == cudaSuccess &&
+      cudaMalloc(&hp.d_small, cap) == cudaSuccess &&
+      cudaMemsetAsync(hp.d_small, 0, 16, hp.st[0]) == cudaSuccess) {
+    hp.cap_small = cap;
+    return true;
+  }
+  cudaGetLastError();
+  return false;
+}
+
 // Brings a small call's results and the error word to the host.
 int small_results(const grass_graph *g, uint8_t *h_out, size_t out, unsigned int *h_err,
                   HostPipe &hp) {
@@ -791,21 +820,8 @@ int small_results(const grass_graph *g, uint8_t *h_out, size_t out, unsigned int
 
 int rw_host_small(const grass_graph *g, const grass_rw_params &p, const uint32_t *h_starts,
                   uint64_t W, uint32_t *h_paths, uint64_t *edges_out, HostPipe &hp) {
-  const size_t in = (W * 4 + 15) & ~15ull, paths = W * ((uint64_t)p.length + 1) * 4;
+  const size_t in = small_in(W), paths = W * ((uint64_t)p.length + 1) * 4;
   const size_t out = 16 + paths;  // the counter, then the paths
-  if (hp.cap_small < in + out + 16) {
-    RelaxedCapture relaxed;
-    cudaFreeHost(hp.h_small);
-    cudaFree(hp.d_small);
-    hp.h_small = hp.d_small = nullptr;
-    hp.cap_small = 0;
-    hp.edges_seen = 0;
-    const size_t cap = std::max<size_t>(2 * (in + out), 64 << 10);
-    GRASS_CUDA(cudaMallocHost(&hp.h_small, cap));
-    GRASS_CUDA(cudaMalloc(&hp.d_small, cap));
-    GRASS_CUDA(cudaMemsetAsync(hp.d_small, 0, 16, hp.st[0]));
-    hp.cap_small = cap;
-  }
   uint8_t *h_out = hp.h_small + in;
   unsigned int *h_err = reinterpret_cast<unsigned int *>(h_out + out);
   memcpy(hp.h_small, h_starts, W * 4);
@@ -858,7 +874,8 @@ int grass_rw_host(const grass_graph *g, const grass_rw_params *p, const uint32_t
     GRASS_CUDA(cudaEventCreateWithFlags(&hp.ev, cudaEventDisableTiming));
     GRASS_CUDA(cudaMalloc(&hp.d_edges, sizeof(unsigned long long)));
   }
-  if (W && W <= kSmallHostBytes / 4 / (L1 + 1))  // (W (L1 + 1) may pass 2^64)
+  if (W && W <= kSmallHostBytes / 4 / (L1 + 1) &&  // (W (L1 + 1) may pass 2^64)
+      small_room(W, L1, hp))
     return rw_host_small(g, *p, h_starts, W, h_paths, edges_out, hp);
   // Chunks of walkers alternate between two streams: while one chunk's paths
   // are copied out, the next chunk is copied in and walked.  Walker ids stay

@@ -49,3 +49,21 @@ def test_a_call_too_large_for_64_bits_is_refused(oracle_mod):
     with contextlib.suppress(G.GrassError):  # (takes the refused allocation's error)
         g.rw(starts, 20, 3)
     np.testing.assert_array_equal(g.rw(starts, 20, 3)[0], og.rw("LE", starts, 20, 3)[0])
+
+
+def test_small_call_without_pinned_memory(oracle_mod):
+    """The test build of the library, where pinned memory cannot be had: the same walks."""
+    lib, P = C.CDLL(os.path.join(os.path.dirname(G.LIB_PATH), "libgrass_b200_stagetest.so")), C.c_void_p
+    lib.grass_open.argtypes = [C.c_char_p, C.c_int, C.c_int, C.POINTER(P)]
+    lib.grass_rw_host.argtypes = [P, P, P, C.c_uint64, P, C.POINTER(C.c_uint64)]
+    lib.grass_close.argtypes = [P]
+    prefix, h, e = os.path.join(golden_graph("rmat_s10_e8")[0], "LE"), P(), C.c_uint64()
+    assert lib.grass_open(prefix.encode(), G.MODE_LE, 0, C.byref(h)) == G.OK
+    starts = np.arange(100, dtype=np.uint32)
+    ref, edges = oracle_mod.OracleGraph(prefix).rw("LE", starts, 20, 3)
+    for _ in range(2):
+        paths, p = np.zeros((100, 21), np.uint32), G.RwParams(20, G.LAYOUT_WALK_MAJOR, 3)
+        assert lib.grass_rw_host(h, C.byref(p), G._p(starts), 100, G._p(paths), C.byref(e)) == G.OK
+        np.testing.assert_array_equal(paths, ref)
+        assert e.value == edges
+    assert lib.grass_close(h) == G.OK
