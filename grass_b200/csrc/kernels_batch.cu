@@ -256,24 +256,25 @@ void split_job(const grass_job &j, uint32_t ji, const grass_batch_config &c,
 
 int launch_batch(const DevGraph &dg, int device, const BatchJob *d_jobs, const BatchTask *d_tasks,
                  const BatchRanges &ranges, unsigned int *d_queue, unsigned long long *d_total,
-                 unsigned int *d_err, cudaStream_t s, BatchSide &side,
+                 unsigned int *d_err, cudaStream_t s, BatchSide *side,
                  const grass_batch_config &c) {
   const bool warps = ranges.rw > ranges.cta;
+  if (!warps || !ranges.cta) side = nullptr;
   if (ranges.cta) {
     cudaStream_t cs = s;
-    if (warps) {
-      cudaError_t e = side.create();
-      if (e == cudaSuccess) e = cudaEventRecord(side.fork, s);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(side.st, side.fork, 0);
+    if (side) {
+      cudaError_t e = side->create();
+      if (e == cudaSuccess) e = cudaEventRecord(side->fork, s);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(side->st, side->fork, 0);
       if (e != cudaSuccess) return cuda_fail(e, "batch side stream");
-      cs = side.st;
+      cs = side->st;
     }
     auto k = dg.mode == GRASS_MODE_CSR_INTERNAL ? batch_cta_kernel<kCsr> : batch_cta_kernel<kSlots>;
     const unsigned grid = std::min<unsigned>(ranges.cta, (unsigned)sm_count(device) * 2);
     k<<<grid, 32 * kBatchCtaWarps, 0, cs>>>(dg, d_jobs, d_tasks, ranges.cta, d_queue, d_total,
                                              d_err);
     cudaError_t e = cudaGetLastError();
-    if (warps && e == cudaSuccess) e = cudaEventRecord(side.join, cs);
+    if (side && e == cudaSuccess) e = cudaEventRecord(side->join, cs);
     if (e != cudaSuccess) return cuda_fail(e, "batch kernel launch");
   }
   if (!warps) return GRASS_OK;
@@ -289,7 +290,7 @@ int launch_batch(const DevGraph &dg, int device, const BatchJob *d_jobs, const B
       (uint32_t)std::min<uint64_t>(8, std::max<uint64_t>(1, (ranges.khop - ranges.mrw) / takes));
   k<<<grid, threads, 0, s>>>(dg, d_jobs, d_tasks, ranges, grab, d_queue, d_total, d_err);
   cudaError_t e = cudaGetLastError();
-  if (ranges.cta && e == cudaSuccess) e = cudaStreamWaitEvent(s, side.join, 0);
+  if (side && e == cudaSuccess) e = cudaStreamWaitEvent(s, side->join, 0);
   return e == cudaSuccess ? GRASS_OK : cuda_fail(e, "batch kernel launch");
 }
 
@@ -404,15 +405,16 @@ int build(grass_batch *b) {
   if (!tasks.empty())
     GRASS_CUDA(cudaMemcpy(b->d_tasks, tasks.data(), tasks.size() * sizeof(BatchTask),
                           cudaMemcpyHostToDevice));
-  // (now, not in launch_batch: a later run may be under capture)
+  // (now, not in launch_batch: a later run may be beside a capture)
   if (b->ranges.cta && b->ranges.rw > b->ranges.cta) GRASS_CUDA(b->side.create());
   b->built_cfg = c;
   b->dirty = false;
   return GRASS_OK;
 }
 
-// Queue reset, multi-RW root restore and the persistent kernel, on stream s.
-int enqueue(grass_batch *b, cudaStream_t s, unsigned long long *total) {
+// Queue reset, multi-RW root restore and the persistent kernels, on stream s
+// (and, not null, beside it on `side`).
+int enqueue(grass_batch *b, cudaStream_t s, BatchSide *side, unsigned long long *total) {
   const grass_batch_config &c = b->built_cfg;
   for (size_t i = 0; i < b->restore.size(); i++)
     GRASS_CUDA(cudaMemcpyAsync(b->restore[i].first, b->restore[i].second, b->restore_n[i] * 4,
@@ -420,7 +422,7 @@ int enqueue(grass_batch *b, cudaStream_t s, unsigned long long *total) {
   GRASS_CUDA(cudaMemsetAsync(b->d_queue, 0, kQueueWords * sizeof(unsigned int), s));
   if (!b->ntasks) return GRASS_OK;
   return launch_batch(b->dg, b->device, b->d_jobs, b->d_tasks, b->ranges, b->d_queue, total, b->d_err,
-                      s, b->side, c);
+                      s, side, c);
 }
 
 int check_job(const grass_job *j) {
@@ -555,7 +557,13 @@ int grass_batch_run(grass_batch *b, void *stream, unsigned long long *d_total_ed
     if (int rc = build(b)) return rc;
   }
   if (resolve(b->cfg, b->mode()).use_graph == 2) {
-    const int rc = enqueue(b, st, d_total_edges);
+    // Under the caller's capture the side stream would be drawn into it and be
+    // unusable to other runs until it ends: both kernels on the captured stream.
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    const bool captured =
+        cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+    if (captured) cudaGetLastError();
+    const int rc = enqueue(b, st, captured ? nullptr : &b->side, d_total_edges);
     if (!rc && b->ntasks) count_launch();
     return rc;
   }
@@ -564,7 +572,7 @@ int grass_batch_run(grass_batch *b, void *stream, unsigned long long *d_total_ed
     b->exec = nullptr;
     if (!b->cap) GRASS_CUDA(cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking));
     GRASS_CUDA(cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal));
-    const int rc = enqueue(b, b->cap, d_total_edges);
+    const int rc = enqueue(b, b->cap, &b->side, d_total_edges);
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(b->cap, &graph);
     if (rc) {

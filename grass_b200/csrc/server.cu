@@ -572,7 +572,7 @@ void grass_server::launch(Batch *b) {
                         reinterpret_cast<const BatchTask *>(d + tasks_off),
                         batch_ranges(cta, mrw, khop, rw, bcfg),
                         reinterpret_cast<unsigned int *>(d + queue_off), nullptr,
-                        reinterpret_cast<unsigned int *>(d + err_off), s, sides[b->slot], bcfg);
+                        reinterpret_cast<unsigned int *>(d + err_off), s, &sides[b->slot], bcfg);
     if (!rc && ntasks) count_launch();
     lap(3);
     if (!rc) {
