@@ -86,6 +86,9 @@ inline BatchRanges batch_ranges(const std::vector<BatchTask> &cta, const std::ve
   return r;
 }
 
+// Kernels that launch_batch launches for the work items.
+inline uint64_t batch_kernels(const BatchRanges &r) { return (r.cta > 0) + (r.rw > r.cta); }
+
 // A stream and events beside a batch's stream, for its block-level items.
 struct BatchSide {
   cudaStream_t st = nullptr;

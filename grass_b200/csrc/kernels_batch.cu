@@ -564,7 +564,7 @@ int grass_batch_run(grass_batch *b, void *stream, unsigned long long *d_total_ed
         cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
     if (captured) cudaGetLastError();
     const int rc = enqueue(b, st, captured ? nullptr : &b->side, d_total_edges);
-    if (!rc && b->ntasks) count_launch();
+    if (!rc) count_launch(batch_kernels(b->ranges));
     return rc;
   }
   if (!b->exec || b->exec_total != d_total_edges) {
@@ -586,7 +586,7 @@ int grass_batch_run(grass_batch *b, void *stream, unsigned long long *d_total_ed
     b->exec_total = d_total_edges;
   }
   GRASS_CUDA(cudaGraphLaunch(b->exec, st));
-  count_launch();
+  count_launch(batch_kernels(b->ranges));
   return GRASS_OK;
 }
 

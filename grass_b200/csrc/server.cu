@@ -567,13 +567,13 @@ void grass_server::launch(Batch *b) {
       if (e != cudaSuccess) rc = cuda_fail(e, "server upload");
       lap(2);
     }
+    const BatchRanges ranges = batch_ranges(cta, mrw, khop, rw, bcfg);
     if (!rc && ntasks)
       rc = launch_batch(g->view(), g->device, reinterpret_cast<const BatchJob *>(d + jobs_off),
-                        reinterpret_cast<const BatchTask *>(d + tasks_off),
-                        batch_ranges(cta, mrw, khop, rw, bcfg),
+                        reinterpret_cast<const BatchTask *>(d + tasks_off), ranges,
                         reinterpret_cast<unsigned int *>(d + queue_off), nullptr,
                         reinterpret_cast<unsigned int *>(d + err_off), s, &sides[b->slot], bcfg);
-    if (!rc && ntasks) count_launch();
+    if (!rc) count_launch(batch_kernels(ranges));
     lap(3);
     if (!rc) {
       e = cudaMemcpyAsync(b->out_host, d + b->d2h_off, b->d2h_bytes, cudaMemcpyDeviceToHost, s);

@@ -1,4 +1,5 @@
-"""Plain runs of a batch of both levels on several streams, under capture and beside one."""
+"""Batches of both levels: plain runs on several streams, under capture and beside
+one; the count of their kernels."""
 import os
 
 import numpy as np
@@ -53,3 +54,20 @@ def test_plain_run_beside_its_own_capture(oracle_mod):
     b.set_config(use_graph=1)
     b.run(stream=other)
     _check(outs)
+
+
+@pytest.mark.parametrize("use_graph", [1, 2])
+def test_every_kernel_of_a_run_is_counted(oracle_mod, use_graph):
+    import torch
+    b, _ = _mixed(oracle_mod)
+    one = G.Batch(b._g)
+    paths = torch.zeros(300, 21, dtype=torch.int32, device="cuda")
+    one.add_rw(b.keep[1], 300, 20, 2, paths)
+    for batch, kernels in ((b, 2), (one, 1), (G.Batch(b._g), 0)):
+        batch.set_config(use_graph=use_graph)
+        batch.run()
+        before = G.launch_count()
+        for _ in range(3):
+            batch.run()
+        assert G.launch_count() - before == 3 * kernels
+    torch.cuda.synchronize()
