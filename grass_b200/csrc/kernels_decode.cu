@@ -882,11 +882,11 @@ template <int DEPTH>
 static void launch_range(const DevGraph &v, const uint64_t *rowptr, uint32_t *cols,
                          const grass_graph *g, unsigned grid, unsigned int *err, cudaStream_t s) {
   const uint32_t smem = kDecodeWarps * WarpSmem<DEPTH>::bytes();
-  static std::once_flag once;  // opt in to more than 48 KB of dynamic shared memory
-  std::call_once(once, [&] {
-    cudaFuncSetAttribute(decode_range_kernel<DEPTH>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  });
+  // The opt-in to more than 48 KB of dynamic shared memory holds for the current
+  // device, so it goes with each launch.  (Its error is the launch's.)
+  if (cudaFuncSetAttribute(decode_range_kernel<DEPTH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)smem) != cudaSuccess)
+    return;
   decode_range_kernel<DEPTH><<<grid, 32 * kDecodeWarps, smem, s>>>(
       v, rowptr, cols, g->d_plan_big, g->plan_nbig, err);
 }
