@@ -650,11 +650,14 @@ int apply_tuning(int device, const grass_tuning &t, const void *base, size_t byt
 // walk 0.5% faster with four.  Blocks of 64 threads spread few walkers over more
 // SMs and leave a place sooner (us at 64 / 256 threads: 4,096 x 80 on s22 63 /
 // 75, on s16 54.7 / 55.1; 1M x 80 2014 / 2032); 512 resident threads a block
-// pair (64 registers) beat 1536 (40: 2.09 -> 2.15 ms).
+// pair (64 registers) beat 1536 (40: 2.09 -> 2.15 ms).  A caller that bounds the
+// blocks per SM and not their threads means blocks of 256, as they were when the
+// bound was the only way to place fewer (1M x 40, two blocks: 1.34 ms, of 64
+// threads 3.27).
 grass_tuning resolve_tuning(const grass_tuning &t, int kind) {
   grass_tuning r = t;
   if (!r.rw_depth) r.rw_depth = kind == 2 ? 4 : 1;
-  if (!r.rw_threads) r.rw_threads = kind == 2 ? 256 : 64;
+  if (!r.rw_threads) r.rw_threads = kind == 2 || r.rw_blocks_per_sm ? 256 : 64;
   return r;  // rw_blocks_per_sm == 0: as many as are resident
 }
 

@@ -161,7 +161,8 @@ int grass_device_view(const grass_graph *g, const uint32_t **words, uint64_t *n_
 typedef struct {
   uint32_t rw_depth;          /* walkers interleaved per thread: 1, 2, 4
                                  (default 1 for LE and GT, 4 for CSR)                */
-  uint32_t rw_threads;        /* threads per block for walks (default 64; CSR 256)   */
+  uint32_t rw_threads;        /* threads per block for walks (default 64; 256 for CSR
+                                 or with rw_blocks_per_sm set)                       */
   uint32_t rw_blocks_per_sm;  /* resident blocks per SM for walks (0 = all resident) */
   uint32_t l2_persist;        /* 1: launches mark the vertex records (or CSR row
                                  pointers) persisting in L2 through a per-launch
