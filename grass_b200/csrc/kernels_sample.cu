@@ -15,7 +15,11 @@
 #include <mutex>
 
 // Resident 512-thread blocks per SM each walk kernel is compiled for (its
-// register budget).
+// register budget).  With two or four walkers a lane the compressed walk needs
+// more than the 64 registers of two blocks (it spilled 160 and 748 bytes) and is
+// compiled for one: 1M walkers x 40, R-MAT s22 ef32, step-major, ms with two /
+// one: two walkers 1.15 / 1.01, four 1.31 / 1.09; 4,096 walkers, us: 48 / 36 and
+// 107 / 50 (with the grid of rw_launch_depth).
 #ifndef GRASS_RW_MIN_BLOCKS
 #define GRASS_RW_MIN_BLOCKS 2
 #endif
@@ -36,7 +40,7 @@ __device__ __forceinline__ void store_path(uint32_t *paths, int layout, uint64_t
 // w0: walker id of starts[0] -- draws use walker id w0 + w, so a batch split
 // into chunks produces the same walks as one launch.
 template <int MODE, int DEPTH>
-__global__ void __launch_bounds__(512, GRASS_RW_MIN_BLOCKS) rw_kernel(DevGraph g, const uint32_t *__restrict__ starts,
+__global__ void __launch_bounds__(512, DEPTH == 1 ? GRASS_RW_MIN_BLOCKS : 1) rw_kernel(DevGraph g, const uint32_t *__restrict__ starts,
                                                  uint64_t W, uint32_t L, uint64_t seed,
                                                  uint64_t w0, int layout,
                                                  uint32_t *__restrict__ paths,
@@ -651,9 +655,8 @@ int apply_tuning(int device, const grass_tuning &t, const void *base, size_t byt
 // SMs and leave a place sooner (us at 64 / 256 threads: 4,096 x 80 on s22 63 /
 // 75, on s16 54.7 / 55.1; 1M x 80 2014 / 2032); 512 resident threads a block
 // pair (64 registers) beat 1536 (40: 2.09 -> 2.15 ms).  A caller that bounds the
-// blocks per SM and not their threads means blocks of 256, as they were when the
-// bound was the only way to place fewer (1M x 40, two blocks: 1.34 ms, of 64
-// threads 3.27).
+// blocks per SM and not their threads means blocks of 256 (1M x 40 at two of
+// them: 1.10 ms, at two of 64 threads 3.16).
 grass_tuning resolve_tuning(const grass_tuning &t, int kind) {
   grass_tuning r = t;
   if (!r.rw_depth) r.rw_depth = kind == 2 ? 4 : 1;
@@ -683,8 +686,9 @@ static void rw_launch_depth(const DevGraph &g, const grass_rw_params &p, const u
   const size_t smem = p.layout == GRASS_LAYOUT_WALK_MAJOR
                           ? (size_t)t.rw_threads / 32 * kPathStageWords<DEPTH> * 4 : 0;
   static_assert(512 / 32 * kPathStageWords<DEPTH> * 4 <= 48 * 1024, "no opt-in needed");
+  // (a lane takes a second walker only where all resident lanes have one)
   const unsigned grid = resident_grid(kern, (int)t.rw_threads, smem, t.rw_blocks_per_sm, W,
-                                      (uint64_t)t.rw_threads * DEPTH);
+                                      t.rw_threads);
   launch_with_window(kern, grid, t.rw_threads, smem, s, win, g, starts, W, p.length, p.seed, w0,
                      (int)p.layout, paths, edges, err);
 }
