@@ -17,7 +17,11 @@
 
 // Resident 256-thread blocks per SM the compiler must allow for: the items wait
 // on memory, so more resident warps pay until spills cost more (the 256-job mix
-// on R-MAT s22 ef32: 1.25 ms at 4, 1.33 at 3).
+// on R-MAT s22 ef32: 1.25 ms at 4, 1.33 at 3).  Several walkers a lane need more
+// registers (at 4 blocks two walkers spilled 276 bytes and four 928): 30 walk jobs
+// there, us at 4 / 3 / 2 blocks: two walkers 1297 / 1065 / 1146, four 1443 / 1499 /
+// 1261; on the CSR, whose draws need no sector, 1356 / 1156 / 1274 and 1438 / 1147 /
+// 1283.
 #ifndef GRASS_BATCH_MIN_BLOCKS
 #define GRASS_BATCH_MIN_BLOCKS 4
 #endif
@@ -95,8 +99,11 @@ __global__ void __launch_bounds__(32 * kBatchCtaWarps, 2)
 // 1.61 and 1.25.)
 // The kinds come in the order of how long an item takes (a chain, 100 steps of
 // a tile of walkers, a seed), so that the last items are short.
+constexpr int batch_min_blocks(int mode, int depth) {
+  return depth == 1 ? GRASS_BATCH_MIN_BLOCKS : depth == 4 && mode != kCsr ? 2 : 3;
+}
 template <int MODE, int DEPTH>
-__global__ void __launch_bounds__(256, GRASS_BATCH_MIN_BLOCKS) batch_kernel(DevGraph g, const BatchJob *__restrict__ jobs,
+__global__ void __launch_bounds__(256, batch_min_blocks(MODE, DEPTH)) batch_kernel(DevGraph g, const BatchJob *__restrict__ jobs,
                                                     const BatchTask *__restrict__ tasks,
                                                     BatchRanges R, uint32_t khop_grab,
                                                     unsigned int *queue,

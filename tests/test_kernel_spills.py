@@ -29,6 +29,12 @@ LIMITS = {
         "n2v_kernel<1>": (64, 0), "n2v_kernel<2>": (64, 0),
         "khop_kernel<1>": (64, 48), "khop_csr_kernel": (64, 24),
     },
+    "kernels_batch.cu": {
+        # four blocks of 256 threads; three with two walkers a lane, two with four (CSR: three)
+        "batch_kernel<1, 1>": (64, 88), "batch_kernel<1, 2>": (80, 56), "batch_kernel<1, 4>": (128, 176),
+        "batch_kernel<2, 1>": (64, 56), "batch_kernel<2, 2>": (80, 56), "batch_kernel<2, 4>": (80, 12),
+        "batch_cta_kernel<1>": (64, 48), "batch_cta_kernel<2>": (64, 36),
+    },
 }
 
 
