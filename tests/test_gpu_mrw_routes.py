@@ -1,0 +1,33 @@
+"""Multi-RW on both sides of the rules that pick its kernels and their shapes,
+against the oracle."""
+import os
+
+import numpy as np
+import pytest
+
+from conftest import golden_graph
+import grass_b200 as G
+
+pytestmark = pytest.mark.gpu
+
+
+def _compare(oracle_mod, name, mode, samples, walkers, steps, select, roots=None):
+    prefix = os.path.join(golden_graph(name)[0], mode)
+    g, og = G.Graph(prefix, mode), oracle_mod.OracleGraph(prefix)
+    if roots is None:
+        roots = np.random.default_rng(steps).integers(0, g.n + 1, (samples, walkers), dtype=np.uint32)
+    got = g.mrw(roots, steps, 4, select)
+    for a, b in zip(got, og.mrw(mode, roots, steps, 4, select)):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("walkers,steps", [
+    (5, 1), (300, 2), (40, 15), (40, 16), (33, 31), (33, 32), (33, 33), (600, 64), (20, 500), (300, 4095), (600, 4097)])
+def test_few_events_to_order(oracle_mod, walkers, steps):
+    """Continuous time with event counts around the numbers of buckets."""
+    _compare(oracle_mod, "rmat_s10_e8", "LE", 3, walkers, steps, G.SELECT_DEGREE_CT)
+
+
+def test_no_events(oracle_mod):
+    """Continuous time from no vertex at all (ids past the last): nothing moves."""
+    _compare(oracle_mod, "edge_cases", "GT", 2, 5, 9, G.SELECT_DEGREE_CT, np.full((2, 5), G.INVALID, np.uint32))
