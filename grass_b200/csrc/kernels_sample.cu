@@ -9,6 +9,7 @@
 // each thread owns DEPTH walkers and interleaves them, which keeps DEPTH
 // independent decode chains in flight per thread.
 #include "graph.h"
+#include "launch_rules.h"
 #include "mrw_cta.cuh"
 #include "sample_warp.cuh"
 
@@ -864,13 +865,8 @@ int launch_mrw(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots, ui
   // samples 46 / 73, 600 103 / 120, 1184 122 / 133, 8192 706 / 300; 2000 x
   // 1024, r = 148: 148 36 / 59, 600 137 / 95; 2000 x 10,000: 600 527 / 723,
   // 1184 865 / 759.  At 100 steps a warp is never slower.
-  // Continuous time with many walkers: 1024 threads at 64 registers (2000 walkers
-  // x 10,000 steps, 1 / 51 samples: 246 / 320 us, 512 threads 279 / 400); with
-  // few, the 116 registers pay (80 x 100, 2000 samples: 279 us against 331).
-  const bool ct = p.select == GRASS_SELECT_DEGREE_CT, wide = ct && p.walkers > 512;
-  const uint64_t want = ct ? p.walkers : p.walkers / 2;
-  const int threads = (int)std::min<uint64_t>(wide ? 1024 : 512,
-                                              std::max<uint64_t>(128, (want + 31) / 32 * 32));
+  const bool ct = p.select == GRASS_SELECT_DEGREE_CT, wide = ct && p.walkers > kWideWalkers;
+  const int threads = mrw_block_threads(S, p.walkers, ct, sm_count(cur_dev()));
   auto cta = wide ? mrw_cta_kernel<kSlots, 32> : mrw_cta_kernel<kSlots, 16>;
   uint64_t resident = 0;
   if (ct || (p.select == GRASS_SELECT_UNIFORM && p.steps >= 512))

@@ -1,0 +1,37 @@
+// launch_rules.h -- which multi-RW kernel runs a call and in what shape: host
+// arithmetic on sizes and on how many samples are resident at once, without
+// anything of CUDA (tests compile it by itself).  Figures: one B200, R-MAT s22 ef32.
+#pragma once
+#include <stdint.h>
+
+#include <algorithm>
+
+namespace grass {
+
+// A number of threads as a block size: whole warps, between `least` and `most`.
+inline int block_size(uint64_t threads, int least, int most) {
+  return (int)std::min<uint64_t>(most, std::max<uint64_t>(least, (threads + 31) / 32 * 32));
+}
+
+// Continuous-time multi-RW of at most kWideWalkers walkers takes the kernel of
+// 116 registers, of more the one of 64 registers and up to 1024 threads (2000
+// walkers x 10,000 steps, 1 / 51 samples: 246 / 320 us, with 512 threads 279 /
+// 400; with few walkers the registers pay: 80 x 100, 2000 samples 279 us against
+// 331).
+constexpr uint32_t kWideWalkers = 512;
+
+// Threads of a block that takes one sample of R walkers, of S samples on `sms`
+// SMs, in a launch of its own (mrw_cta_kernel).  Continuous time: a thread a
+// walker is fastest while every sample has an SM to itself.  With more samples
+// blocks of 160 threads pay, three of which are resident where one of 288 to 512
+// is (us with a thread a walker / 160 / R / 2 and the radix sort: 257
+// walkers x 400 steps, 148 samples 73 / 85 / 145, 300 130 / 92 / 153, 8192 3022 /
+// 1613 / 1984.  512 x 400: 148 56 / 89 / 111, 300 119 / 98 / 195, 8192 2463 / 1838 /
+// 2851).
+inline int mrw_block_threads(uint64_t S, uint32_t R, bool continuous, int sms) {
+  if (!continuous) return block_size(R / 2, 128, 512);
+  if (R > kWideWalkers) return block_size(R, 128, 1024);
+  return block_size(R, 128, S <= (uint64_t)sms ? 512 : 160);
+}
+
+}  // namespace grass

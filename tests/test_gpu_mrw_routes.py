@@ -31,3 +31,9 @@ def test_few_events_to_order(oracle_mod, walkers, steps):
 def test_no_events(oracle_mod):
     """Continuous time from no vertex at all (ids past the last): nothing moves."""
     _compare(oracle_mod, "edge_cases", "GT", 2, 5, 9, G.SELECT_DEGREE_CT, np.full((2, 5), G.INVALID, np.uint32))
+
+
+@pytest.mark.parametrize("samples,walkers,steps", [(148, 257, 40), (149, 257, 40), (200, 512, 33), (150, 161, 20), (149, 200, 500)])
+def test_more_continuous_time_samples_than_sms(oracle_mod, samples, walkers, steps):
+    """Blocks of fewer threads than walkers."""
+    _compare(oracle_mod, "rmat_s10_e8", "GT", samples, walkers, steps, G.SELECT_DEGREE_CT)

@@ -1,0 +1,32 @@
+"""The rules that pick multi-RW kernels, at sizes where the choices were measured to
+differ (CPU only: grass_b200/csrc/launch_rules.h is plain C++)."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+pytestmark = pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+
+
+@pytest.fixture(scope="module")
+def rule(tmp_path_factory):
+    """rule("expression"): its value as an integer."""
+    tmp = tmp_path_factory.mktemp("rules")
+
+    def value(expression):
+        src, exe = tmp / "rule.cpp", tmp / "rule"
+        src.write_text('#include <stdio.h>\n#include "launch_rules.h"\nusing namespace grass;\n'
+                       f'int main() {{ printf("%lld", (long long)({expression})); }}\n')
+        subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-I" + os.path.join(ROOT, "grass_b200", "csrc"),
+                        "-o", str(exe), str(src)], check=True)
+        return int(subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout)
+    return value
+
+
+@pytest.mark.parametrize("samples,walkers,threads", [
+    (1, 80, 128), (8192, 80, 128), (148, 160, 160), (8192, 160, 160), (148, 257, 288), (149, 257, 160), (8192, 512, 160),
+    (1, 512, 512), (1, 513, 544), (8192, 2000, 1024)])
+def test_threads_of_a_continuous_time_sample(rule, samples, walkers, threads):
+    assert rule(f"mrw_block_threads({samples}, {walkers}, true, 148)") == threads
