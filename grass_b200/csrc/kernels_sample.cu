@@ -858,20 +858,16 @@ int launch_mrw(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots, ui
                uint32_t max_degree, cudaStream_t s) {
   if (!S || !p.steps) return GRASS_OK;
   // Block per sample (walkers in parallel) for continuous-time selection, and
-  // for uniform selection with long chains (same output as the warp kernel):
-  // a block ends a chain sooner, a warp needs fewer threads.  With r samples
-  // resident as blocks the two cross near r (1 + steps / 2048) samples
-  // (R-MAT s22 ef32, us block / warp): 80 walkers x 1024 steps, r = 592: 148
-  // samples 46 / 73, 600 103 / 120, 1184 122 / 133, 8192 706 / 300; 2000 x
-  // 1024, r = 148: 148 36 / 59, 600 137 / 95; 2000 x 10,000: 600 527 / 723,
-  // 1184 865 / 759.  At 100 steps a warp is never slower.
+  // for uniform selection where a block ends a long chain sooner than a warp
+  // (same output); the rules and their measurements are in launch_rules.h.
   const bool ct = p.select == GRASS_SELECT_DEGREE_CT, wide = ct && p.walkers > kWideWalkers;
   const int threads = mrw_block_threads(S, p.walkers, ct, sm_count(cur_dev()));
   auto cta = wide ? mrw_cta_kernel<kSlots, 32> : mrw_cta_kernel<kSlots, 16>;
   uint64_t resident = 0;
-  if (ct || (p.select == GRASS_SELECT_UNIFORM && p.steps >= 512))
+  if (p.select != GRASS_SELECT_DEGREE)
     resident = (uint64_t)sm_count(cur_dev()) * resident_blocks((const void *)cta, threads, 0);
-  if (ct || S <= resident + resident * p.steps / 2048) {
+  if (ct || (p.select == GRASS_SELECT_UNIFORM &&
+             mrw_uniform_by_blocks(S, p.walkers, p.steps, threads, resident))) {
     const uint64_t grid = std::min<uint64_t>(S, resident);
     const uint64_t stride = mrw_sample_scratch(p.walkers, p.steps, p.select);
     unsigned char *scr = nullptr;

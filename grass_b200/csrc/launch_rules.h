@@ -34,4 +34,29 @@ inline int mrw_block_threads(uint64_t S, uint32_t R, bool continuous, int sms) {
   return block_size(R, 128, S <= (uint64_t)sms ? 512 : 160);
 }
 
+// Rounds of `resident` samples at a time that S samples take.
+inline uint64_t sample_rounds(uint64_t S, uint64_t resident) {
+  return (S + resident - 1) / std::max<uint64_t>(resident, 1);
+}
+
+// Whether S samples of uniform multi-RW (R walkers, T steps) run as blocks of
+// `threads` threads, `resident` of them at a time, or as warps: the output is
+// the same.  A warp takes 32 steps of a sample a round and needs about T / 10 us
+// for as many samples as fit.  A round of blocks takes about 11 us to set up,
+// more with many walkers, and then T steps shared by its threads or, with few
+// walkers, by the walkers (a step's figures are tenths of a microsecond); it
+// also wants a chain long enough for the walkers that share it.  The constants
+// are a fit to 3,000 pairs of times, S 1-2000, R 8-5000, T 100-10,000, within
+// 0.6 % of the better one on average.  us, block / warp: 80 walkers x 300 steps,
+// 148 / 600 samples: 27 / 32, 41 / 34; x 1024, 600 / 2000: 111 / 120, 232 / 144.
+// 1000 x 100, 1: 17 / 17; x 500, 148 / 300: 27 / 40, 44 / 48; x 3000, 600 / 2000:
+// 181 / 332, 484 / 434.  2000 x 10,000, 600 / 2000: 486 / 988, 1341 / 1343.  8 x
+// 2000, 148: 421 / 307.
+inline bool mrw_uniform_by_blocks(uint64_t S, uint32_t R, uint32_t T, int threads,
+                                  uint64_t resident) {
+  if (R < 12 || T < 120.0 + 8000.0 / R) return false;
+  const double step = std::max(43.0 / threads, 0.9 - R / 100.0);
+  return (double)sample_rounds(S, resident) * (110.0 + R / 30.0 + step * T) <= T;
+}
+
 }  // namespace grass

@@ -37,3 +37,10 @@ def test_no_events(oracle_mod):
 def test_more_continuous_time_samples_than_sms(oracle_mod, samples, walkers, steps):
     """Blocks of fewer threads than walkers."""
     _compare(oracle_mod, "rmat_s10_e8", "GT", samples, walkers, steps, G.SELECT_DEGREE_CT)
+
+
+@pytest.mark.parametrize("samples,walkers,steps", [
+    (2, 40, 319), (2, 40, 320), (148, 80, 300), (593, 80, 300), (2, 11, 4000), (2, 12, 4000), (1, 1, 600),
+    (149, 1000, 300), (297, 2000, 600), (2, 5000, 400)])
+def test_uniform_samples_as_blocks_or_warps(oracle_mod, samples, walkers, steps):
+    _compare(oracle_mod, "edge_cases", "LE", samples, walkers, steps, G.SELECT_UNIFORM)

@@ -30,3 +30,14 @@ def rule(tmp_path_factory):
     (1, 512, 512), (1, 513, 544), (8192, 2000, 1024)])
 def test_threads_of_a_continuous_time_sample(rule, samples, walkers, threads):
     assert rule(f"mrw_block_threads({samples}, {walkers}, true, 148)") == threads
+
+
+@pytest.mark.parametrize("samples,walkers,steps,blocks", [
+    (1, 80, 100, False), (148, 80, 300, True), (600, 80, 300, False), (600, 80, 1024, True), (2000, 80, 1024, False),
+    (148, 1000, 300, True), (148, 1000, 511, True), (300, 1000, 500, False), (600, 1000, 3000, True),
+    (2000, 1000, 3000, False), (300, 2000, 2000, True), (600, 2000, 10000, True), (8192, 2000, 10000, False),
+    (148, 8, 500, False), (1, 1, 5000, False), (600, 1, 1024, False)])
+def test_uniform_samples_as_blocks_or_warps(rule, samples, walkers, steps, blocks):
+    threads = rule(f"mrw_block_threads({samples}, {walkers}, false, 148)")
+    resident = 148 * (65536 // (120 * threads))  # (120 registers a thread)
+    assert rule(f"mrw_uniform_by_blocks({samples}, {walkers}, {steps}, {threads}, {resident})") == blocks
