@@ -832,21 +832,44 @@ static int mrw_block_warps(uint64_t warps, size_t bytes) {
   return w;
 }
 
+// Shape of mrw_degree_kernel<.., G, ..> for S samples of R walkers: warps per
+// block, bytes of shared memory per warp (0: the state is in global memory), blocks.
+struct DegreeShape {
+  int w;
+  size_t per_warp;
+  unsigned grid;
+};
+template <int G>
+static DegreeShape mrw_degree_shape(uint64_t S, uint32_t R) {
+  const uint64_t warps = (S + 32 / G - 1) / (32 / G);
+  DegreeShape d;
+  d.per_warp = (size_t)R * 20 * (32 / G);
+  if (d.per_warp > 48 * 1024) d.per_warp = 0;  // too many walkers for shared memory (G = 32)
+  d.w = mrw_block_warps(warps, d.per_warp);
+  d.grid = grid_warps(warps, d.w, cur_dev(), 64 / d.w);
+  return d;
+}
+// Samples of that shape that are resident at once.
+template <int G, class Sum>
+static uint64_t mrw_degree_resident(uint64_t S, uint32_t R) {
+  const DegreeShape d = mrw_degree_shape<G>(S, R);
+  return (uint64_t)sm_count(cur_dev()) * d.w * (32 / G) *
+         std::min(64 / d.w, resident_blocks((const void *)mrw_degree_kernel<kSlots, G, Sum>,
+                                            d.w * 32, d.per_warp * d.w));
+}
+
 template <int G, class Sum>
 static int launch_mrw_degree(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots,
                              uint64_t S, uint32_t *src, uint32_t *dst, unsigned long long *edges,
                              unsigned int *err, cudaStream_t s) {
-  const uint64_t warps = (S + 32 / G - 1) / (32 / G);
-  size_t per_warp = (size_t)p.walkers * 20 * (32 / G);
+  const DegreeShape d = mrw_degree_shape<G>(S, p.walkers);
   uint4 *rec = nullptr;
-  if (per_warp > 48 * 1024) {  // too many walkers for shared memory (G = 32)
+  if (!d.per_warp) {
     cudaError_t e =
         scratch_alloc(reinterpret_cast<void **>(&rec), S * (uint64_t)p.walkers * sizeof(uint4), s);
     if (e != cudaSuccess) return cuda_fail(e, "multi-RW scratch");
-    per_warp = 0;
   }
-  const int w = mrw_block_warps(warps, per_warp);
-  mrw_degree_kernel<kSlots, G, Sum><<<grid_warps(warps, w, cur_dev(), 64 / w), w * 32, per_warp * w, s>>>(
+  mrw_degree_kernel<kSlots, G, Sum><<<d.grid, d.w * 32, d.per_warp * d.w, s>>>(
       g, roots, rec, S, p.walkers, p.steps, p.seed, src, dst, edges, err);
   count_launch();
   if (rec) scratch_free(rec, s);
@@ -880,8 +903,16 @@ int launch_mrw(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots, ui
     return GRASS_OK;
   }
   if (p.select == GRASS_SELECT_DEGREE) {
-    if (p.walkers > 256) return launch_mrw_degree<32, uint64_t>(g, p, roots, S, src, dst, edges, err, s);
-    if ((uint64_t)p.walkers * max_degree >> 32)
+    const bool wide = (uint64_t)p.walkers * max_degree >> 32;  // (sums of 64 bits)
+    bool groups = p.walkers <= kSurelyGroups;
+    if (!groups && p.walkers <= kGroupWalkers)
+      groups = mrw_degree_by_groups(S, p.walkers, p.steps,
+                                    wide ? mrw_degree_resident<8, uint64_t>(S, p.walkers)
+                                         : mrw_degree_resident<8, uint32_t>(S, p.walkers),
+                                    mrw_degree_resident<32, uint64_t>(S, p.walkers));
+    if (!groups)
+      return launch_mrw_degree<32, uint64_t>(g, p, roots, S, src, dst, edges, err, s);
+    if (wide)
       return launch_mrw_degree<8, uint64_t>(g, p, roots, S, src, dst, edges, err, s);
     return launch_mrw_degree<8, uint32_t>(g, p, roots, S, src, dst, edges, err, s);
   }

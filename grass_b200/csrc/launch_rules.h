@@ -59,4 +59,23 @@ inline bool mrw_uniform_by_blocks(uint64_t S, uint32_t R, uint32_t T, int thread
   return (double)sample_rounds(S, resident) * (110.0 + R / 30.0 + step * T) <= T;
 }
 
+// Whether S samples of degree-proportional multi-RW (R walkers of at most
+// kGroupWalkers, T steps) run as groups of eight lanes or as warps, given how many
+// of each are resident.  A step of a group costs less with few walkers a lane to
+// search, and its samples take four times fewer warps, but fewer of them fit with
+// many walkers, and there are fewer loads under way for the first records.  us,
+// groups / warps, 100 steps: 80 walkers, 1500 / 8192 samples 106 / 131, 184 / 361;
+// 160, 121 / 133, 222 / 365; 192, 128 / 134, 232 / 366; 208 (7104 groups
+// resident), 131 / 134, 413 / 369; 256, 141 / 136, 430 / 376.  192 walkers, 12,000
+// samples, 5 / 10 / 50 steps: 77 / 50, 98 / 75, 246 / 285.  (A lone sample has its
+// warp to itself: 256 walkers x 300, 293 / 313, where 148 take 374 / 320.)  Up to
+// kSurelyGroups walkers groups are never slower by more than 2 us, and a launch
+// does not ask what is resident.
+constexpr uint32_t kGroupWalkers = 256, kSurelyGroups = 128;
+inline bool mrw_degree_by_groups(uint64_t S, uint32_t R, uint32_t T, uint64_t groups,
+                                 uint64_t warps) {
+  return S == 1 || (double)sample_rounds(S, groups) * T * (410 + R) + 0.0025 * (double)S * R <=
+                       (double)sample_rounds(S, warps) * T * 600;
+}
+
 }  // namespace grass

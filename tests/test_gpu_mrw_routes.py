@@ -44,3 +44,9 @@ def test_more_continuous_time_samples_than_sms(oracle_mod, samples, walkers, ste
     (149, 1000, 300), (297, 2000, 600), (2, 5000, 400)])
 def test_uniform_samples_as_blocks_or_warps(oracle_mod, samples, walkers, steps):
     _compare(oracle_mod, "edge_cases", "LE", samples, walkers, steps, G.SELECT_UNIFORM)
+
+
+@pytest.mark.parametrize("samples,walkers,steps", [
+    (3, 178, 40), (3, 181, 40), (5, 256, 9), (8000, 208, 30), (5000, 208, 30), (9000, 20, 5), (9000, 160, 5)])
+def test_degree_samples_as_groups_or_warps(oracle_mod, samples, walkers, steps):
+    _compare(oracle_mod, "edge_cases", "GT", samples, walkers, steps, G.SELECT_DEGREE)

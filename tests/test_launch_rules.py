@@ -41,3 +41,11 @@ def test_uniform_samples_as_blocks_or_warps(rule, samples, walkers, steps, block
     threads = rule(f"mrw_block_threads({samples}, {walkers}, false, 148)")
     resident = 148 * (65536 // (120 * threads))  # (120 registers a thread)
     assert rule(f"mrw_uniform_by_blocks({samples}, {walkers}, {steps}, {threads}, {resident})") == blocks
+
+
+@pytest.mark.parametrize("samples,walkers,steps,groups,warps,by_groups", [
+    (1, 80, 100, 15000, 4736, True), (8192, 160, 100, 8288, 4736, True), (8192, 192, 100, 8288, 4736, True),
+    (3000, 192, 100, 8288, 4736, False), (8192, 208, 100, 7104, 4736, False), (7000, 208, 100, 7104, 4736, True),
+    (148, 256, 100, 5920, 4736, False), (1, 256, 100, 5920, 4736, True), (12000, 192, 5, 8288, 4736, False), (12000, 192, 50, 8288, 4736, True)])
+def test_degree_samples_as_groups_or_warps(rule, samples, walkers, steps, groups, warps, by_groups):
+    assert rule(f"mrw_degree_by_groups({samples}, {walkers}, {steps}, {groups}, {warps})") == by_groups
