@@ -3,6 +3,7 @@
 #include <vector>
 
 #include "graph.h"
+#include "launch_rules.h"
 #include "mrw_cta.cuh"
 #include "sample_warp.cuh"
 
@@ -30,9 +31,9 @@ struct BatchTask {
 
 // The work items by kind, in this order: ends of the block-level multi-RW
 // samples, the sequential multi-RW samples, the k-hop seeds and the walker
-// tiles.  parts: warps per k-hop seed.
+// tiles.  parts: warps per k-hop seed; walkers: the most of a block-level sample.
 struct BatchRanges {
-  uint32_t cta, mrw, khop, rw, parts;
+  uint32_t cta, mrw, khop, rw, parts, walkers;
 };
 // Words of the device queue: a counter per kind, zero before a run.
 constexpr uint32_t kQueueWords = 4;
@@ -74,15 +75,22 @@ void split_job(const grass_job &j, uint32_t ji, const grass_batch_config &c,
                std::vector<BatchTask> &cta, std::vector<BatchTask> &mrw,
                std::vector<BatchTask> &khop, std::vector<BatchTask> &rw);
 
+// Walkers of a job's block-level samples (0: it has none).
+inline uint32_t block_walkers(const grass_job &j) {
+  return j.type == GRASS_JOB_MRW && j.select != GRASS_SELECT_DEGREE ? j.walkers : 0;
+}
+
 inline BatchRanges batch_ranges(const std::vector<BatchTask> &cta, const std::vector<BatchTask> &mrw,
                                 const std::vector<BatchTask> &khop,
-                                const std::vector<BatchTask> &rw, const grass_batch_config &c) {
+                                const std::vector<BatchTask> &rw, const grass_batch_config &c,
+                                uint32_t walkers) {
   BatchRanges r;
   r.cta = (uint32_t)cta.size();
   r.mrw = r.cta + (uint32_t)mrw.size();
   r.khop = r.mrw + (uint32_t)khop.size();
   r.rw = r.khop + (uint32_t)rw.size();
   r.parts = c.warps_per_vertex;
+  r.walkers = walkers;
   return r;
 }
 

@@ -54,9 +54,9 @@ __device__ __forceinline__ void count_item(const BatchJob &jb, uint64_t cnt, uin
 }
 
 // Multi-RW samples whose walkers move in parallel, a block each, in a kernel of
-// their own: they want more threads a sample (51 samples of 2000 walkers x
-// 10,000 events alone: 0.50 ms, with 8 warps 0.75), and their workspace would
-// come out of the other items' L1.
+// their own: they want other numbers of threads (batch_block_threads), and their
+// workspace would come out of the other items' L1.  kBatchCtaWarps: the most warps
+// of a block.
 constexpr int kBatchCtaWarps = 16;
 template <int MODE>
 __global__ void __launch_bounds__(32 * kBatchCtaWarps, 2)
@@ -277,8 +277,11 @@ int launch_batch(const DevGraph &dg, int device, const BatchJob *d_jobs, const B
       cs = side->st;
     }
     auto k = dg.mode == GRASS_MODE_CSR_INTERNAL ? batch_cta_kernel<kCsr> : batch_cta_kernel<kSlots>;
-    const unsigned grid = std::min<unsigned>(ranges.cta, (unsigned)sm_count(device) * 2);
-    k<<<grid, 32 * kBatchCtaWarps, 0, cs>>>(dg, d_jobs, d_tasks, ranges.cta, d_queue, d_total,
+    const int threads = batch_block_threads(ranges.cta, ranges.walkers, sm_count(device));
+    const unsigned grid =
+        std::min<unsigned>(ranges.cta, (unsigned)sm_count(device) *
+                                           resident_blocks((const void *)k, threads, 0));
+    k<<<grid, threads, 0, cs>>>(dg, d_jobs, d_tasks, ranges.cta, d_queue, d_total,
                                              d_err);
     cudaError_t e = cudaGetLastError();
     if (side && e == cudaSuccess) e = cudaEventRecord(side->join, cs);
@@ -382,8 +385,10 @@ int build(grass_batch *b) {
   b->free_device();
   std::vector<BatchJob> hj;
   std::vector<BatchTask> cta, mrw, khop, rw;
+  uint32_t walkers = 0;
   for (size_t i = 0; i < b->jobs.size(); i++) {
     const grass_job &j = b->jobs[i];
+    walkers = std::max(walkers, block_walkers(j));
     unsigned char *mscr = nullptr;
     if (j.type == GRASS_JOB_MRW) {
       const uint64_t nr = (uint64_t)j.count * j.walkers;
@@ -402,7 +407,7 @@ int build(grass_batch *b) {
   tasks.insert(tasks.end(), rw.begin(), rw.end());
   if (tasks.size() > 0xFFFFFFF0ull) return set_error(GRASS_E_ARG, "batch: too many work items");
   b->ntasks = (uint32_t)tasks.size();
-  b->ranges = batch_ranges(cta, mrw, khop, rw, c);
+  b->ranges = batch_ranges(cta, mrw, khop, rw, c, walkers);
   GRASS_CUDA(cudaMalloc(&b->d_jobs, std::max<size_t>(hj.size(), 1) * sizeof(BatchJob)));
   GRASS_CUDA(cudaMalloc(&b->d_tasks, std::max<size_t>(tasks.size(), 1) * sizeof(BatchTask)));
   GRASS_CUDA(cudaMalloc(&b->d_queue, kQueueWords * sizeof(unsigned int)));

@@ -34,6 +34,19 @@ inline int mrw_block_threads(uint64_t S, uint32_t R, bool continuous, int sms) {
   return block_size(R, 128, S <= (uint64_t)sms ? 512 : 160);
 }
 
+// Threads of a block of the batch's block-level kernel, which takes `samples`
+// multi-RW samples of up to R walkers (a thread a walker, 64 registers).  Two
+// blocks of 512 fit on an SM.  With more samples than that, the blocks are half as
+// wide as the walkers and 256 threads at most, and more of them are resident.  us
+// in a batch at 512 threads / here, of 256 threads before block-level items had a
+// kernel of their own, LE, R-MAT s22 ef32: uniform, 10,000 samples of 20 walkers x 30
+// 281 / 84 / 225, 2000 of 80 x 100 71 / 34 / 64, 500 of 2000 x 500 57 / 56 / 92;
+// continuous time, the same, 1390 / 473 / 1362, 317 / 143 / 343, 203 / 187 / 361.
+// 51 samples of 2000 x 10,000, at 512 / 256: 106 / 169, 406 / 636.
+inline int batch_block_threads(uint64_t samples, uint32_t R, int sms) {
+  return samples <= 2 * (uint64_t)sms ? block_size(R, 128, 512) : block_size(R / 2, 128, 256);
+}
+
 // Rounds of `resident` samples at a time that S samples take.
 inline uint64_t sample_rounds(uint64_t S, uint64_t resident) {
   return (S + resident - 1) / std::max<uint64_t>(resident, 1);

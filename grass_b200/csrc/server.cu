@@ -463,6 +463,7 @@ void grass_server::launch(Batch *b) {
   const uint64_t jobs_off = off;
   off += align_up(nj * sizeof(BatchJob));
   grass_job gj{};
+  uint32_t walkers = 0;
   for (size_t i = 0; i < nj; i++) {
     const grass_request &r = b->reqs[i]->rq;
     gj.type = r.type;
@@ -470,6 +471,7 @@ void grass_server::launch(Batch *b) {
     gj.walkers = r.walkers;
     gj.steps = r.steps;
     gj.select = r.select;
+    walkers = std::max(walkers, block_walkers(gj));
     split_job(gj, (uint32_t)i, bcfg, cta, mrw, khop, rw);
   }
   const uint64_t ntasks = cta.size() + mrw.size() + khop.size() + rw.size();
@@ -567,7 +569,7 @@ void grass_server::launch(Batch *b) {
       if (e != cudaSuccess) rc = cuda_fail(e, "server upload");
       lap(2);
     }
-    const BatchRanges ranges = batch_ranges(cta, mrw, khop, rw, bcfg);
+    const BatchRanges ranges = batch_ranges(cta, mrw, khop, rw, bcfg, walkers);
     if (!rc && ntasks)
       rc = launch_batch(g->view(), g->device, reinterpret_cast<const BatchJob *>(d + jobs_off),
                         reinterpret_cast<const BatchTask *>(d + tasks_off), ranges,

@@ -50,3 +50,25 @@ def test_uniform_samples_as_blocks_or_warps(oracle_mod, samples, walkers, steps)
     (3, 178, 40), (3, 181, 40), (5, 256, 9), (8000, 208, 30), (5000, 208, 30), (9000, 20, 5), (9000, 160, 5)])
 def test_degree_samples_as_groups_or_warps(oracle_mod, samples, walkers, steps):
     _compare(oracle_mod, "edge_cases", "GT", samples, walkers, steps, G.SELECT_DEGREE)
+
+
+@pytest.mark.parametrize("select", [G.SELECT_UNIFORM, G.SELECT_DEGREE_CT])
+@pytest.mark.parametrize("shapes", [[(296, 40, 20)], [(297, 40, 20)], [(3, 600, 30), (400, 20, 9)], [(100, 300, 40)] * 3])
+def test_block_level_samples_of_a_batch(oracle_mod, shapes, select):
+    """Few and many samples, of one job and of several sizes: blocks of 128 to 512 threads."""
+    import torch
+    prefix = os.path.join(golden_graph("rmat_s10_e8")[0], "LE")
+    g, og = G.Graph(prefix, "LE"), oracle_mod.OracleGraph(prefix)
+    b, checks, rng = G.Batch(g), [], np.random.default_rng(3)
+    for i, (samples, walkers, steps) in enumerate(shapes):
+        roots = rng.integers(0, g.n, (samples, walkers), dtype=np.uint32)
+        outs = [torch.from_numpy(roots.view(np.int32)).cuda(),
+                *(torch.zeros(samples, steps, dtype=torch.int32, device="cuda") for _ in range(2))]
+        b.add_mrw(outs[0], samples, walkers, steps, i, outs[1], outs[2], select=select)
+        src, dst, end, _ = og.mrw("LE", roots, steps, i, select)
+        checks += zip(outs, (end, src, dst))
+    for _ in range(2):
+        b.run()
+        torch.cuda.synchronize()
+        for got, ref in checks:
+            np.testing.assert_array_equal(got.cpu().numpy().view(np.uint32), ref)

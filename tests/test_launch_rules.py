@@ -49,3 +49,9 @@ def test_uniform_samples_as_blocks_or_warps(rule, samples, walkers, steps, block
     (148, 256, 100, 5920, 4736, False), (1, 256, 100, 5920, 4736, True), (12000, 192, 5, 8288, 4736, False), (12000, 192, 50, 8288, 4736, True)])
 def test_degree_samples_as_groups_or_warps(rule, samples, walkers, steps, groups, warps, by_groups):
     assert rule(f"mrw_degree_by_groups({samples}, {walkers}, {steps}, {groups}, {warps})") == by_groups
+
+
+@pytest.mark.parametrize("samples,walkers,threads", [
+    (1, 8, 128), (296, 80, 128), (296, 300, 320), (296, 2000, 512), (297, 300, 160), (297, 2000, 256), (10000, 20, 128)])
+def test_threads_of_a_batch_sample(rule, samples, walkers, threads):
+    assert rule(f"batch_block_threads({samples}, {walkers}, 148)") == threads
