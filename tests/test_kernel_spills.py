@@ -28,12 +28,20 @@ LIMITS = {
         "rw_csr_kernel<1>": (64, 0), "rw_csr_kernel<2>": (64, 0), "rw_csr_kernel<4>": (64, 0),
         "n2v_kernel<1>": (64, 0), "n2v_kernel<2>": (64, 0),
         "khop_kernel<1>": (64, 48), "khop_csr_kernel": (64, 24),
+        # eight blocks of 256 threads
+        "mrw_kernel<1>": (32, 48),
+        "mrw_degree_kernel<1, 8, unsigned int>": (64, 0), "mrw_degree_kernel<1, 8, unsigned long>": (64, 0),
+        "mrw_degree_kernel<1, 32, unsigned long>": (64, 0),
+        # a block of 512 threads; the wide kernel a block of 1024
+        "mrw_cta_kernel<1, 16>": (120, 0), "mrw_cta_kernel<1, 32>": (64, 64),
     },
+    "kernels_decode.cu": {"decode_flat_kernel<1>": (64, 36)},  # 16 blocks of 64 threads
+    "kernels_compact.cu": {"compact_fill_kernel<0>": (64, 0), "compact_fill_kernel<1>": (64, 0)},
     "kernels_batch.cu": {
         # four blocks of 256 threads; three with two walkers a lane, two with four (CSR: three)
         "batch_kernel<1, 1>": (64, 88), "batch_kernel<1, 2>": (80, 56), "batch_kernel<1, 4>": (128, 176),
         "batch_kernel<2, 1>": (64, 56), "batch_kernel<2, 2>": (80, 56), "batch_kernel<2, 4>": (80, 12),
-        "batch_cta_kernel<1>": (64, 48), "batch_cta_kernel<2>": (64, 36),
+        "batch_cta_kernel<1>": (64, 48), "batch_cta_kernel<2>": (64, 44),
     },
 }
 
