@@ -435,7 +435,7 @@ extern "C" {
 
 const char *grass_last_error(void) { return grass::t_err.c_str(); }
 uint64_t grass_launch_count(void) { return grass::g_launches.load(); }
-const char *grass_version(void) { return "grass_b200 0.1 (sm_100a)"; }
+const char *grass_version(void) { return "grass_b200 0.2 (sm_100a)"; }
 
 int grass_open(const char *prefix, int mode, int device, grass_graph **out) {
   grass::Nvtx nvtx_("grass_open");

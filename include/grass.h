@@ -57,7 +57,8 @@ extern "C" {
 const char *grass_last_error(void);
 /* Number of CUDA kernels this library has launched in this process. */
 uint64_t grass_launch_count(void);
-/* Library version string. */
+/* Library version string, "grass_b200 <major>.<minor> (sm_100a)": the minor
+ * number changes with the layout that grass_device_view hands out. */
 const char *grass_version(void);
 
 /* =========================================================================
@@ -122,7 +123,9 @@ typedef struct {
   int32_t device;
   uint64_t graph_file_bytes;  /* .graph size                              */
   uint64_t offset_file_bytes; /* .offset size                             */
-  uint64_t device_bytes;      /* resident: stream words + offset index    */
+  uint64_t device_bytes;      /* resident: slot words + vertex records (not the
+                                 decode plan and the node2vec index that the
+                                 first such calls add)                     */
   double read_seconds;        /* file read into pinned memory             */
   double upload_seconds;      /* copies + device index build              */
 } grass_graph_info;
@@ -146,7 +149,9 @@ int grass_check_device_error(grass_graph *g, void *stream);
  * kernels): the slot words (n_words + at least 16 zero guard words, each word
  * the next 32 bits MSB-first) and the n vertex records, 16 bytes each, which
  * replace the reference's uint64 bit-offset table (GT/src/utils.hpp:363).
- * The layout is the library's own, the same for GT and LE files: neighbors
+ * The layout is the library's own and goes with its version (grass_version):
+ * 0.2 on as here, in 0.1 the words held the files' codes and the records other
+ * fields.  The same for GT and LE files: neighbors
  * cT .. cT + T - 1 of a vertex share slot c,
  *   [head n_cT - n_0 (a bits)][offsets n_i - n_cT (b bits) of i = cT+1 ..],
  * of cb = a + (T - 1) b bits at bit P + (c / K) 256 + (c % K) cb, inside one
