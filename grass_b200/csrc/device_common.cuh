@@ -410,17 +410,6 @@ __device__ __forceinline__ VHdr record_header(const uint4 r) {
   return h;
 }
 
-// Exact x / d for x < 2^32 and 2 <= d < 2^32 by one 64-bit multiply-high.
-// M = floor((2^64 - 1) / d) + 1 = 2^64 / d + e with 0 <= e < 1, so
-// x M / 2^64 = x / d + x e / 2^64, and x e / 2^64 < 2^-32 < 1 / d never
-// carries the quotient past the next integer.  d = 1 passes x through.
-__host__ __device__ __forceinline__ uint64_t div_magic(uint32_t d) {
-  return d >= 2 ? ~0ull / d + 1 : 0ull;
-}
-__device__ __forceinline__ uint32_t div_by(uint32_t x, uint32_t d, uint64_t M) {
-  return d >= 2 ? (uint32_t)__umul64hi((uint64_t)x, M) : x;
-}
-
 // Exact x / d for x < 2^31 (degrees are below it) and the layout's small
 // divisors 1 <= d < 64 (chunk length T, slots per sector K): with 2^(s-1) < d
 // <= 2^s and m = ceil(2^(31+s) / d) < 2^32, x m / 2^(31+s) = x / d + x e /
@@ -506,11 +495,6 @@ __device__ __forceinline__ VHdr header(const DevGraph &g, uint32_t v) {
 
 __device__ __forceinline__ uint32_t record_degree(const DevGraph &g, uint32_t v) {
   return __ldg(&g.recs[v].z);
-}
-
-// Length of gamma(x): 2 floor(log2(x+1)) + 1.
-__device__ __forceinline__ uint32_t gamma_len(uint32_t x) {
-  return 2u * (31u - __clz(x + 1u)) + 1u;
 }
 
 template <int MODE>

@@ -63,17 +63,18 @@ struct grass_graph {
   unsigned int *d_err = nullptr;   // device error word (GRASS_E_DATA on bad ids)
   grass_graph_info info{};
   grass_tuning tuning{};
-  // Decode plan, built by the first grass_decode_all and kept: the neighbor
-  // ranges (v, i0, i1, 0) of vertices with degree >= 32, at most 2048
-  // neighbors each, and the vertices of degree 1..31 grouped by
-  // floor(log2(degree)).
+  // Plan of the staged decode sweep (tuning.decode_stage_depth > 0), built by the
+  // first such grass_decode_all and kept: the neighbor ranges (v, i0, i1, 0) of
+  // vertices with degree >= 32, at most 2048 neighbors each, and the vertices of
+  // degree 1..31 grouped by floor(log2(degree)).
   mutable std::mutex plan_mu;
   mutable uint4 *d_plan_big = nullptr;
   mutable uint32_t *d_plan_small = nullptr;
   mutable uint64_t plan_nbig = 0, plan_nsmall = 0;
   mutable bool plan_ok = false;
-  // The flat plan of the default (unstaged) sweep: runs of consecutive
-  // vertices (v0, v1, 0, 0) and hub neighbor ranges (v, v + 1, i0, i1).
+  // The flat plan of the default (unstaged) sweep, built by the first
+  // grass_decode_all without staging and kept: runs of consecutive vertices
+  // (v0, v1, 0, 0) and hub neighbor ranges (v, v + 1, i0, i1).
   mutable uint4 *d_plan_flat = nullptr;
   mutable uint64_t plan_nflat = 0;
   mutable bool plan_flat_ok = false;

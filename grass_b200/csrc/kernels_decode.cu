@@ -153,11 +153,11 @@ __global__ void __launch_bounds__(256) decode_all_kernel(DevGraph g, const uint6
 }
 
 // ---------------------------------------------------------------------------
-// Planned sweep.  The first sweep of a graph builds a plan once: vertices of
-// degree >= 32 become neighbor ranges of at most 2048 (hubs are split), the
-// others are grouped by floor(log2(degree)).  Then
-//  * a range is decoded by one warp, one lane per chunk slot, 32 slots at a
-//    time (decode_range_kernel);
+// Plan of the staged sweep (decode_stage_depth 1, 2 or 4), built by the first
+// such sweep of a graph: vertices of degree >= 32 become neighbor ranges of at
+// most 2048 (hubs are split), the others are grouped by floor(log2(degree)).
+//  * A range is decoded by one warp, a neighbor per lane, from whole sectors
+//    staged in shared memory (decode_range_kernel);
 //  * a small vertex is decoded by one lane, slot after slot; a warp takes 32
 //    vertices of one degree class, so its lanes run for similar lengths.
 constexpr uint32_t kBigDegree = 32;

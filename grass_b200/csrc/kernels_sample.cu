@@ -264,11 +264,6 @@ __global__ void __launch_bounds__(256, MODE == kCsr ? GRASS_N2V_CSR_MIN_BLOCKS :
   if (bad && err) atomicOr(err, 1u);
 }
 
-// Replays a walk (same stream as rw_kernel) and sums, per draw, the
-// algorithmic bytes 16 (vertex record) + ceil(slot bits read / 8) + 4
-// (path entry) and the 32-byte sectors the reads span (+1 for the record).
-// out[0] = bytes, out[1] = sectors, out[2] = draws.  Start entries add 4
-// bytes each.
 // Independent random 4-byte reads: each thread draws xorshift64 indices into
 // buf[0, mask] and keeps 8 loads in flight; the sum goes to *sink so the loads
 // are not dropped.  Used to measure the device's random-read ceiling.
@@ -295,6 +290,11 @@ __global__ void __launch_bounds__(256) random_read_kernel(const uint32_t *__rest
   if ((threadIdx.x & 31) == 0) atomicAdd(sink, (unsigned long long)acc);
 }
 
+// Replays a walk (same stream as rw_kernel) and sums, per draw, the
+// algorithmic bytes 16 (vertex record) + ceil(slot bits read / 8) + 4
+// (path entry) and the 32-byte sectors the reads span (+1 for the record).
+// out[0] = bytes, out[1] = sectors, out[2] = draws.  Start entries add 4
+// bytes each.
 __global__ void __launch_bounds__(256) rw_account_kernel(DevGraph g,
                                                          const uint32_t *__restrict__ starts,
                                                          uint64_t W, uint32_t L, uint64_t seed,

@@ -18,7 +18,7 @@
 //    process (next mover x with probability d_x / sum d).  Each walker's
 //    events come from its own Philox stream (counter {k, sample, walker,
 //    TAG_MRW_CT}); the block simulates all walkers up to a time horizon,
-//    raising the horizon in phases until T events exist, sorts the events by
+//    raising the horizon in phases until T events exist, orders the events by
 //    (time, walker) and keeps the first T.  Event times use det_log, so the
 //    host oracle (an event heap) reproduces them bit for bit.
 #pragma once
@@ -72,7 +72,7 @@ struct CtaSmem {
   uint32_t hist[NW][256];
   uint32_t tot[256];
   uint64_t red[32];
-  uint32_t n_events, overflow, skip, task;
+  uint32_t n_events, skip, task;
 };
 
 __host__ __device__ inline uint64_t mrw_ct_cap(uint32_t T) { return 2ull * T + 4096; }
@@ -416,10 +416,7 @@ __device__ void mrw_ct_cta(const DevGraph &g, uint32_t *roots, uint32_t *src, ui
       rec[w] = r;
       dsum += r.z;
     }
-    if (tid == 0) {
-      sm.n_events = 0;
-      sm.overflow = 0;
-    }
+    if (tid == 0) sm.n_events = 0;
     dsum = cta_sum_u64(dsum, sm);
     if (dsum == 0) {
       N = 0;
@@ -427,7 +424,6 @@ __device__ void mrw_ct_cta(const DevGraph &g, uint32_t *roots, uint32_t *src, ui
       break;
     }
     H = frac * (double)T / (double)dsum;
-    bool overflow = false;
     for (int phase = 0; phase < 512; phase++) {
       // Every walker runs its events with time <= H.  (One walker per thread at
       // a time: two or four side by side took 286 and 371 us a sample, not 250;
@@ -455,10 +451,7 @@ __device__ void mrw_ct_cta(const DevGraph &g, uint32_t *roots, uint32_t *src, ui
       }
       __syncthreads();
       N = sm.n_events;
-      if (N > cap) {
-        overflow = true;
-        break;
-      }
+      if (N > cap) break;
       if (N >= T) {
         done = true;
         break;
@@ -478,7 +471,6 @@ __device__ void mrw_ct_cta(const DevGraph &g, uint32_t *roots, uint32_t *src, ui
     if (!done) {  // too many events in one phase (or no convergence): smaller steps
       frac *= 0.25;
       ext *= 0.5;
-      (void)overflow;
     }
   }
   if (!done) {
