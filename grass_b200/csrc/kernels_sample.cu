@@ -891,10 +891,15 @@ int launch_mrw(const DevGraph &g, const grass_mrw_params &p, uint32_t *roots, ui
     resident = (uint64_t)sm_count(cur_dev()) * resident_blocks((const void *)cta, threads, 0);
   if (ct || (p.select == GRASS_SELECT_UNIFORM &&
              mrw_uniform_by_blocks(S, p.walkers, p.steps, threads, resident))) {
-    const uint64_t grid = std::min<uint64_t>(S, resident);
     const uint64_t stride = mrw_sample_scratch(p.walkers, p.steps, p.select);
+    uint64_t grid = std::min<uint64_t>(S, resident);
     unsigned char *scr = nullptr;
     cudaError_t e = scratch_alloc(reinterpret_cast<void **>(&scr), grid * stride, s);
+    while (e == cudaErrorMemoryAllocation && grid > 1) {  // a block takes one sample after another
+      cudaGetLastError();
+      grid /= 2;
+      e = scratch_alloc(reinterpret_cast<void **>(&scr), grid * stride, s);
+    }
     if (e != cudaSuccess) return cuda_fail(e, "multi-RW scratch");
     cta<<<(unsigned)grid, threads, 0, s>>>(
         g, roots, S, p.walkers, p.steps, p.select, p.seed, src, dst, scr, stride, edges, err);

@@ -72,3 +72,23 @@ def test_block_level_samples_of_a_batch(oracle_mod, shapes, select):
         torch.cuda.synchronize()
         for got, ref in checks:
             np.testing.assert_array_equal(got.cpu().numpy().view(np.uint32), ref)
+
+
+def test_scratch_for_fewer_blocks(oracle_mod):
+    """Block-level samples where the scratch of all resident blocks does not fit (some 4 GB): the same chains."""
+    import torch
+    g = G.Graph(os.path.join(golden_graph("rmat_s10_e8")[0], "LE"), "LE")
+    S, R, T = 500, 400, 100_000
+    roots = torch.randint(0, g.n, (S, R), dtype=torch.int32, device="cuda")
+    calls = [[roots.clone(), *(torch.zeros(S, T, dtype=torch.int32, device="cuda") for _ in range(2))] for _ in range(2)]
+    hog = []
+    for walkers, src, dst in calls:
+        g.mrw_device(walkers, S, R, T, 3, src, dst, select=G.SELECT_DEGREE_CT)
+        g.check_device_error()
+        torch.cuda.empty_cache()
+        if not hog:  # (the library's pool gives back what it freed when the device is idle)
+            hog.append(torch.empty(torch.cuda.mem_get_info()[0] - (2 << 30), dtype=torch.uint8, device="cuda"))
+    del hog
+    torch.cuda.empty_cache()
+    for a, b in zip(*calls):
+        assert torch.equal(a, b)
