@@ -106,10 +106,10 @@ struct BatchSide {
 };
 
 // Launches the persistent kernels on graph `dg` (compressed or CSR) of device
-// `device` over the work items of `ranges`: block-level and warp-level items
-// have a kernel each, which run side by side where both kinds are present
-// (side, created here, joins stream s again; null: one after the other on s).  d_queue: kQueueWords zeroed
-// words.  Corrupt payloads set bit 0 of *d_err.
+// `device` over the work items of `ranges`: block-level and warp-level items have
+// a kernel each, which run side by side where both kinds are present (side,
+// created here, joins stream s again; null: one after the other on s).  d_queue:
+// kQueueWords zeroed words.  Corrupt payloads set bit 0 of *d_err.
 int launch_batch(const DevGraph &dg, int device, const BatchJob *d_jobs, const BatchTask *d_tasks,
                  const BatchRanges &ranges, unsigned int *d_queue, unsigned long long *d_total,
                  unsigned int *d_err, cudaStream_t s, BatchSide *side,

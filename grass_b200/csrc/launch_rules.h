@@ -24,10 +24,10 @@ constexpr uint32_t kWideWalkers = 512;
 // SMs, in a launch of its own (mrw_cta_kernel).  Continuous time: a thread a
 // walker is fastest while every sample has an SM to itself.  With more samples
 // blocks of 160 threads pay, three of which are resident where one of 288 to 512
-// is (us with a thread a walker / 160 / R / 2 and the radix sort: 257
-// walkers x 400 steps, 148 samples 73 / 85 / 145, 300 130 / 92 / 153, 8192 3022 /
-// 1613 / 1984.  512 x 400: 148 56 / 89 / 111, 300 119 / 98 / 195, 8192 2463 / 1838 /
-// 2851).
+// is.  us with a thread a walker / 160 threads / half a thread a walker and the
+// radix sort: 257 walkers x 400 steps, 148 samples 73 / 85 / 145, 300 130 / 92 /
+// 153, 8192 3022 / 1613 / 1984; 512 x 400, 148 56 / 89 / 111, 300 119 / 98 / 195,
+// 8192 2463 / 1838 / 2851.
 inline int mrw_block_threads(uint64_t S, uint32_t R, bool continuous, int sms) {
   if (!continuous) return block_size(R / 2, 128, 512);
   if (R > kWideWalkers) return block_size(R, 128, 1024);
